@@ -59,32 +59,54 @@ __global__ void k_state_init(double* st, int NV, int nva) {
   st[S_STEPS * NV + v] = v < nva ? 0.0 : 1.0;
 }
 
+// The per-CTA partials [ncta][NV] are summed by one CTA of kFinThreads
+// threads per 32 vectors: thread t takes vector t % VB of the rows t / VB,
+// t / VB + slots, ..., then the slots are added by halves. One thread per
+// vector walking all ncta (up to 1184) rows was a chain of dependent L2
+// loads: 80-150 us per launch against 5-8 us.
+constexpr int kFinThreads = 512;
+
+template <typename S>
+__device__ __forceinline__ S fin_sum(int NV, int ncta, const S* __restrict__ partial, S* sh) {
+  const int VB = min(NV, 32), slots = kFinThreads / VB;
+  const int v = blockIdx.x * VB + threadIdx.x % VB;
+  S t = 0;
+  for (int b = threadIdx.x / VB; b < ncta; b += slots) t += partial[static_cast<int64_t>(b) * NV + v];
+  sh[threadIdx.x] = t;
+  for (int o = kFinThreads / 2; o >= VB; o >>= 1) {
+    __syncthreads();
+    if (static_cast<int>(threadIdx.x) < o) sh[threadIdx.x] += sh[threadIdx.x + o];
+  }
+  return sh[threadIdx.x];  // valid for threadIdx.x < VB
+}
+
 // alpha_j = Re<q_j, H q_j>: exact sum of the H*V kernels' fixed-point
 // partials, so it does not depend on their grid or row scheduling.
-__global__ void k_alpha_fin(int NV, int ncta, const fx128* __restrict__ partial, double* __restrict__ st,
-                            double* __restrict__ alpha_j) {
-  const int v = threadIdx.x;
-  if (v >= NV) return;
-  fx128 t = 0;
-  for (int b = 0; b < ncta; ++b) t += partial[static_cast<int64_t>(b) * NV + v];
+__global__ void __launch_bounds__(kFinThreads) k_alpha_fin(int NV, int ncta, const fx128* __restrict__ partial,
+                                                           double* __restrict__ st, double* __restrict__ alpha_j) {
+  __shared__ fx128 sh[kFinThreads];
+  const fx128 t = fin_sum(NV, ncta, partial, sh);
+  const int v = blockIdx.x * min(NV, 32) + threadIdx.x;
+  if (static_cast<int>(threadIdx.x) >= min(NV, 32)) return;
   const double s = fx_to_double(t);
   alpha_j[v] = s;
   st[S_CA * NV + v] = s * st[S_CUR * NV + v];
   st[S_CB * NV + v] = st[S_BPREV * NV + v] * st[S_PREV * NV + v];
 }
 
-__global__ void k_beta_fin(int NV, int ncta, const double* __restrict__ partial, double* __restrict__ st,
-                           double* __restrict__ beta_j, int j, int kdim) {
-  const int v = threadIdx.x;
-  if (v >= NV) return;
+__global__ void __launch_bounds__(kFinThreads) k_beta_fin(int NV, int ncta, const double* __restrict__ partial,
+                                                          double* __restrict__ st, double* __restrict__ beta_j, int j,
+                                                          int kdim) {
+  __shared__ double sh[kFinThreads];
+  const double s = fin_sum(NV, ncta, partial, sh);
+  const int v = blockIdx.x * min(NV, 32) + threadIdx.x;
+  if (static_cast<int>(threadIdx.x) >= min(NV, 32)) return;
   if (st[S_DONE * NV + v] != 0.0) {
     st[S_CUR * NV + v] = 0.0;
     st[S_PREV * NV + v] = 0.0;
     st[S_BPREV * NV + v] = 0.0;
     return;
   }
-  double s = 0.0;
-  for (int b = 0; b < ncta; ++b) s += partial[static_cast<int64_t>(b) * NV + v];
   const double bet = sqrt(s);
   if (bet < 1e-12 || j + 1 == kdim) {
     st[S_STEPS * NV + v] = static_cast<double>(j + 1);
@@ -632,7 +654,7 @@ void run_ftlm_block(Ctx& c, int n_up, int n_dn, int mx, int my, Spectrum& out, c
         FTLM_CUDA(cudaEventRecord(e1, c.stream));
         evs.emplace_back(e0, e1);
       }
-      k_alpha_fin<<<1, 128, 0, c.stream>>>(NV, ncta, c.partial.as<fx128>(), st, alpha + static_cast<int64_t>(j) * ld);
+      k_alpha_fin<<<(NV + 31) / 32, kFinThreads, 0, c.stream>>>(NV, ncta, c.partial.as<fx128>(), st, alpha + static_cast<int64_t>(j) * ld);
       if (fp32) {
         using V = float4;
         if (split)
@@ -654,7 +676,7 @@ void run_ftlm_block(Ctx& c, int n_up, int n_dn, int mx, int my, Spectrum& out, c
               nchunks, NV, c.vec_h.as<V>(), static_cast<const V*>(cur), static_cast<V*>(prev), st,
               c.partial.as<double>(), nullptr, nullptr, nullptr, fph);
       }
-      k_beta_fin<<<1, 128, 0, c.stream>>>(NV, ugrid, c.partial.as<double>(), st, beta + static_cast<int64_t>(j) * ld, j, K);
+      k_beta_fin<<<(NV + 31) / 32, kFinThreads, 0, c.stream>>>(NV, ugrid, c.partial.as<double>(), st, beta + static_cast<int64_t>(j) * ld, j, K);
       FTLM_LAUNCH_CHECK();
       c.prof.kernel_launches += 3;
       std::swap(cur, prev);
