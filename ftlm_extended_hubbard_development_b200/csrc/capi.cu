@@ -203,6 +203,7 @@ void ftlm_ctx_destroy(ftlm_ctx* ctx) {
                         &c.sb_rp, &c.sb_col, &c.sb_val, &c.sb_diag, &c.sb_meta, &c.sb_steps,
                         &c.scan_tmp, &c.dense_arena, &c.dense_meta, &c.dense_out, &c.spectra, &c.th_beta,
                         &c.th_mu, &c.th_state, &c.hl_ptr, &c.hl_ent, &c.flip_map, &c.vec_xd, &c.vec_yd, &c.seg_counter, &c.stn_crb, &c.stn_rp, &c.stn_rp32, &c.stn_ent, &c.stn_cnt,
+                        &c.stn_rp4, &c.stn_row, &c.stn_ent4, &c.stn_deg, &c.stn_coef, &c.stn_seg, &c.stn_cls, &c.stn_diag,
                         &c.defer_arena, &c.defer_ev, &c.defer_work, &c.defer_ab, &c.defer_st};
   for (auto* b : bufs) b->release();
   if (c.flipped) {
@@ -211,7 +212,8 @@ void ftlm_ctx_destroy(ftlm_ctx* ctx) {
                         &f.sec.d_star, &f.sec.d_hs, &f.sec.d_stab, &f.sec.d_chi, &f.sec.d_cidx, &f.sec.canon,
                         &f.sec.tmp_a, &f.sec.tmp_b, &f.sec.tmp_c, &f.sec.tmp_d, &f.sec.tmp_e, &f.blk.act,
                         &f.blk.act_list, &f.blk.aoff, &f.blk.dtab, &f.blk.row_meta, &f.blk.row_dn, &f.scan_tmp,
-                        &f.stn_crb, &f.stn_rp, &f.stn_rp32, &f.stn_ent, &f.stn_cnt};
+                        &f.stn_crb, &f.stn_rp, &f.stn_rp32, &f.stn_ent, &f.stn_cnt,
+                        &f.stn_rp4, &f.stn_row, &f.stn_ent4, &f.stn_deg, &f.stn_coef, &f.stn_seg, &f.stn_cls, &f.stn_diag};
     for (auto* b : fb) b->release();  // binom tables are the owner's
     c.flipped.reset();
   }

@@ -219,6 +219,10 @@ struct Ctx {
   bool stn_ok = false;
   int64_t stn_for[3] = {-1, -1, -1};  // (sector generation, mx, my) they belong to
   DBuf stn_crb, stn_rp, stn_rp32, stn_ent, stn_cnt;
+  DBuf stn_rp4, stn_row, stn_ent4, stn_deg, stn_coef;  // entries of the wide sweeps in runs of one coefficient
+  DBuf stn_seg, stn_cls;           // segments by class, class list
+  DBuf stn_diag;                   // diagonal per row, in the sweeps' type
+  std::vector<int64_t> stn_classes;  // per class with rows: number of segments, rows per segment
   bool hv_rows = true;  // narrow sweeps on the hop list: 8 lanes per row (FTLM_HV_ROWS=0: warp per row)
   bool small_blocks = true;  // batched FTLM runs blocks <= kSmallMaxDim in one launch (FTLM_SMALL_BLOCKS=0: off)
   int64_t hl_nnz = 0;
@@ -316,6 +320,9 @@ bool split_prepare(Ctx& c, int nv, bool fp32);
 // that row count.
 int hv_apply_split(Ctx& c, const void* in, const void* in_d, void* out, void* out_d, int nv, bool fp32,
                    const double* scale, fx128* partial);
+// Whether those sweeps leave y unscaled (the wide stencil kernel): the
+// Lanczos update then applies the scale.
+bool hv_split_unscaled(const Ctx& c, int nv, bool fp32);
 int hv_split_max_grid(const Ctx& c);
 // x_D[p(q)] = conj(f_q) x[q];  y[q] += f_q y_D[p(q)].
 void flip_scatter(Ctx& c, const void* x, void* xd, int nv, bool fp32);

@@ -122,7 +122,8 @@ __global__ void __launch_bounds__(kFinThreads) k_beta_fin(int NV, int ncta, cons
   st[S_BPREV * NV + v] = bet;
 }
 
-// w_prev <- y - ca*w_cur - cb*w_prev, per-vector |.|^2 partials.
+// w_prev <- cy*y - ca*w_cur - cb*w_prev, per-vector |.|^2 partials; cy is the
+// current vector's scale where the H*V kernel left y unscaled, else 1.
 // FLIP (split-spin H*V): y is completed by the flipped-order output,
 // y[q] + f_q y_D[p(q)], and the new vector is also written in the flipped
 // order, x_D[p(q)] = conj(f_q) w[q].
@@ -134,16 +135,17 @@ __global__ void __launch_bounds__(kUpdThreads) k_update(int64_t nchunks, int NV,
                                                         const typename VT<T>::V* __restrict__ yd,
                                                         typename VT<T>::V* __restrict__ xd,
                                                         const uint64_t* __restrict__ fmap,
-                                                        const __grid_constant__ FlipPhase ph) {
+                                                        const __grid_constant__ FlipPhase ph, int unscaled) {
   using V = typename VT<T>::V;
   constexpr int VPL = VT<T>::VPL;
   const int CPR = NV / VPL;
   __shared__ double red[kUpdThreads * 2];
   const int tid = threadIdx.x;
   const int cv = tid % CPR;  // stride is a multiple of CPR, so fixed per thread
-  double ca[VPL], cb[VPL], acc[VPL];
+  double ca[VPL], cb[VPL], cy[VPL], acc[VPL];
 #pragma unroll
   for (int e = 0; e < VPL; ++e) {
+    cy[e] = unscaled ? st[S_CUR * NV + cv * VPL + e] : 1.0;
     ca[e] = st[S_CA * NV + cv * VPL + e];
     cb[e] = st[S_CB * NV + cv * VPL + e];
     acc[e] = 0.0;
@@ -169,10 +171,10 @@ __global__ void __launch_bounds__(kUpdThreads) k_update(int64_t nchunks, int NV,
         h2 += fr * d.z - fim * d.w;
         h3 += fr * d.w + fim * d.z;
       }
-      const double r0 = h0 - ca[0] * x.x - cb[0] * p.x;
-      const double r1 = h1 - ca[0] * x.y - cb[0] * p.y;
-      const double r2 = h2 - ca[1] * x.z - cb[1] * p.z;
-      const double r3 = h3 - ca[1] * x.w - cb[1] * p.w;
+      const double r0 = cy[0] * h0 - ca[0] * x.x - cb[0] * p.x;
+      const double r1 = cy[0] * h1 - ca[0] * x.y - cb[0] * p.y;
+      const double r2 = cy[1] * h2 - ca[1] * x.z - cb[1] * p.z;
+      const double r3 = cy[1] * h3 - ca[1] * x.w - cb[1] * p.w;
       r = make_float4(static_cast<float>(r0), static_cast<float>(r1), static_cast<float>(r2), static_cast<float>(r3));
       acc[0] += static_cast<double>(r.x) * r.x + static_cast<double>(r.y) * r.y;
       acc[1] += static_cast<double>(r.z) * r.z + static_cast<double>(r.w) * r.w;
@@ -183,8 +185,8 @@ __global__ void __launch_bounds__(kUpdThreads) k_update(int64_t nchunks, int NV,
         h0 += fr * d.x - fim * d.y;
         h1 += fr * d.y + fim * d.x;
       }
-      r.x = h0 - ca[0] * x.x - cb[0] * p.x;
-      r.y = h1 - ca[0] * x.y - cb[0] * p.y;
+      r.x = cy[0] * h0 - ca[0] * x.x - cb[0] * p.x;
+      r.y = cy[0] * h1 - ca[0] * x.y - cb[0] * p.y;
       acc[0] += r.x * r.x + r.y * r.y;
     }
     wp[i] = r;
@@ -637,6 +639,7 @@ void run_ftlm_block(Ctx& c, int n_up, int n_dn, int mx, int my, Spectrum& out, c
     k_state_init<<<1, 128, 0, c.stream>>>(st, NV, nva);
     void* cur = c.vec_a.p;
     void* prev = c.vec_b.p;
+    const int unscaled = split && hv_split_unscaled(c, NV, fp32) ? 1 : 0;
     for (int j = 0; j < K; ++j) {
       cudaEvent_t e0 = nullptr, e1 = nullptr;
       if (c.timing) {
@@ -660,21 +663,21 @@ void run_ftlm_block(Ctx& c, int n_up, int n_dn, int mx, int my, Spectrum& out, c
         if (split)
           k_update<float, true><<<ugrid, kUpdThreads, 0, c.stream>>>(
               nchunks, NV, c.vec_h.as<V>(), static_cast<const V*>(cur), static_cast<V*>(prev), st,
-              c.partial.as<double>(), c.vec_yd.as<V>(), c.vec_xd.as<V>(), fmap, fph);
+              c.partial.as<double>(), c.vec_yd.as<V>(), c.vec_xd.as<V>(), fmap, fph, unscaled);
         else
           k_update<float, false><<<ugrid, kUpdThreads, 0, c.stream>>>(
               nchunks, NV, c.vec_h.as<V>(), static_cast<const V*>(cur), static_cast<V*>(prev), st,
-              c.partial.as<double>(), nullptr, nullptr, nullptr, fph);
+              c.partial.as<double>(), nullptr, nullptr, nullptr, fph, 0);
       } else {
         using V = double2;
         if (split)
           k_update<double, true><<<ugrid, kUpdThreads, 0, c.stream>>>(
               nchunks, NV, c.vec_h.as<V>(), static_cast<const V*>(cur), static_cast<V*>(prev), st,
-              c.partial.as<double>(), c.vec_yd.as<V>(), c.vec_xd.as<V>(), fmap, fph);
+              c.partial.as<double>(), c.vec_yd.as<V>(), c.vec_xd.as<V>(), fmap, fph, unscaled);
         else
           k_update<double, false><<<ugrid, kUpdThreads, 0, c.stream>>>(
               nchunks, NV, c.vec_h.as<V>(), static_cast<const V*>(cur), static_cast<V*>(prev), st,
-              c.partial.as<double>(), nullptr, nullptr, nullptr, fph);
+              c.partial.as<double>(), nullptr, nullptr, nullptr, fph, 0);
       }
       k_beta_fin<<<(NV + 31) / 32, kFinThreads, 0, c.stream>>>(NV, ugrid, c.partial.as<double>(), st, beta + static_cast<int64_t>(j) * ld, j, K);
       FTLM_LAUNCH_CHECK();

@@ -38,7 +38,6 @@ namespace ftlm {
 namespace {
 
 constexpr int kSegGrab = 2;  // rows a warp takes from the shared row counter at a time
-constexpr int kStnGrab = 4;  // the same for the stencil sweeps
 
 int grid_rows(int64_t n, int threads) {
   return static_cast<int>(std::max<int64_t>(1, std::min<int64_t>((n + threads - 1) / threads, 1 << 20)));
@@ -294,129 +293,272 @@ __global__ void k_stencil(int fill, const __grid_constant__ Geom g, int nclass, 
   }
 }
 
-// The segment sweep (same contract as k_hv_seg) with the class stencils as
-// the operator source.
-template <typename W, typename T, int NV, int U, int MINB>
-__global__ void __launch_bounds__(kHvThreads, MINB) k_hv_stn(const __grid_constant__ HvParams<W> P,
-                                                           const int64_t* __restrict__ crb,
-                                                           const int32_t* __restrict__ srp,
-                                                           const uint32_t* __restrict__ sent,
-                                                           const typename CT<T>::V* __restrict__ in,
-                                                           typename CT<T>::V* __restrict__ out,
-                                                           const double* __restrict__ scale,
-                                                           fx128* __restrict__ partial, int with_diag,
-                                                           unsigned long long* __restrict__ next_row) {
+// Entries of the wide stencil sweeps, 4 bytes each: target index inside the
+// segment : 16 | coefficient id : 15, id = ((ratio * 64 + shift) * 8 + dir) * 2
+// + sign, ratio numbering the values of sqrt(deg_t / deg_s) (stn_ratios). Rows
+// start at multiples of 4 entries, so four hops cost one 16-byte broadcast
+// load. At a trivial stabiliser the id is dir * 2 + sign and the coefficient
+// comes from the kernel's parameters (constant cache), else from a table in
+// global memory. What this buys: a load of 16 bytes by every lane occupies the
+// L1 data pipe for 4 cycles whether or not the address is the same for all
+// lanes, so a 16-byte {index, re, im} entry per hop cost as much as the 16-byte
+// gather it described (4x4 (4,5), 128 vectors: 73% of the L1 data pipe).
+constexpr int kStnMaxRatios = 32;
+constexpr int kStnCoefs = 16;  // per (ratio, shift): 8 directions x sign
+
+struct StnRatios {
+  int n;                       // number of distinct deg_t / deg_s
+  uint8_t num[kStnMaxRatios];  // deg_t, deg_s of the first pair with that ratio
+  uint8_t den[kStnMaxRatios];
+};
+
+template <typename T>
+struct CoefT;
+template <>
+struct CoefT<float> {
+  using C = float2;
+};
+template <>
+struct CoefT<double> {
+  using C = double2;
+};
+
+// One class of segments (equal stabiliser, hence equal stencil): its segments
+// are seg_ur[seg0 .. seg0 + nseg), `rows` rows each, stencil rows crb .. .
+struct StnClass {
+  int32_t seg0, nseg, rows, c0;  // c0: trivial stabiliser
+  int64_t crb;
+};
+
+// One sweep: y = diag * x + M_dn x over all segments of one row order.
+template <typename T>
+struct StnJob {
+  const typename CT<T>::V* in;
+  typename CT<T>::V* out;
+  const T* diag;  // per row, null: none
+  const int64_t* aoff;
+  const int32_t* seg_ur;
+  const int2* srow;  // per stencil row: first entry / 4, entries
+  const uint4* ent;
+  const typename CoefT<T>::C* coef;
+  const StnClass* cls;
+  int32_t ncls;
+  int32_t units;  // work units (below) of the job
+};
+template <typename T>
+struct StnJobs {
+  StnJob<T> j[2];
+  int32_t njobs;
+  typename CoefT<T>::C c0[kStnCoefs];  // class 0: +-amplitude of each direction
+};
+
+// N hops of a row (entries e): all gathers issued before the first FMA.
+template <typename T, int CPR, int G, int LPL, int N, bool C0>
+__device__ __forceinline__ void stn_hops(const uint32_t* e, const StnJobs<T>& P, const typename CoefT<T>::C* coef,
+                                         const typename CT<T>::V* __restrict__ xs, typename CT<T>::V (&acc)[LPL]) {
+  using V = typename CT<T>::V;
+  V x[N][LPL];
+#pragma unroll
+  for (int u = 0; u < N; ++u)
+#pragma unroll
+    for (int l = 0; l < LPL; ++l) x[u][l] = __ldg(xs + static_cast<uint64_t>(e[u] & 0xFFFFu) * CPR + l * G);
+  typename CoefT<T>::C c[N];
+#pragma unroll
+  for (int u = 0; u < N; ++u) {
+    if constexpr (C0) c[u] = P.c0[e[u] >> 16];
+    else c[u] = __ldg(coef + (e[u] >> 16));
+  }
+#pragma unroll
+  for (int u = 0; u < N; ++u)
+#pragma unroll
+    for (int l = 0; l < LPL; ++l) cfma<T>(acc[l], c[u].x, c[u].y, x[u][l]);
+}
+
+// All hops of a row, U (4 or 8) at a time, then the remainder.
+template <typename T, int CPR, int G, int LPL, int U, bool C0>
+__device__ __forceinline__ void stn_row(const uint4* q, int left, const StnJobs<T>& P,
+                                        const typename CoefT<T>::C* coef, const typename CT<T>::V* __restrict__ xs,
+                                        typename CT<T>::V (&acc)[LPL]) {
+  uint4 p = __ldg(q);
+  if constexpr (U == 8) {
+    while (left >= 8) {
+      const uint4 p2 = __ldg(q + 1);
+      const uint32_t e[8] = {p.x, p.y, p.z, p.w, p2.x, p2.y, p2.z, p2.w};
+      q += 2;
+      p = __ldg(q);
+      stn_hops<T, CPR, G, LPL, 8, C0>(e, P, coef, xs, acc);
+      left -= 8;
+    }
+  }
+  while (left >= 4) {
+    const uint32_t e[4] = {p.x, p.y, p.z, p.w};
+    p = __ldg(++q);
+    stn_hops<T, CPR, G, LPL, 4, C0>(e, P, coef, xs, acc);
+    left -= 4;
+  }
+  const uint32_t e[3] = {p.x, p.y, p.z};
+  if (left == 1) stn_hops<T, CPR, G, LPL, 1, C0>(e, P, coef, xs, acc);
+  else if (left == 2) stn_hops<T, CPR, G, LPL, 2, C0>(e, P, coef, xs, acc);
+  else if (left == 3) stn_hops<T, CPR, G, LPL, 3, C0>(e, P, coef, xs, acc);
+}
+
+__device__ __forceinline__ void stn_finish(float4& y, const float4& x, float d, double* dot) {
+  y.x = fmaf(d, x.x, y.x);
+  y.y = fmaf(d, x.y, y.y);
+  y.z = fmaf(d, x.z, y.z);
+  y.w = fmaf(d, x.w, y.w);
+  dot[0] += static_cast<double>(x.x) * y.x + static_cast<double>(x.y) * y.y;
+  dot[1] += static_cast<double>(x.z) * y.z + static_cast<double>(x.w) * y.w;
+}
+__device__ __forceinline__ void stn_finish(double2& y, const double2& x, double d, double* dot) {
+  y.x = fma(d, x.x, y.x);
+  y.y = fma(d, x.y, y.y);
+  dot[0] += x.x * y.x + x.y * y.y;
+}
+
+// The segment sweeps on the class stencils, one launch for both row orders.
+//
+// All segments of a class have the same stencil, so a warp takes one stencil
+// row for 32/G segments at once (G lanes of LPL 16-byte chunks per segment):
+// the row's entries are warp-uniform (one broadcast load per four hops, no
+// shuffles, no divergence, no partial sums to fold) whatever the sweep's
+// width. A work unit is kStnRows stencil rows, kStnLane apart, of one group of
+// segments; kStnLane consecutive units cover kStnLane * kStnRows consecutive
+// rows. A CTA takes one unit per warp, consecutive ones, from a shared counter,
+// so at any moment its warps are on neighbouring rows, which share gather
+// targets (hops among the low sites stay within a few hundred rows): a quarter
+// of the gathered sectors hit L1.
+//
+// Bound: the L1 data pipe (68% busy) and L2 reads (12.5 TB/s) together; a hop
+// costs 4 LPL + 1 cycles of the pipe for 512 LPL bytes. Per H*V, both sweeps,
+// against one warp per row with shuffled entries and one launch per sweep:
+// 4x4 (8,8) k=0 128 FP32 vectors 34.8 -> 22.3 ms, 64 vectors 20.5 -> 11.1,
+// 6x3 (5,5) 16 vectors 5.27 -> 1.78, 4x4 (4,4) 8 FP64 vectors 0.283 -> 0.119,
+// 4x4 (5,6) 128 FP64 vectors 11.7 -> 7.4 (17-20 TB/s of gathered bytes).
+//
+// y is NOT scaled (the Lanczos update applies the scale of the unnormalised
+// vectors). The dot terms Re<x, y> of a unit are summed in FP64 in row order,
+// scaled by scale^2 and added as 128-bit integers: neither the grid, the CTA
+// shape nor the assignment of units changes the sum.
+constexpr int kStnRows = 8;
+constexpr int kStnLane = 8;
+// Units of one group of segments of `rows` rows.
+__host__ __device__ __forceinline__ unsigned int stn_chunks(int64_t rows) {
+  const int64_t full = rows / (kStnLane * kStnRows), rest = rows % (kStnLane * kStnRows);
+  return static_cast<unsigned int>(full * kStnLane + (rest < kStnLane ? rest : kStnLane));
+}
+
+template <typename T, int NV, int LPL, int U, int NT, int MINB>
+__global__ void __launch_bounds__(NT, MINB) k_hv_stn(const __grid_constant__ StnJobs<T> P,
+                                                     const double* __restrict__ scale, fx128* __restrict__ partial,
+                                                     unsigned int* __restrict__ next_item) {
   using V = typename CT<T>::V;
   constexpr int VPL = CT<T>::VPL;
   constexpr int CPR = NV / VPL;
-  constexpr int G = CPR < 32 ? CPR : 32;
-  constexpr int LPL = CPR / G;
-  __shared__ double s_ph[2][64];
-  __shared__ double s_amp[2][8];
-  __shared__ double s_sq[65];
-  __shared__ double s_sc[NV];  // vector scales, read at the end of a row (keeps registers for gathers)
-  __shared__ fx128 s_acc[kHvWarps][NV];
-  const Geom& g = P.g;
-  const BlockView<W>& v = P.v;
+  constexpr int G = CPR / LPL;   // lanes per segment
+  constexpr int RPW = 32 / G;    // segments per warp
+  constexpr int NW = NT / 32;
+  __shared__ double s_dot[2][NW][RPW * NV];
+  __shared__ unsigned int s_item[2];
   const int tid = threadIdx.x;
-  for (int i = tid; i < 64; i += kHvThreads) {
-    s_ph[0][i] = v.phase_re[i];
-    s_ph[1][i] = v.phase_im[i];
-  }
-  if (tid < 8) {
-    s_amp[0][tid] = g.amp_re[tid];
-    s_amp[1][tid] = g.amp_im[tid];
-  }
-  if (tid < 65) s_sq[tid] = g.sqrt_deg[tid];
-  for (int i = tid; i < NV; i += kHvThreads) s_sc[i] = scale ? scale[i] : 1.0;
-  for (int i = tid; i < kHvWarps * NV; i += kHvThreads) s_acc[i / NV][i % NV] = 0;
-  __syncthreads();
   const int lane = tid & 31;
   const int wid = tid >> 5;
   const int grp = lane / G;
   const int sub = lane % G;
-  const int64_t nwarps = static_cast<int64_t>(gridDim.x) * kHvWarps;
-  int64_t grab = 0, grab_end = 0;
-  int64_t row = static_cast<int64_t>(blockIdx.x) * kHvWarps + wid;
-  // lane 0 keeps the next grab in flight while the current rows are processed
-  unsigned long long pend = 0;
-  if (next_row && lane == 0) pend = atomicAdd(next_row, static_cast<unsigned long long>(kStnGrab));
-  // Re<s x, y> of the rows of one grab (kStnGrab consecutive rows starting at
-  // a multiple of kStnGrab, always in row order) summed in FP64, then added
-  // to the exact fixed-point accumulator once per grab: deterministic.
-  double gdot[LPL][VPL];
+  const unsigned int total = static_cast<unsigned int>(P.j[0].units) + (P.njobs > 1 ? P.j[1].units : 0);
+  const unsigned int nitems = (total + NW - 1) / NW;
+  fx128 facc = 0;  // column tid of the dot product
+  const double sc = scale && tid < NV ? scale[tid] : 1.0;
+  int jb = 0, cl = 0;
+  unsigned int cbase = 0;  // first unit of class cl of job jb
+  unsigned int item = blockIdx.x;
+  if (next_item) {
+    if (tid == 0) s_item[1] = atomicAdd(next_item, 1u);
+    __syncthreads();
+    item = s_item[1];
+  }
+  for (int it = 0; item < nitems; ++it) {
+    unsigned int nxt = item + gridDim.x;
+    if (next_item && tid == 0) nxt = atomicAdd(next_item, 1u);
+    const unsigned int unit = item * NW + wid;
+    double dot[LPL][VPL];
 #pragma unroll
-  for (int l = 0; l < LPL; ++l)
+    for (int l = 0; l < LPL; ++l)
 #pragma unroll
-    for (int e = 0; e < VPL; ++e) gdot[l][e] = 0.0;
-  while (true) {
-    if (next_row) {
-      if (grab >= grab_end) {
-        grab = static_cast<int64_t>(__shfl_sync(0xffffffffu, pend, 0));
-        grab_end = min(grab + kStnGrab, v.dim);
-        if (lane == 0 && grab < v.dim) pend = atomicAdd(next_row, static_cast<unsigned long long>(kStnGrab));
+      for (int e = 0; e < VPL; ++e) dot[l][e] = 0.0;
+    if (unit < total) {
+      // units grow monotonically, so job and class only move forward
+      unsigned int ju = unit;
+      if (ju >= static_cast<unsigned int>(P.j[0].units)) {
+        ju -= P.j[0].units;
+        if (jb == 0) {
+          jb = 1;
+          cl = 0;
+          cbase = 0;
+        }
       }
-      row = grab++;
-    }
-    if (row >= v.dim) break;
-    const uint32_t meta = __ldg(v.row_meta + row);
-    const uint32_t ur = meta & 0x3FFFFFFu;
-    const double inv_s = 1.0 / s_sq[static_cast<int>(meta >> 26) + 1];
-    const int64_t seg = __ldg(v.aoff + ur);
-    const int64_t cr = __ldg(crb + __ldg(v.ur_class + ur)) + (row - seg);
-    const int h0 = __ldg(srp + cr), h1 = __ldg(srp + cr + 1);
-    V acc[LPL];
-#pragma unroll
-    for (int l = 0; l < LPL; ++l) vzero(acc[l]);
-    for (int b = h0; b < h1; b += 32) {
-      const int q = b + lane;
-      int64_t col = -1;
-      T cr_ = 0, ci = 0;
-      if (q < h1) {
-        const uint32_t e = __ldg(sent + q);
-        col = seg + static_cast<int64_t>(e & 0xFFFFu);
-        const int dir = static_cast<int>((e >> 16) & 7);
-        const int p = static_cast<int>((e >> 19) & 1);
-        const int shift = static_cast<int>((e >> 20) & 63);
-        const int deg_t = static_cast<int>((e >> 26) & 63) + 1;
-        const double ar = p ? -s_amp[0][dir] : s_amp[0][dir];
-        const double ai = p ? -s_amp[1][dir] : s_amp[1][dir];
-        const double pr = s_ph[0][shift], pi = s_ph[1][shift];
-        const double ratio = s_sq[deg_t] * inv_s;
-        cr_ = static_cast<T>((ar * pr - ai * pi) * ratio);
-        ci = static_cast<T>((ar * pi + ai * pr) * ratio);
+      const StnJob<T>& J = P.j[jb];
+      StnClass C = J.cls[cl];
+      unsigned int nch = stn_chunks(C.rows);
+      unsigned int cu = nch * ((C.nseg + RPW - 1) / RPW);
+      while (ju >= cbase + cu) {
+        cbase += cu;
+        C = J.cls[++cl];
+        nch = stn_chunks(C.rows);
+        cu = nch * ((C.nseg + RPW - 1) / RPW);
       }
-      gather_batch<T, NV, U>(in, col, cr_, ci, min(32, h1 - b), acc);
-    }
+      const unsigned int q = (ju - cbase) / nch;
+      const int ch = static_cast<int>(ju - cbase - q * nch);
+      const int a0 = (ch / kStnLane) * (kStnLane * kStnRows) + ch % kStnLane;
+      const int si = static_cast<int>(q) * RPW + grp;
+      const bool ok = si < C.nseg;
+      const int64_t row0 = __ldg(J.aoff + __ldg(J.seg_ur + C.seg0 + (ok ? si : C.nseg - 1)));
+      const V* xs = J.in + row0 * CPR + sub;
+      V* ys = J.out + row0 * CPR + sub;
+      const int nr = min(kStnRows, (C.rows - a0 + kStnLane - 1) / kStnLane);
+      const int2 hp = __ldg(J.srow + C.crb + a0 + kStnLane * min(lane, nr - 1));
+      for (int r = 0; r < nr; ++r) {
+        const int a = a0 + r * kStnLane;
+        const uint4* q4 = J.ent + __shfl_sync(0xffffffffu, hp.x, r);
+        const int left = __shfl_sync(0xffffffffu, hp.y, r);
+        V acc[LPL];
 #pragma unroll
-    for (int o = G; o < 32; o <<= 1)
+        for (int l = 0; l < LPL; ++l) vzero(acc[l]);
+        const T d = J.diag ? __ldg(J.diag + row0 + a) : T(0);
+        V xo[LPL];
 #pragma unroll
-      for (int l = 0; l < LPL; ++l) vadd(acc[l], shfl_xor_v(acc[l], o));
-    if (grp == 0) {
-      const double diag = with_diag ? diag_energy(__ldg(v.ur_bits + ur), __ldg(v.row_dn + row), g) : 0.0;
+        for (int l = 0; l < LPL; ++l) xo[l] = __ldg(xs + static_cast<int64_t>(a) * CPR + l * G);
+        if (C.c0) stn_row<T, CPR, G, LPL, U, true>(q4, left, P, J.coef, xs, acc);
+        else stn_row<T, CPR, G, LPL, U, false>(q4, left, P, J.coef, xs, acc);
 #pragma unroll
-      for (int l = 0; l < LPL; ++l) {
-        const V x = ld_stream(in + row * CPR + l * G + sub);
-        double sc[VPL], dt2[VPL];
-#pragma unroll
-        for (int e = 0; e < VPL; ++e) sc[e] = s_sc[(l * G + sub) * VPL + e];
-        st_stream(out + row * CPR + l * G + sub, finish_row(x, acc[l], diag, sc, dt2));
-#pragma unroll
-        for (int e = 0; e < VPL; ++e) gdot[l][e] += dt2[e];
+        for (int l = 0; l < LPL; ++l) {
+          stn_finish(acc[l], xo[l], d, dot[l]);
+          if (ok) st_stream(ys + static_cast<int64_t>(a) * CPR + l * G, acc[l]);
+        }
       }
-      if (partial && (!next_row || grab >= grab_end)) {  // end of a grab (every row when grid-stride)
+      if (!ok)
 #pragma unroll
         for (int l = 0; l < LPL; ++l)
 #pragma unroll
-          for (int e = 0; e < VPL; ++e) {
-            s_acc[wid][(l * G + sub) * VPL + e] += fx_of(gdot[l][e]);
-            gdot[l][e] = 0.0;
-          }
-      }
+          for (int e = 0; e < VPL; ++e) dot[l][e] = 0.0;
     }
-    if (!next_row) row += nwarps;
+    if (partial) {
+#pragma unroll
+      for (int l = 0; l < LPL; ++l)
+#pragma unroll
+        for (int e = 0; e < VPL; ++e) s_dot[it & 1][wid][grp * NV + (l * G + sub) * VPL + e] = dot[l][e];
+    }
+    if (tid == 0) s_item[it & 1] = nxt;
+    __syncthreads();
+    item = s_item[it & 1];
+    if (partial && tid < NV) {
+#pragma unroll
+      for (int w = 0; w < NW; ++w)
+#pragma unroll
+        for (int g = 0; g < RPW; ++g) facc += fx_of(sc * (sc * s_dot[it & 1][w][g * NV + tid]));
+    }
   }
-  flush_dot<NV>(s_acc, partial);
+  if (partial && tid < NV) partial[static_cast<int64_t>(blockIdx.x) * NV + tid] = facc;
 }
 
 // Narrow sweeps (rows of at most 4 chunks: <= 8 FP32 / 4 FP64 vectors) on the
@@ -631,17 +773,14 @@ void launch_seg_t(Ctx& c, Ctx& t, const void* in, void* out, const double* scale
         return;
       }
     }
-    k_hv_stn<W, T, NV, U, MINB><<<grid, kHvThreads, 0, c.stream>>>(
-        P, t.stn_crb.as<int64_t>(), t.stn_rp32.as<int32_t>(), t.stn_ent.as<uint32_t>(), static_cast<const V*>(in),
-        static_cast<V*>(out), scale, partial, with_diag ? 1 : 0, next_row);
-    return;
+    throw Error(FTLM_ERR_INTERNAL, "wide stencil sweeps are launched by launch_stn");
   }
   const R* gb = sizeof(R) == 4 ? reinterpret_cast<const R*>(c.binom32.p) : reinterpret_cast<const R*>(c.binom.p);
   k_hv_seg<W, R, T, NV, U, MINB><<<grid, kHvThreads, 0, c.stream>>>(P, static_cast<const V*>(in), static_cast<V*>(out),
                                                                     scale, partial, gb, with_diag ? 1 : 0, next_row);
 }
 
-// Variants (gather unroll U, CTAs per SM), as for k_hv; each runs one wave
+// Variants of k_hv_seg (gather unroll U, CTAs per SM), as for k_hv; each runs one wave
 // of sm_count x CTAs-per-SM CTAs (the grid does not change the results: the
 // dot partials are exact fixed-point sums).
 constexpr int kSegVariants = 5;
@@ -703,6 +842,117 @@ void launch_seg(Ctx& c, Ctx& t, int var, const void* in, void* out, int nv, bool
   FTLM_LAUNCH_CHECK();
 }
 
+// ---- wide stencil sweeps
+template <typename T>
+StnJob<T> stn_job(Ctx& t, const void* in, void* out, bool with_diag, int rpw) {
+  StnJob<T> j;
+  j.in = static_cast<const typename CT<T>::V*>(in);
+  j.out = static_cast<typename CT<T>::V*>(out);
+  j.diag = with_diag ? t.stn_diag.as<T>() : nullptr;
+  j.aoff = t.blk.aoff.as<int64_t>();
+  j.seg_ur = t.stn_seg.as<int32_t>();
+  j.srow = t.stn_row.as<int2>();
+  j.ent = t.stn_ent4.as<uint4>();
+  j.coef = t.stn_coef.as<typename CoefT<T>::C>();
+  j.cls = t.stn_cls.as<StnClass>();
+  j.ncls = static_cast<int32_t>(t.stn_classes.size() / 2);
+  int64_t units = 0;
+  for (size_t k = 0; k + 1 < t.stn_classes.size(); k += 2)
+    units += stn_chunks(t.stn_classes[k + 1]) * ((t.stn_classes[k] + rpw - 1) / rpw);
+  j.units = static_cast<int32_t>(units);
+  return j;
+}
+
+struct StnSweep {  // the two sweeps of one H*V: block order (with the diagonal), flipped order
+  Ctx* t[2];
+  const void* in[2];
+  void* out[2];
+  int n;
+};
+
+template <typename T, int NV, int LPL, int U, int NT, int MINB>
+int launch_stn_t(Ctx& c, const StnSweep& w, const double* scale, fx128* partial, unsigned int* counter) {
+  constexpr int RPW = 32 / (NV / CT<T>::VPL / LPL);
+  StnJobs<T> P;
+  P.njobs = w.n;
+  for (int k = 0; k < kStnCoefs; ++k) {  // shift 0 (phase 1), ratio 1
+    const double sg = k & 1 ? -1.0 : 1.0;
+    P.c0[k].x = static_cast<T>(sg * c.geom.amp_re[k / 2]);
+    P.c0[k].y = static_cast<T>(sg * c.geom.amp_im[k / 2]);
+  }
+  int64_t units = 0;
+  for (int i = 0; i < w.n; ++i) {
+    P.j[i] = stn_job<T>(*w.t[i], w.in[i], w.out[i], i == 0, RPW);
+    units += P.j[i].units;
+  }
+  const int64_t items = (units + NT / 32 - 1) / (NT / 32);
+  const int grid = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(items, int64_t(c.sm_count) * MINB)));
+  // the rest of the SM's 228 KB serves as L1, where most of the gather reuse is
+  constexpr size_t kSmem = 2 * sizeof(double) * NT * LPL * CT<T>::VPL + 2048;
+  constexpr int kCarve = static_cast<int>((kSmem * MINB * 100 + 228 * 1024 - 1) / (228 * 1024));
+  FTLM_CUDA(cudaFuncSetAttribute(k_hv_stn<T, NV, LPL, U, NT, MINB>, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                 kCarve));
+  k_hv_stn<T, NV, LPL, U, NT, MINB><<<grid, NT, 0, c.stream>>>(P, scale, partial, counter);
+  return grid;
+}
+
+// Variants: chunks per lane (more amortise the entry load, fewer leave
+// registers for warps), gathers in flight, CTA shape. All sum a row's hops in
+// the same order. Fastest on B200: 1 or 4 for rows of 256 bytes and more, 2 or
+// 3 below.
+template <typename T, int NV>
+int launch_stn_var(Ctx& c, int var, const StnSweep& w, const double* scale, fx128* partial, unsigned int* nr) {
+  constexpr int CPR = NV / CT<T>::VPL;
+  constexpr int L0 = CPR > 32 ? CPR / 32 : 1;
+  constexpr int L1 = CPR >= 16 && CPR <= 32 ? 2 : L0;
+  switch (var) {
+    case 0: return launch_stn_t<T, NV, L1, 4, 256, 3>(c, w, scale, partial, nr);
+    case 1: return launch_stn_t<T, NV, L1, 8, 256, 2>(c, w, scale, partial, nr);
+    case 2: return launch_stn_t<T, NV, L0, 8, 256, 3>(c, w, scale, partial, nr);
+    case 3: return launch_stn_t<T, NV, L0, 4, 256, 4>(c, w, scale, partial, nr);
+    case 4: return launch_stn_t<T, NV, L1, 8, 512, 1>(c, w, scale, partial, nr);
+    default: break;
+  }
+  throw Error(FTLM_ERR_ARG, "bad H*V kernel variant");
+}
+
+template <typename T>
+int launch_stn_nv(Ctx& c, int var, const StnSweep& w, int nv, const double* scale, fx128* partial, unsigned int* nr) {
+  switch (nv) {
+    case 1:
+      if constexpr (sizeof(T) == 8) return launch_stn_var<T, 1>(c, var, w, scale, partial, nr);
+      break;
+    case 2: return launch_stn_var<T, 2>(c, var, w, scale, partial, nr);
+    case 4: return launch_stn_var<T, 4>(c, var, w, scale, partial, nr);
+    case 8: return launch_stn_var<T, 8>(c, var, w, scale, partial, nr);
+    case 16: return launch_stn_var<T, 16>(c, var, w, scale, partial, nr);
+    case 32: return launch_stn_var<T, 32>(c, var, w, scale, partial, nr);
+    case 64: return launch_stn_var<T, 64>(c, var, w, scale, partial, nr);
+    case 128: return launch_stn_var<T, 128>(c, var, w, scale, partial, nr);
+    default: break;
+  }
+  throw Error(FTLM_ERR_ARG, "unsupported vectors per sweep: " + std::to_string(nv));
+}
+
+// Returns the grid, which is the number of rows of dot partials.
+int launch_stn(Ctx& c, int var, const StnSweep& w, int nv, bool fp32, const double* scale, fx128* partial) {
+  unsigned int* nr = nullptr;
+  if (c.seg_dynamic) {
+    c.seg_counter.ensure(sizeof(unsigned long long) * 4);
+    nr = c.seg_counter.as<unsigned int>();
+    FTLM_CUDA(cudaMemsetAsync(nr, 0, sizeof(unsigned int), c.stream));
+  }
+  const int grid = fp32 ? launch_stn_nv<float>(c, var, w, nv, scale, partial, nr)
+                        : launch_stn_nv<double>(c, var, w, nv, scale, partial, nr);
+  FTLM_LAUNCH_CHECK();
+  return grid;
+}
+
+// Whether sweeps of nv vectors over block c run the wide stencil kernel.
+bool stn_wide(const Ctx& c, int nv, bool fp32) {
+  return c.split_stencil && c.stn_ok && !(c.stn_rows && (fp32 ? nv / 2 : nv) <= 4);
+}
+
 int seg_grid(const Ctx& c, int var) {
   const int64_t by_rows = (c.blk.dim + kHvWarps - 1) / kHvWarps;
   const int64_t cap = static_cast<int64_t>(c.sm_count) * kSegMinB[var];
@@ -743,6 +993,110 @@ __global__ void k_rp_narrow(const int64_t* __restrict__ in, int32_t* __restrict_
     out[i] = static_cast<int32_t>(in[i]);
 }
 
+// ---- entries of the wide sweeps
+
+// Rounded-up entry counts (multiples of 4) for the row offsets.
+__global__ void k_stn_round(const int64_t* __restrict__ rp, int64_t rows, int32_t* __restrict__ counts) {
+  for (int64_t r = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; r < rows;
+       r += static_cast<int64_t>(gridDim.x) * blockDim.x)
+    counts[r] = static_cast<int32_t>((rp[r + 1] - rp[r] + 3) & ~int64_t(3));
+}
+
+// The wide sweeps' entries from the packed ones, same order.
+__global__ void k_stn_wide(int64_t rows, const int64_t* __restrict__ rp, const uint32_t* __restrict__ ent,
+                           const uint8_t* __restrict__ row_deg, const __grid_constant__ StnRatios R,
+                           const int64_t* __restrict__ rp4, int2* __restrict__ srow, uint32_t* __restrict__ out) {
+  for (int64_t r = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; r < rows;
+       r += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+    const int64_t h0 = rp[r];
+    const int n = static_cast<int>(rp[r + 1] - h0), ds = row_deg[r];
+    uint32_t* o = out + rp4[r];
+    for (int k = 0; k < n; ++k) {
+      const uint32_t e = ent[h0 + k];
+      const int dt = static_cast<int>(e >> 26) + 1;
+      uint32_t ratio = 0;
+      while (R.num[ratio] * ds != R.den[ratio] * dt) ++ratio;
+      const uint32_t id = ((ratio * 64 + ((e >> 20) & 63u)) * 8 + ((e >> 16) & 7u)) * 2 + ((e >> 19) & 1u);
+      o[k] = (e & 0xFFFFu) | (id << 16);
+    }
+    srow[r] = make_int2(static_cast<int>(rp4[r] / 4), n);
+  }
+}
+
+__global__ void k_stn_coef(const __grid_constant__ Geom g, const __grid_constant__ FlipPhase ph,
+                           const __grid_constant__ StnRatios R, float2* __restrict__ c32, double2* __restrict__ c64) {
+  const int id = blockIdx.x * blockDim.x + threadIdx.x;
+  if (id >= R.n * 64 * kStnCoefs) return;
+  const int dir = (id >> 1) & 7, h = (id >> 4) & 63, ratio = id >> 10;
+  double re = 0.0, im = 0.0;
+  if (h < g.n) {
+    const double q = g.sqrt_deg[R.num[ratio]] * (1.0 / g.sqrt_deg[R.den[ratio]]);
+    re = (g.amp_re[dir] * ph.re[h] - g.amp_im[dir] * ph.im[h]) * q;
+    im = (g.amp_re[dir] * ph.im[h] + g.amp_im[dir] * ph.re[h]) * q;
+    if (id & 1) {
+      re = -re;
+      im = -im;
+    }
+  }
+  if (c32) c32[id] = make_float2(static_cast<float>(re), static_cast<float>(im));
+  else c64[id] = make_double2(re, im);
+}
+
+// Stabiliser size of every stencil row.
+__global__ void k_stn_deg(int nclass, const int64_t* __restrict__ crb, int64_t c_dn,
+                          const uint32_t* __restrict__ act_list, const uint64_t* __restrict__ dtab, int64_t rows,
+                          uint8_t* __restrict__ deg) {
+  for (int64_t r = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; r < rows;
+       r += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+    int c = 0;
+    while (c + 1 < nclass && crb[c + 1] <= r) ++c;
+    const int64_t base = static_cast<int64_t>(c - 1) * c_dn;
+    deg[r] = c == 0 ? 1 : static_cast<uint8_t>((dtab[base + act_list[base + (r - crb[c])]] >> 48) & 0xFF);
+  }
+}
+
+// The distinct values of deg_t / deg_s: orbit stabilisers are subgroups, so
+// both divide the number of sites. False when there are more than the entry
+// format numbers (a lattice with three prime factors such as 60 sites).
+bool stn_ratios(int n, StnRatios& R) {
+  R.n = 0;
+  for (int dt = 1; dt <= n; ++dt)
+    for (int ds = 1; ds <= n; ++ds) {
+      if (n % dt || n % ds) continue;
+      bool known = false;
+      for (int k = 0; k < R.n; ++k) known = known || R.num[k] * ds == R.den[k] * dt;
+      if (known) continue;
+      if (R.n == kStnMaxRatios) return false;
+      R.num[R.n] = static_cast<uint8_t>(dt);
+      R.den[R.n] = static_cast<uint8_t>(ds);
+      ++R.n;
+    }
+  return true;
+}
+
+bool stn_wide_build(Ctx& c, Ctx& t, int64_t rows) {
+  StnRatios R;
+  if (!stn_ratios(c.geom.n, R)) return false;
+  const int grid = grid_rows(rows, 128);
+  k_stn_round<<<grid, 128, 0, c.stream>>>(t.stn_rp.as<int64_t>(), rows, t.stn_cnt.as<int32_t>());
+  t.stn_rp4.ensure(sizeof(int64_t) * (rows + 1));
+  const int64_t total = scan_excl_i32_to_i64(c, t.stn_cnt.as<int32_t>(), t.stn_rp4.as<int64_t>(), rows);
+  t.stn_ent4.ensure(sizeof(uint32_t) * (total + 8));  // sweeps read up to two quads past a row
+  t.stn_row.ensure(sizeof(int2) * std::max<int64_t>(rows, 1));
+  t.stn_deg.ensure(std::max<int64_t>(rows, 1));
+  k_stn_deg<<<grid, 128, 0, c.stream>>>(t.sec.nclass, t.stn_crb.as<int64_t>(), t.sec.c_dn, t.blk.act_list.as<uint32_t>(),
+                                        t.blk.dtab.as<uint64_t>(), rows, t.stn_deg.as<uint8_t>());
+  k_stn_wide<<<grid, 128, 0, c.stream>>>(rows, t.stn_rp.as<int64_t>(), t.stn_ent.as<uint32_t>(), t.stn_deg.as<uint8_t>(),
+                                         R, t.stn_rp4.as<int64_t>(), t.stn_row.as<int2>(), t.stn_ent4.as<uint32_t>());
+  const bool fp32 = c.opts.precision == FTLM_PREC_MIXED;
+  t.stn_coef.ensure((fp32 ? sizeof(float2) : sizeof(double2)) * R.n * 64 * kStnCoefs);
+  k_stn_coef<<<R.n * 8, 128, 0, c.stream>>>(c.geom, flip_phase(t), R, fp32 ? t.stn_coef.as<float2>() : nullptr,
+                                            fp32 ? nullptr : t.stn_coef.as<double2>());
+  FTLM_LAUNCH_CHECK();
+  c.prof.kernel_launches += 4;
+  return true;
+}
+
 // Class stencils of the prepared block of tables t (its own sector and
 // block); false when a class has more than kStencilMaxRows rows.
 template <typename W>
@@ -771,6 +1125,27 @@ bool stencil_build_t(Ctx& c, Ctx& t) {
                                            B.act_list.as<uint32_t>(), B.dtab.as<uint64_t>(), S.dns.as<W>(),
                                            c.binom.as<uint64_t>(), rows, nullptr, t.stn_rp.as<int64_t>(),
                                            t.stn_ent.as<uint32_t>());
+  if (!stn_wide_build(c, t, rows)) return false;
+  // segments by class, and the classes that have rows in this block
+  std::vector<int32_t> seg(S.nur);
+  std::vector<int64_t> first(S.nclass + 1, 0);
+  for (int64_t u = 0; u < S.nur; ++u) ++first[S.h_ur_class[u] + 1];
+  for (int k = 0; k < S.nclass; ++k) first[k + 1] += first[k];
+  std::vector<int64_t> at(first.begin(), first.end() - 1);
+  for (int64_t u = 0; u < S.nur; ++u) seg[at[S.h_ur_class[u]]++] = static_cast<int32_t>(u);
+  std::vector<StnClass> cls;
+  t.stn_classes.clear();
+  for (int k = 0; k < S.nclass; ++k) {
+    const int64_t nseg = first[k + 1] - first[k], nrow = crb[k + 1] - crb[k];
+    if (nseg == 0 || nrow == 0) continue;
+    cls.push_back({static_cast<int32_t>(first[k]), static_cast<int32_t>(nseg), static_cast<int32_t>(nrow), k == 0 ? 1 : 0, crb[k]});
+    t.stn_classes.push_back(nseg);
+    t.stn_classes.push_back(nrow);
+  }
+  t.stn_seg.ensure(sizeof(int32_t) * std::max<int64_t>(S.nur, 1));
+  t.stn_cls.ensure(sizeof(StnClass) * std::max<size_t>(cls.size(), 1));
+  FTLM_CUDA(cudaMemcpyAsync(t.stn_seg.p, seg.data(), sizeof(int32_t) * seg.size(), cudaMemcpyHostToDevice, c.stream));
+  FTLM_CUDA(cudaMemcpyAsync(t.stn_cls.p, cls.data(), sizeof(StnClass) * cls.size(), cudaMemcpyHostToDevice, c.stream));
   // row offsets as int32 for the sweeps (fewer registers per row)
   t.stn_rp32.ensure(sizeof(int32_t) * (rows + 1));
   k_rp_narrow<<<grid_rows(rows + 1, 256), 256, 0, c.stream>>>(t.stn_rp.as<int64_t>(), t.stn_rp32.as<int32_t>(),
@@ -781,12 +1156,43 @@ bool stencil_build_t(Ctx& c, Ctx& t) {
   return true;
 }
 
+// Diagonal energy of every row of the prepared block, in the sweeps' type.
+template <typename W, typename T>
+__global__ void k_row_diag(const __grid_constant__ HvParams<W> P, T* __restrict__ diag) {
+  const BlockView<W>& v = P.v;
+  for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < v.dim;
+       i += static_cast<int64_t>(gridDim.x) * blockDim.x)
+    diag[i] = static_cast<T>(diag_energy(v.ur_bits[v.row_meta[i] & 0x3FFFFFFu], v.row_dn[i], P.g));
+}
+
+template <typename W>
+void row_diag_build(Ctx& c) {
+  HvParams<W> P;
+  P.g = c.geom;
+  if constexpr (sizeof(W) == 4) P.v = view32(c);
+  else P.v = view64(c);
+  const int64_t D = c.blk.dim;
+  if (c.opts.precision == FTLM_PREC_MIXED) {
+    c.stn_diag.ensure(sizeof(float) * D);
+    k_row_diag<W, float><<<grid_rows(D, 256), 256, 0, c.stream>>>(P, c.stn_diag.as<float>());
+  } else {
+    c.stn_diag.ensure(sizeof(double) * D);
+    k_row_diag<W, double><<<grid_rows(D, 256), 256, 0, c.stream>>>(P, c.stn_diag.as<double>());
+  }
+  FTLM_LAUNCH_CHECK();
+  c.prof.kernel_launches += 1;
+}
+
 // Stencils of tables t for its prepared block, built once per (sector
 // generation, block).
 void stencil_prepare(Ctx& c, Ctx& t) {
   const int64_t key[3] = {t.sec_gen, t.blk.mx, t.blk.my};
   if (std::memcmp(key, t.stn_for, sizeof key) == 0) return;
   t.stn_ok = c.wide ? stencil_build_t<uint64_t>(c, t) : stencil_build_t<uint32_t>(c, t);
+  if (t.stn_ok && &t == &c) {
+    if (c.wide) row_diag_build<uint64_t>(c);
+    else row_diag_build<uint32_t>(c);
+  }
   std::memcpy(t.stn_for, key, sizeof key);
 }
 
@@ -868,15 +1274,21 @@ int seg_variant(Ctx& c, const void* in, void* out, int nv, bool fp32) {
   FTLM_CUDA(cudaEventCreate(&e0));
   FTLM_CUDA(cudaEventCreate(&e1));
   // best of 3 single-launch timings per variant, variants interleaved
+  const bool wide = stn_wide(c, nv, fp32);
+  const StnSweep one{{&c, nullptr}, {in, nullptr}, {out, nullptr}, 1};
+  auto run = [&](int v) {
+    if (wide) launch_stn(c, v, one, nv, fp32, nullptr, nullptr);
+    else launch_seg(c, c, v, in, out, nv, fp32, nullptr, nullptr, seg_grid(c, v), true, 0);
+  };
   float best_ms[kSegVariants];
   for (int v = 0; v < kSegVariants; ++v) {
     best_ms[v] = 1e30f;
-    launch_seg(c, c, v, in, out, nv, fp32, nullptr, nullptr, seg_grid(c, v), true, 0);  // warm
+    run(v);  // warm
   }
   for (int rep = 0; rep < 3; ++rep)
     for (int v = 0; v < kSegVariants; ++v) {
       FTLM_CUDA(cudaEventRecord(e0, c.stream));
-      launch_seg(c, c, v, in, out, nv, fp32, nullptr, nullptr, seg_grid(c, v), true, 0);
+      run(v);
       FTLM_CUDA(cudaEventRecord(e1, c.stream));
       FTLM_CUDA(cudaEventSynchronize(e1));
       float ms = 0.f;
@@ -899,6 +1311,12 @@ int hv_apply_split(Ctx& c, const void* in, const void* in_d, void* out, void* ou
   Ctx& f = flipped_tables(c);
   const int var = seg_variant(c, in, out, nv, fp32);
   c.prof.hv_variant = var;
+  if (stn_wide(c, nv, fp32)) {
+    const StnSweep both{{&c, &f}, {in, in_d}, {out, out_d}, 2};
+    const int rows = launch_stn(c, var, both, nv, fp32, scale, partial);
+    c.prof.kernel_launches += 1;
+    return rows;
+  }
   const int grid = seg_grid(c, var);
   // flipped sweep first: its partials follow this block's in the array
   launch_seg(c, f, var, in_d, out_d, nv, fp32, scale, partial ? partial + static_cast<int64_t>(grid) * nv : nullptr,
@@ -907,6 +1325,8 @@ int hv_apply_split(Ctx& c, const void* in, const void* in_d, void* out, void* ou
   c.prof.kernel_launches += 2;
   return 2 * grid;
 }
+
+bool hv_split_unscaled(const Ctx& c, int nv, bool fp32) { return stn_wide(c, nv, fp32); }
 
 int hv_split_max_grid(const Ctx& c) { return 2 * c.sm_count * 4; }
 
