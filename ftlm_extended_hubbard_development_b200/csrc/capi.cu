@@ -194,17 +194,25 @@ void ftlm_ctx_destroy(ftlm_ctx* ctx) {
   Ctx& c = ctx->c;
   cudaSetDevice(c.device);
   if (c.stream) cudaStreamSynchronize(c.stream);
+  for (cudaStream_t s : c.side)
+    if (s) {
+      cudaStreamSynchronize(s);
+      cudaStreamDestroy(s);
+    }
+  if (c.side_ev) cudaEventDestroy(c.side_ev);
   ftlm::DBuf* bufs[] = {&c.binom, &c.binom32, &c.sec.ups, &c.sec.dns, &c.sec.up_info, &c.sec.ur_bits,
                         &c.sec.ur_class, &c.sec.ur_poff, &c.sec.d_star, &c.sec.d_hs, &c.sec.d_stab,
                         &c.sec.d_chi, &c.sec.d_cidx, &c.sec.canon, &c.sec.tmp_a, &c.sec.tmp_b, &c.sec.tmp_c,
                         &c.sec.tmp_d, &c.sec.tmp_e, &c.blk.act, &c.blk.act_list, &c.blk.aoff, &c.blk.dtab,
                         &c.blk.row_meta, &c.blk.row_dn, &c.vec_a, &c.vec_b, &c.vec_h, &c.partial,
                         &c.lz_alpha, &c.lz_beta, &c.lz_scale, &c.lz_state, &c.host_start, &c.ritz_tmp, &c.ritz_out, &c.ritz_meta,
-                        &c.sb_rp, &c.sb_col, &c.sb_val, &c.sb_diag, &c.sb_meta, &c.sb_steps,
+                        &c.sb_ent, &c.sb_cnt, &c.sb_diag, &c.sb_start, &c.sb_meta, &c.sb_steps, &c.sb_alpha, &c.sb_beta,
+                        &c.pack.act, &c.pack.act_list, &c.pack.dtab, &c.pack.aoff, &c.pack.nact, &c.pack.dims,
+                        &c.pack.row_meta, &c.pack.row_dn, &c.pack.phase, &c.pack.items,
                         &c.scan_tmp, &c.dense_arena, &c.dense_meta, &c.dense_out, &c.spectra, &c.th_beta,
                         &c.th_mu, &c.th_state, &c.hl_ptr, &c.hl_ent, &c.flip_map, &c.vec_xd, &c.vec_yd, &c.seg_counter, &c.stn_crb, &c.stn_rp, &c.stn_rp32, &c.stn_ent, &c.stn_cnt,
                         &c.stn_rp4, &c.stn_row, &c.stn_ent4, &c.stn_deg, &c.stn_coef, &c.stn_seg, &c.stn_cls, &c.stn_diag,
-                        &c.defer_arena, &c.defer_ev, &c.defer_work, &c.defer_ab, &c.defer_st};
+                        &c.defer_arena, &c.defer_ev, &c.defer_work};
   for (auto* b : bufs) b->release();
   if (c.flipped) {
     ftlm::Ctx& f = *c.flipped;
@@ -336,7 +344,7 @@ int ftlm_block_spectrum(ftlm_ctx* ctx, int32_t mx, int32_t my, int32_t exact, do
     const auto key = std::make_pair(static_cast<int>(mx), static_cast<int>(my));
     auto it = c.spec.find(key);
     const bool have = it != c.spec.end() && it->second.exact == (exact != 0);
-    if (have && (it->second.pending >= 0 || it->second.pending_ritz >= 0)) {  // pooled: solve the pool now
+    if (have && (it->second.pending >= 0 || it->second.pending_small >= 0)) {  // pooled: solve the pool now
       ftlm::flush_deferred(c);
       it = c.spec.find(key);
     }
@@ -404,10 +412,10 @@ int ftlm_thermo_accumulate_block(ftlm_ctx* ctx, int32_t mx, int32_t my) {
     ftlm::check_k(c, mx, my);
     auto it = c.spec.find({mx, my});
     if (it == c.spec.end()) throw Error(FTLM_ERR_STATE, "block spectrum not computed");
-    if (it->second.pending >= 0 || it->second.pending_ritz >= 0) {  // accumulated when the pool is solved
+    if (it->second.pending >= 0 || it->second.pending_small >= 0) {  // accumulated when the pool is solved
       if (c.nbeta <= 0 || c.nmu <= 0) throw Error(FTLM_ERR_STATE, "thermo accumulators not configured");
-      const bool ritz = it->second.pending_ritz >= 0;
-      c.defer_acc.push_back({ritz, ritz ? it->second.pending_ritz : it->second.pending});
+      const bool small = it->second.pending_small >= 0;
+      c.defer_acc.push_back({small, small ? it->second.pending_small : it->second.pending});
       return;
     }
     ftlm::thermo_accumulate(c, it->second);

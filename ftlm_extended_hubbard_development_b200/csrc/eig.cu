@@ -24,24 +24,6 @@ namespace {
 constexpr int kEigThreads = 256;
 constexpr int kMaxDense = 7000;  // two complex work vectors in shared memory: 2*7000*16 B <= 227 KB
 
-// (M + M^H)/2 with a real diagonal (main.cpp:875-886); upper triangle
-// holds the average, the lower triangle its conjugate.
-__global__ void k_dense_herm(int64_t n, double2* __restrict__ A) {
-  for (int64_t t = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; t < n * n;
-       t += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const int64_t i = t % n, j = t / n;
-    if (i > j) continue;
-    if (i == j) {
-      A[i + i * n].y = 0.0;
-      continue;
-    }
-    const double2 a = A[i + j * n], b = A[j + i * n];
-    const double re = 0.5 * (a.x + b.x), im = 0.5 * (a.y - b.y);
-    A[i + j * n] = make_double2(re, im);
-    A[j + i * n] = make_double2(re, -im);
-  }
-}
-
 __device__ double block_sum(double v, double* red) {
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   __syncthreads();
@@ -226,17 +208,16 @@ std::vector<DenseItem> dense_items(Ctx& c, const std::vector<std::pair<int, int>
 
 // Dense Hermitian matrix of every item at arena + aoff (zeroed by the caller).
 void dense_fill(Ctx& c, const std::vector<DenseItem>& items, double2* arena, int64_t abase) {
+  std::vector<PackItem> rows;
   for (const DenseItem& it : items) {
-    // the block's rows are built in stream order; the fill reads them before
-    // the next block_prepare overwrites them
-    block_prepare(c, it.mx, it.my);
-    double2* A = arena + abase + it.aoff;
-    block_dense_device(c, A);
-    const int g2 = static_cast<int>(std::min<int64_t>((it.n * it.n + 255) / 256, 4096));
-    k_dense_herm<<<g2, 256, 0, c.stream>>>(it.n, A);
-    FTLM_LAUNCH_CHECK();
-    c.prof.kernel_launches += 1;
+    PackItem p{};
+    p.mx = it.mx;
+    p.my = it.my;
+    p.n = it.n;
+    p.off = abase + it.aoff;
+    rows.push_back(p);
   }
+  pack_dense(c, rows, arena);
 }
 
 // One k_dense_eig launch over matrices (dims, aoff into arena) writing the
@@ -371,18 +352,20 @@ void queue_exact_blocks(Ctx& c, const std::vector<std::pair<int, int>>& blocks) 
 }
 
 int64_t defer_pool_bytes(const Ctx& c) {
-  return static_cast<int64_t>(sizeof(double2)) * c.defer_asz + static_cast<int64_t>(sizeof(double)) * c.defer_ab_used +
-         static_cast<int64_t>(sizeof(int32_t)) * c.defer_st_used;
+  return static_cast<int64_t>(sizeof(double2)) * (c.defer_asz + c.sb_start_used) +
+         static_cast<int64_t>(sizeof(uint32_t)) * c.sb_ent_used +
+         static_cast<int64_t>(sizeof(int32_t) + sizeof(double)) * c.sb_row_used +
+         static_cast<int64_t>(2 * sizeof(double)) * c.sb_ab_used;
 }
 
 void flush_deferred(Ctx& c) {
   const size_t nb = c.defer_items.size();
-  const size_t nr = c.defer_ritz.size();
+  const size_t nr = c.defer_small.size();
   if (nb == 0 && nr == 0) {
     c.defer_acc.clear();
     return;
   }
-  // exact blocks: one dense-solver launch
+  // exact blocks: one dense solve
   std::vector<int64_t> eoff(nb);
   if (nb > 0) {
     std::vector<int32_t> dims(nb);
@@ -400,27 +383,23 @@ void flush_deferred(Ctx& c) {
     dense_solve(c, dims, aoff, eoff, c.defer_arena.as<double2>(), c.defer_ev.as<double>(), c.defer_work.as<double>());
     t.stop();
   }
-  // small FTLM blocks: one Ritz-stage launch; the spectra land in this
-  // sector's arena (those of earlier sectors are dropped with it later)
+  // small FTLM blocks: their Lanczos is running; one Ritz-stage launch; the spectra land
+  // in this sector's arena (those of earlier sectors are dropped with it later)
   std::vector<Spectrum> rs(nr);
   if (nr > 0) {
+    small_join(c);
     std::vector<RitzJob> jobs;
-    jobs.reserve(nr);
-    for (size_t i = 0; i < nr; ++i) {
-      const DeferRitz& d = c.defer_ritz[i];
-      jobs.push_back(RitzJob{d.R, d.R, d.ld, d.K, c.defer_ab.as<double>() + d.alpha_off,
-                             c.defer_ab.as<double>() + d.beta_off, c.defer_st.as<int32_t>() + d.steps_off, &rs[i]});
-    }
+    for (size_t i = 0; i < nr; ++i) jobs.push_back(small_ritz_job(c, c.defer_small[i].d, &rs[i]));
     ritz_stage_many(c, jobs);
     for (size_t i = 0; i < nr; ++i) {
-      rs[i].prefactor = static_cast<double>(c.defer_ritz[i].dim);
-      rs[i].particles = c.defer_ritz[i].n_up + c.defer_ritz[i].n_dn;
-      rs[i].dim = c.defer_ritz[i].dim;
+      rs[i].prefactor = static_cast<double>(c.defer_small[i].d.dim);
+      rs[i].particles = c.defer_small[i].n_up + c.defer_small[i].n_dn;
+      rs[i].dim = c.defer_small[i].d.dim;
     }
   }
   for (const DeferAcc& a : c.defer_acc) {
     const size_t i = static_cast<size_t>(a.idx);
-    if (a.ritz) {
+    if (a.small) {
       thermo_accumulate(c, rs[i]);
     } else {
       const DeferItem& d = c.defer_items[i];
@@ -440,18 +419,17 @@ void flush_deferred(Ctx& c) {
     it->second.pending = -1;
   }
   for (size_t i = 0; i < nr; ++i) {
-    const DeferRitz& d = c.defer_ritz[i];
+    const DeferSmall& d = c.defer_small[i];
     if (d.sec_gen != c.sec_gen) continue;
     auto it = c.spec.find({d.mx, d.my});
-    if (it == c.spec.end() || it->second.pending_ritz != static_cast<int>(i)) continue;
+    if (it == c.spec.end() || it->second.pending_small != static_cast<int>(i)) continue;
     it->second = rs[i];
   }
   c.defer_items.clear();
-  c.defer_ritz.clear();
+  c.defer_small.clear();
+  small_rows_reset(c);
   c.defer_acc.clear();
   c.defer_asz = 0;
-  c.defer_ab_used = 0;
-  c.defer_st_used = 0;
 }
 
 }  // namespace ftlm

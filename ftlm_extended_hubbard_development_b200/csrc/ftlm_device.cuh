@@ -229,6 +229,22 @@ __device__ __forceinline__ void philox_phase(int64_t row, int sample, uint64_t s
   im = amp * sn;
 }
 
+// Stabiliser character test of a canonical word for momentum (mx, my):
+// active iff sign(s) * exp(2 pi i (mx dx/lx + my dy/ly)) == 1 on the whole
+// stabiliser (exact integer form of the dnf > 1e-12 test, main.cpp:748-768:
+// the orbit sum of a group character is |stab| or exactly zero).
+__device__ __forceinline__ bool char_trivial(uint64_t stab, uint64_t chi, int mx, int my, const Geom& g) {
+  const int L = g.lx * g.ly;
+  for (uint64_t m = stab & ~1ULL; m; m &= m - 1) {
+    const int s = __ffsll(static_cast<long long>(m)) - 1;
+    const int q = (mx * shift_dx(s, g) * g.ly + my * shift_dy(s, g) * g.lx) % L;
+    const bool neg = (chi >> s) & 1ULL;
+    if (!neg && q != 0) return false;
+    if (neg && 2 * q != L) return false;
+  }
+  return true;
+}
+
 // Packed lookup entries.
 //  up_info: ur(32) | g0(8)<<32 | sign(1)<<40   (T_g0 maps the up
 //           representative onto this up word with that sign)

@@ -36,17 +36,20 @@ struct DBuf {
   size_t cap = 0;
   void ensure(size_t bytes) {
     if (bytes <= cap) return;
+    // small buffers grow by doubling from 64 KB: a curve over many small
+    // sectors otherwise spends its time in cudaMalloc / cudaFree
+    if (bytes <= kSmallBytes) bytes = std::max(bytes, std::max(kFirstBytes, std::min(2 * cap, kSmallBytes)));
     if (p) FTLM_CUDA(cudaFree(p));
     p = nullptr;
     cap = 0;
-    if (bytes == 0) return;
     FTLM_CUDA(cudaMalloc(&p, bytes));
     cap = bytes;
   }
+  static constexpr size_t kFirstBytes = size_t(64) << 10, kSmallBytes = size_t(16) << 20;
   // Grows (by at least half) keeping the first `cap` bytes; stream-ordered copy.
   void ensure_keep(size_t bytes, cudaStream_t stream) {
     if (bytes <= cap) return;
-    const size_t want = std::max(bytes, cap + cap / 2);
+    const size_t want = std::max(bytes, std::max(cap + cap / 2, size_t(1) << 20));
     void* q = nullptr;
     FTLM_CUDA(cudaMalloc(&q, want));
     if (p) {
@@ -138,7 +141,7 @@ struct Spectrum {
   int particles = 0;
   int64_t dim = 0;
   int pending = -1;       // exact block queued for a deferred solve: index into Ctx::defer_items
-  int pending_ritz = -1;  // small FTLM block whose Ritz stage is deferred: index into Ctx::defer_ritz
+  int pending_small = -1;  // small FTLM block whose solve is deferred: index into Ctx::defer_small
 };
 
 // An exact block whose dense matrix waits in the deferred pool.
@@ -148,18 +151,62 @@ struct DeferItem {
   int64_t sec_gen;   // sector generation it was assembled in
 };
 
-// A small FTLM block whose Lanczos coefficients wait in the deferred pool.
-struct DeferRitz {
-  int n_up, n_dn, mx, my;
-  int R, ld, K;
-  int64_t alpha_off, beta_off;  // doubles into defer_ab ([K][ld] each)
-  int64_t steps_off;            // int32 into defer_st ([R])
-  int64_t dim, sec_gen;
+// One block of a small-block Lanczos launch (smallblock.cu): offsets into the
+// context's sb_* arrays.
+struct SmallBlockDesc {
+  int64_t ent_off;    // entry k of row i at ent[ent_off + k * dim + i]
+  int64_t row_off;    // row lengths and diagonal
+  int64_t ab_off;     // alpha/beta [K][ld]
+  int64_t start_off;  // reference start vectors [R][dim] complex, -1: Philox
+  int64_t steps_off;  // steps[steps_off + r]
+  uint64_t seed;      // block seed (Philox key)
+  int32_t dim, K, ld, k;  // k: momentum index my * lx + mx
 };
 
-// A queued accumulation: an exact (ritz = false) or FTLM block of the pool.
+// A small FTLM block whose rows wait in the deferred pool.
+struct DeferSmall {
+  int n_up, n_dn, mx, my;
+  SmallBlockDesc d;
+  int64_t sec_gen;
+};
+
+// Entries of small-block rows: column : 12 | direction * 2 + parity : 4 |
+// shift : 6 | number of the orbit-size ratio deg_t / deg_s : 6.
+constexpr int kSmallRatios = 64;
+struct SmallRatios {
+  int n;
+  uint8_t num[kSmallRatios], den[kSmallRatios];  // deg_t, deg_s of the first pair with that ratio
+};
+__host__ __device__ inline uint32_t small_entry(int col, int dir, int par, int shift, int ratio) {
+  return static_cast<uint32_t>(col) | (static_cast<uint32_t>(dir * 2 + par) << 12) |
+         (static_cast<uint32_t>(shift) << 16) | (static_cast<uint32_t>(ratio) << 22);
+}
+
+// Tables of every momentum block of a small sector (pack.cu).
+struct SectorPack {
+  int64_t gen = -1;  // sector generation they belong to
+  bool ok = false;
+  std::vector<int64_t> row0;  // [n_k + 1] first row of each block
+  DBuf act, act_list, dtab, aoff, nact, dims, row_meta, row_dn;
+  DBuf phase;  // [n_k][64] complex e^{i k.s}, the context's
+  DBuf items;
+};
+
+// A block whose rows are built: dense matrix at arena + off, or entries at
+// ent + off with lengths and diagonal at off2.
+struct PackItem {
+  int32_t mx, my;
+  int64_t n, off, off2;
+  const int64_t* aoff;
+  const uint64_t* dtab;
+  const uint32_t* row_meta;
+  const void* row_dn;
+  const double* phase;
+};
+
+// A queued accumulation: an exact (small = false) or FTLM block of the pool.
 struct DeferAcc {
-  bool ritz;
+  bool small;
   int idx;
 };
 
@@ -242,18 +289,26 @@ struct Ctx {
   // exact batch
   DBuf dense_arena, dense_meta, dense_out;
   // deferred block spectra (ftlm_spectra_defer): dense matrices of exact
-  // blocks and Lanczos coefficients of small FTLM blocks of any number of
-  // sectors, solved together by flush_deferred, then the queued accumulations
+  // blocks and rows of small FTLM blocks of any number of sectors, solved
+  // together by flush_deferred, then the queued accumulations
   bool spectra_defer = false;
   DBuf defer_arena, defer_ev, defer_work;
   int64_t defer_asz = 0;
   std::vector<DeferItem> defer_items;
-  DBuf defer_ab, defer_st;
-  int64_t defer_ab_used = 0, defer_st_used = 0;
-  std::vector<DeferRitz> defer_ritz;
+  std::vector<DeferSmall> defer_small;
   std::vector<DeferAcc> defer_acc;
-  // small-block FTLM batch: CSR arenas, task list, per-vector step counts
-  DBuf sb_rp, sb_col, sb_val, sb_diag, sb_meta, sb_steps;
+  // small FTLM blocks, running or pooled: entries, row lengths, diagonals,
+  // start vectors, Lanczos coefficients, step counts, task lists. A pooled
+  // sector's Lanczos runs on a side stream while the next sectors' tables are
+  // built; the buffers move only when the side streams are idle, and c.stream
+  // waits for them before the Ritz stage.
+  DBuf sb_ent, sb_cnt, sb_diag, sb_start, sb_alpha, sb_beta, sb_steps, sb_meta;
+  int64_t sb_ent_used = 0, sb_row_used = 0, sb_start_used = 0, sb_ab_used = 0, sb_st_used = 0, sb_meta_used = 0;
+  static constexpr int kSide = 8;
+  cudaStream_t side[kSide] = {};
+  cudaEvent_t side_ev = nullptr;
+  int side_next = 0;
+  SectorPack pack;
   // spectra of the current sector's blocks (device arena)
   DBuf spectra;
   int64_t spectra_used = 0;
@@ -281,9 +336,16 @@ void block_csr(Ctx& c, std::vector<int32_t>& row_ptr, std::vector<int32_t>& col,
                std::vector<double>& val, std::vector<double>& diag);
 // Device CSR of the prepared block (reference entry order); returns nnz.
 int64_t block_csr_device(Ctx& c, DBuf& row_ptr, DBuf& col, DBuf& val, DBuf& diag);
-// Dense column-major matrix of the prepared block added into A (zeroed by the
-// caller), entries summed in the CSR's order; no host synchronisation.
-void block_dense_device(Ctx& c, double2* A);
+// e^{i k.s} of momentum (mx, my) for every translation s, at re/im[s * stride].
+void block_phases(const Geom& g, int mx, int my, double* re, double* im, int stride);
+// ---- rows of many blocks of the prepared sector (pack.cu); items carry mx,
+// my, n and the offsets, the rest is filled in. No host synchronisation beyond
+// one per sector.
+// Dense Hermitian matrices (M + M^H)/2, column-major, at arena + off (zeroed).
+void pack_dense(Ctx& c, std::vector<PackItem>& items, double2* arena);
+// Entries, row lengths and diagonals of small blocks.
+void pack_entries(Ctx& c, std::vector<PackItem>& items, uint32_t* ent, int32_t* cnt, double* diag);
+SmallRatios small_ratios(int n);
 // H*V of the prepared block on device arrays [dim][nv] complex (FP64 or FP32).
 // partial_dev[grid][nv] receives each CTA's fixed-point sum of Re<s x, y>.
 void hv_apply(Ctx& c, const void* in, void* out, int nv, bool fp32, const double* scale_dev,
@@ -336,14 +398,7 @@ void run_ftlm_block(Ctx& c, int n_up, int n_dn, int mx, int my, Spectrum& out,
                     const double* host_start /* [R][dim] complex or null */,
                     std::vector<double>* alpha_out, std::vector<double>* beta_out,
                     std::vector<int32_t>* steps_out);
-// FTLM spectra of several small blocks (dim <= kSmallMaxDim) of the prepared
-// sector in one persistent launch; stored like run_ftlm_block's.
-void run_small_ftlm_blocks(Ctx& c, const std::vector<std::pair<int, int>>& blocks);
-// Ritz values and weights of R Lanczos runs (alpha/beta [sweep][K][ld],
-// nvmax vectors per sweep, steps[R] on the device) into the spectra arena.
-void ritz_stage(Ctx& c, int R, int nvmax, int ld, int K, const double* alpha, const double* beta,
-                const int32_t* steps, Spectrum& out);
-// The same for several blocks with one host synchronisation.
+// One block of a Ritz stage.
 struct RitzJob {
   int R, nvmax, ld, K;
   const double* alpha;
@@ -351,6 +406,18 @@ struct RitzJob {
   const int32_t* steps;
   Spectrum* out;
 };
+// FTLM spectra of several small blocks (dim <= kSmallMaxDim) of the prepared
+// sector; stored like run_ftlm_block's, or pooled until flush_deferred.
+void run_small_ftlm_blocks(Ctx& c, const std::vector<std::pair<int, int>>& blocks);
+// Empties the sb_* arrays. Makes c.stream wait for the side streams' Lanczos.
+void small_rows_reset(Ctx& c);
+void small_join(Ctx& c);
+RitzJob small_ritz_job(Ctx& c, const SmallBlockDesc& d, Spectrum* out);
+// Ritz values and weights of R Lanczos runs (alpha/beta [sweep][K][ld],
+// nvmax vectors per sweep, steps[R] on the device) into the spectra arena.
+void ritz_stage(Ctx& c, int R, int nvmax, int ld, int K, const double* alpha, const double* beta,
+                const int32_t* steps, Spectrum& out);
+// The same for several blocks with one host synchronisation.
 void ritz_stage_many(Ctx& c, std::vector<RitzJob>& jobs);
 // Exact spectra of several blocks of the prepared sector (one batched launch).
 void run_exact_blocks(Ctx& c, const std::vector<std::pair<int, int>>& blocks);
@@ -358,20 +425,19 @@ void run_exact_blocks(Ctx& c, const std::vector<std::pair<int, int>>& blocks);
 // first when they would push it past kDeferPoolBytes) and registers them as
 // pending spectra of the current sector.
 void queue_exact_blocks(Ctx& c, const std::vector<std::pair<int, int>>& blocks);
-// Diagonalises every pooled matrix in one launch, runs the Ritz stage of
-// every pooled FTLM block in one more, then the queued accumulations in
-// queue order, and turns the current sector's pending spectra into ordinary
+// Diagonalises the pooled matrices, runs Lanczos and the Ritz stage of the
+// pooled FTLM blocks, then the queued accumulations in queue order, and turns the current sector's pending spectra into ordinary
 // ones; empties the pool.
 void flush_deferred(Ctx& c);
-// Bytes held by the pool (matrices and Lanczos coefficients).
+// Bytes held by the pool (matrices, small-block rows, start vectors and coefficients).
 int64_t defer_pool_bytes(const Ctx& c);
 constexpr int64_t kDeferPoolBytes = int64_t(4) << 30;
 // Thermo
 void thermo_configure(Ctx& c, int nbeta, const double* beta, int nmu, const double* mu);
 void thermo_accumulate(Ctx& c, const Spectrum& s);
-void thermo_accumulate_host(Ctx& c, const double* ev, const double* w, int64_t count, double pref, int particles);
 // Accumulates a spectrum already on the device (w null: unit weights).
 void thermo_accumulate_dev(Ctx& c, const double* ev, const double* w, int64_t count, double pref, int particles);
+void thermo_accumulate_host(Ctx& c, const double* ev, const double* w, int64_t count, double pref, int particles);
 void thermo_read(Ctx& c, double* emin, double* z, double* n, double* n2);
 
 // Seeds and reference start vectors (main.cpp:514-533, 1015-1025)

@@ -12,9 +12,10 @@ namespace {
 
 // Resolve a hop target (tu, td) to its block column, translation shift,
 // sign parity and orbit stabiliser size. Returns false when the target's
-// orbit is inactive in this block (main.cpp:790-793).
-template <typename W, typename R>
-__device__ __forceinline__ bool resolve(W tu, W td, bool up_hop, uint32_t ur_src, const BlockView<W>& v,
+// orbit is inactive in this block (main.cpp:790-793). View: BlockView or any
+// struct with its lookup tables.
+template <typename W, typename R, typename View>
+__device__ __forceinline__ bool resolve(W tu, W td, bool up_hop, uint32_t ur_src, const View& v,
                                         const Geom& g, const R* binom, int64_t& col, int& shift, int& sgn,
                                         int& deg) {
   uint32_t ur = ur_src;

@@ -211,10 +211,11 @@ __global__ void k_dn_class(const W* __restrict__ dns, int64_t c_dn, int ncls, co
   }
 }
 
-__global__ void k_narrow(const int64_t* __restrict__ in, int32_t* __restrict__ out, int64_t n) {
+// Scan positions relative to the start of their class of c_dn words.
+__global__ void k_narrow(const int64_t* __restrict__ in, int32_t* __restrict__ out, int64_t n, int64_t c_dn) {
   for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < n;
        i += static_cast<int64_t>(gridDim.x) * blockDim.x)
-    out[i] = static_cast<int32_t>(in[i]);
+    out[i] = static_cast<int32_t>(in[i] - in[i / c_dn * c_dn]);
 }
 
 __global__ void k_class_counts(const uint16_t* __restrict__ ur_class, int64_t nur,
@@ -225,22 +226,6 @@ __global__ void k_class_counts(const uint16_t* __restrict__ ur_class, int64_t nu
 }
 
 // ------------------------------------------------------------------ block
-
-// Stabiliser character test of a canonical word for momentum (mx, my):
-// active iff sign(s) * exp(2 pi i (mx dx/lx + my dy/ly)) == 1 on the whole
-// stabiliser (exact integer form of the dnf > 1e-12 test, main.cpp:748-768:
-// the orbit sum of a group character is |stab| or exactly zero).
-__device__ __forceinline__ bool char_trivial(uint64_t stab, uint64_t chi, int mx, int my, const Geom& g) {
-  const int L = g.lx * g.ly;
-  for (uint64_t m = stab & ~1ULL; m; m &= m - 1) {
-    const int s = __ffsll(static_cast<long long>(m)) - 1;
-    const int q = (mx * shift_dx(s, g) * g.ly + my * shift_dy(s, g) * g.lx) % L;
-    const bool neg = (chi >> s) & 1ULL;
-    if (!neg && q != 0) return false;
-    if (neg && 2 * q != L) return false;
-  }
-  return true;
-}
 
 __global__ void k_dn_active(int64_t total, const int32_t* __restrict__ canon, const uint64_t* __restrict__ d_stab,
                             const uint64_t* __restrict__ d_chi, int mx, int my, const __grid_constant__ Geom g,
@@ -385,6 +370,16 @@ __global__ void k_debug_relations(int64_t c_up, int64_t c_dn, const __grid_const
 template <typename W>
 W* wptr(const DBuf& b) { return b.as<W>(); }
 
+// Values of a scan over ncls classes of c_dn words at the class starts, in one
+// strided copy ([ncls + 1], the last one left to the caller).
+std::vector<int64_t> class_bases(const int64_t* scan, int ncls, int64_t c_dn, cudaStream_t st) {
+  std::vector<int64_t> base(ncls + 1, 0);
+  FTLM_CUDA(cudaMemcpy2DAsync(base.data(), sizeof(int64_t), scan, sizeof(int64_t) * c_dn, sizeof(int64_t), ncls,
+                              cudaMemcpyDeviceToHost, st));
+  FTLM_CUDA(cudaStreamSynchronize(st));
+  return base;
+}
+
 template <typename W>
 void sector_prepare_t(Ctx& c, int n_up, int n_dn) {
   SectorTables& S = c.sec;
@@ -493,11 +488,12 @@ void sector_prepare_t(Ctx& c, int n_up, int n_dn) {
                                                         S.d_star.as<uint32_t>(), S.d_hs.as<uint16_t>(), canon,
                                                         S.d_stab.as<uint64_t>(), S.d_chi.as<uint64_t>());
     FTLM_LAUNCH_CHECK();
-    for (int cl = 1; cl < S.nclass; ++cl) {
-      const int64_t base = static_cast<int64_t>(cl - 1) * S.c_dn;
-      S.cls_ncanon[cl] = scan_excl_i32_to_i64(c, canon + base, S.tmp_d.as<int64_t>() + base, S.c_dn);
-    }
-    k_narrow<<<blocks_for(tot, 256), 256, 0, st>>>(S.tmp_d.as<int64_t>(), S.d_cidx.as<int32_t>(), tot);
+    // one scan over all classes; a word's index counts from its class's start
+    const int64_t all = scan_excl_i32_to_i64(c, canon, S.tmp_d.as<int64_t>(), tot);
+    std::vector<int64_t> base = class_bases(S.tmp_d.as<int64_t>(), ncls, S.c_dn, st);
+    base[ncls] = all;
+    for (int cl = 1; cl < S.nclass; ++cl) S.cls_ncanon[cl] = base[cl] - base[cl - 1];
+    k_narrow<<<blocks_for(tot, 256), 256, 0, st>>>(S.tmp_d.as<int64_t>(), S.d_cidx.as<int32_t>(), tot, S.c_dn);
     FTLM_LAUNCH_CHECK();
   }
   // keep the canonical flags for block builds and the debug views
@@ -544,20 +540,8 @@ void block_prepare_t(Ctx& c, int mx, int my, bool rows) {
                                                       mx, my, g, flag);
     FTLM_LAUNCH_CHECK();
     const int64_t all = scan_excl_i32_to_i64(c, flag, S.tmp_d.as<int64_t>(), tot);
-    (void)all;
     // class bases within the global scan
-    std::vector<int64_t> base(ncls + 1);
-    for (int cl = 0; cl <= ncls; ++cl) {
-      const int64_t idx = static_cast<int64_t>(cl) * S.c_dn;
-      int64_t v = 0;
-      if (idx < tot) {
-        FTLM_CUDA(cudaMemcpyAsync(&v, S.tmp_d.as<int64_t>() + idx, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
-      } else {
-        v = all;
-      }
-      base[cl] = v;
-    }
-    FTLM_CUDA(cudaStreamSynchronize(st));
+    std::vector<int64_t> base = class_bases(S.tmp_d.as<int64_t>(), ncls, S.c_dn, st);
     base[ncls] = all;
     for (int cl = 1; cl < S.nclass; ++cl) B.cls_nact[cl] = base[cl] - base[cl - 1];
     DBuf& bb = S.tmp_e;
@@ -582,16 +566,7 @@ void block_prepare_t(Ctx& c, int mx, int my, bool rows) {
   B.aoff.ensure(sizeof(int64_t) * (S.nur + 1));
   B.dim = scan_excl_i32_to_i64(c, per_ur, B.aoff.as<int64_t>(), S.nur);
   FTLM_CUDA(cudaMemcpyAsync(B.aoff.as<int64_t>() + S.nur, &B.dim, sizeof(int64_t), cudaMemcpyHostToDevice, st));
-  // momentum phases, computed exactly as main.cpp:736-743
-  const double kPi = 3.141592653589793238462643383279502884;
-  for (int s = 0; s < g.n; ++s) {
-    const int dx = s % g.lx, dy = s / g.lx;
-    const double arg = 2.0 * kPi *
-                       (static_cast<double>(mx * dx) / static_cast<double>(g.lx) +
-                        static_cast<double>(my * dy) / static_cast<double>(g.ly));
-    B.phase_re[s] = std::cos(arg);
-    B.phase_im[s] = std::sin(arg);
-  }
+  block_phases(g, mx, my, B.phase_re, B.phase_im, 1);
   B.mx = mx;
   B.my = my;
   if (rows && B.dim > 0) {
@@ -607,6 +582,18 @@ void block_prepare_t(Ctx& c, int mx, int my, bool rows) {
 }
 
 }  // namespace
+
+void block_phases(const Geom& g, int mx, int my, double* re, double* im, int stride) {  // main.cpp:736-743
+  const double kPi = 3.141592653589793238462643383279502884;
+  for (int s = 0; s < g.n; ++s) {
+    const int dx = s % g.lx, dy = s / g.lx;
+    const double arg = 2.0 * kPi *
+                       (static_cast<double>(mx * dx) / static_cast<double>(g.lx) +
+                        static_cast<double>(my * dy) / static_cast<double>(g.ly));
+    re[s * stride] = std::cos(arg);
+    im[s * stride] = std::sin(arg);
+  }
+}
 
 int64_t scan_excl_i32_to_i64(Ctx& c, const int32_t* flags, int64_t* out, int64_t n) {
   if (n <= 0) return 0;

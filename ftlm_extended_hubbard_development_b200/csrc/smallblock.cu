@@ -1,15 +1,29 @@
-// Small FTLM blocks in one persistent launch (run_ftlm_block,
-// main.cpp:996-1113, for every block of a sector up to kSmallMaxDim rows).
+// Small FTLM blocks (run_ftlm_block, main.cpp:996-1113, for every block of a
+// sector up to kSmallMaxDim rows).
 //
 // A block of a few thousand rows gives one H*V far too little work to fill
 // the GPU, so stepping it with the sweep kernels spends its time in launch
 // latency (four launches per Lanczos step). Here one CTA runs the whole
-// Lanczos recurrence of one (block, random vector) pair: the three working
-// vectors live in shared memory, the block's CSR (reference entry order) is
-// read from L2, where all CTAs of the block share it, and alpha/beta go to
-// the same [K][ld] layout the sweep path writes, so the Ritz stage
-// (k_tridiag) and everything after it are shared. Tasks are ordered largest
-// block first and taken in a grid-stride loop by a grid sized to the SMs.
+// Lanczos recurrence of one (block, random vector) pair: the two working
+// vectors live in shared memory, H's rows are 4-byte entries read from L2
+// (column, direction, sign, shift, orbit-size ratio; the coefficient is a
+// table entry times a ratio), and alpha/beta go to the same [K][ld] layout the
+// sweep path writes, so the Ritz stage (k_tridiag) and everything after it are
+// shared. With pooled spectra a sector's launches go to a side stream, so the
+// small blocks of several sectors run beside each other and beside the table
+// builds of the next ones.
+//
+// A thread owns whole rows (i, i + threads, ...): entry k of consecutive rows
+// is consecutive in memory, H v stays in registers until alpha is known, and
+// the next vector overwrites the previous one in place, so a step has three
+// barriers. Size classes pick the threads: 256 up to 512 rows, 512 up to 1024,
+// 1024 above, one launch each, so a small block does not wait behind the
+// shared memory and barriers of a large one. Bound: reads of x and of the
+// coefficients in shared memory (32 bytes per FP64 hop). 3x3 curve, 5 FP64
+// vectors x 80 steps, 288 blocks up to 1764 rows: 82 ms in 32 launches of 256
+// threads on 20-byte CSR entries, one after another (45 of 148 SMs busy),
+// against 27 ms of launches that overlap; 4x2 curve, 32 mixed vectors x 120
+// steps: 24 ms against 8.2.
 //
 // Arithmetic is the reference's: w = H v; alpha = Re<v, w>;
 // w -= alpha v + beta_prev v_prev; beta = |w|; stop at beta < 1e-12 or the
@@ -26,21 +40,6 @@ namespace ftlm {
 
 namespace {
 
-constexpr int kSmallThreads = 256;
-constexpr int kRowLanes = 8;  // lanes sharing one CSR row
-constexpr int kWarps = kSmallThreads / 32;
-
-struct SmallBlockDesc {
-  int64_t rp_off;     // row pointers (int32) at rp[rp_off .. rp_off+dim]
-  int64_t nz_off;     // CSR entries start at col/val[nz_off]
-  int64_t diag_off;   // diagonal at diag[diag_off ..)
-  int64_t ab_off;     // alpha/beta [K][ld] at ab[ab_off ..)
-  int64_t start_off;  // reference start vectors [R][dim] complex at start[start_off ..), -1: Philox
-  int64_t steps_off;  // steps[steps_off + r]
-  uint64_t seed;      // block seed (Philox key)
-  int32_t dim, K, ld, pad;
-};
-
 template <typename T>
 struct CT;
 template <>
@@ -56,51 +55,79 @@ struct CT<float> {
   }
 };
 
-// Fixed-order CTA sum of one double per thread; every thread gets the result.
+// Fixed-order CTA sum of one double per thread, the same in every thread; red
+// must not be the one of the previous call (one barrier per call).
+template <int NW>
 __device__ __forceinline__ double cta_sum(double v, double* red) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  const int warp = threadIdx.x >> 5;
-  if ((threadIdx.x & 31) == 0) red[warp] = v;
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
   __syncthreads();
-  double s = 0.0;
+  double s = (threadIdx.x & 31) < NW ? red[threadIdx.x & 31] : 0.0;
 #pragma unroll
-  for (int i = 0; i < kWarps; ++i) s += red[i];
-  __syncthreads();  // red is reused by the next sum
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
   return s;
 }
 
-template <typename T>
-__global__ void __launch_bounds__(kSmallThreads) k_lanczos_small(
-    int ntasks, const int2* __restrict__ tasks, const SmallBlockDesc* __restrict__ blocks,
-    const int32_t* __restrict__ rp_all, const int32_t* __restrict__ col_all, const double2* __restrict__ val_all,
-    const double* __restrict__ diag_all, const double2* __restrict__ start_all, double* __restrict__ alpha_all,
-    double* __restrict__ beta_all, int32_t* __restrict__ steps_all, int cap) {
+struct SmallArgs {
+  int ntasks, cap, nsite;
+  const int2* tasks;  // (block, vector)
+  const SmallBlockDesc* blocks;
+  const uint32_t* ent;
+  const int32_t* cnt;
+  const double* diag;
+  const double* phase;  // [n_k][64] complex
+  const double2* start;
+  double* alpha;
+  double* beta;
+  int32_t* steps;
+  double amp_re[8], amp_im[8];
+  double sqrt_deg[65];
+  SmallRatios ratios;
+};
+
+template <typename T, int NT, int RPT>
+__global__ void __launch_bounds__(NT) k_lanczos_small(const __grid_constant__ SmallArgs A) {
   using C = typename CT<T>::C;
+  constexpr int NW = NT / 32;
   extern __shared__ __align__(16) unsigned char small_smem[];
-  C* b0 = reinterpret_cast<C*>(small_smem);
-  __shared__ double red[kWarps];
+  __shared__ double red[2][32];
+  __shared__ double s_ratio[kSmallRatios];
+  double2* coef = reinterpret_cast<double2*>(small_smem);  // [shift][dir * 2 + parity]
+  C* b0 = reinterpret_cast<C*>(coef + A.nsite * 16);
   const int tid = threadIdx.x;
-  const int lane8 = tid & (kRowLanes - 1);
-  const int group = tid / kRowLanes;
-  constexpr int kGroups = kSmallThreads / kRowLanes;
-  for (int t = blockIdx.x; t < ntasks; t += gridDim.x) {
-    const int2 task = tasks[t];
-    const SmallBlockDesc B = blocks[task.x];
-    const int r = task.y;
-    const int D = B.dim;
-    const int32_t* rp = rp_all + B.rp_off;
-    const int32_t* col = col_all + B.nz_off;
-    const double2* val = val_all + B.nz_off;
-    const double* diag = diag_all + B.diag_off;
+  for (int i = tid; i < A.ratios.n; i += NT)
+    s_ratio[i] = __ddiv_rn(A.sqrt_deg[A.ratios.num[i]], A.sqrt_deg[A.ratios.den[i]]);
+  for (int t = blockIdx.x; t < A.ntasks; t += gridDim.x) {
+    const int2 task = A.tasks[t];
+    const SmallBlockDesc B = A.blocks[task.x];
+    const int r = task.y, D = B.dim;
     C* v = b0;
-    C* vp = b0 + cap;
-    C* w = b0 + 2 * cap;
+    C* vp = b0 + A.cap;
+    __syncthreads();  // the previous task's vectors and table are no longer read
+    for (int i = tid; i < A.nsite * 16; i += NT) {
+      // (amp * sign) * phase, the operation order of main.cpp:794-797
+      const int dir = (i >> 1) & 7;
+      const double ar = i & 1 ? -A.amp_re[dir] : A.amp_re[dir];
+      const double ai = i & 1 ? -A.amp_im[dir] : A.amp_im[dir];
+      const double pr = A.phase[128 * B.k + 2 * (i >> 4)], pi = A.phase[128 * B.k + 2 * (i >> 4) + 1];
+      coef[i] = make_double2(__dsub_rn(__dmul_rn(ar, pr), __dmul_rn(ai, pi)),
+                             __dadd_rn(__dmul_rn(ar, pi), __dmul_rn(ai, pr)));
+    }
     const double amp = 1.0 / sqrt(static_cast<double>(D));
-    for (int i = tid; i < D; i += kSmallThreads) {
+    int len[RPT];
+    double dg[RPT];
+#pragma unroll
+    for (int q = 0; q < RPT; ++q) {
+      const int i = tid + q * NT;
+      len[q] = 0;
+      dg[q] = 0.0;
+      if (i >= D) continue;
+      len[q] = A.cnt[B.row_off + i];
+      dg[q] = A.diag[B.row_off + i];
       double re, im;
       if (B.start_off >= 0) {
-        const double2 z = start_all[B.start_off + static_cast<int64_t>(r) * D + i];
+        const double2 z = A.start[B.start_off + static_cast<int64_t>(r) * D + i];
         re = z.x;
         im = z.y;
       } else {
@@ -113,220 +140,178 @@ __global__ void __launch_bounds__(kSmallThreads) k_lanczos_small(
     double beta_prev = 0.0;
     int steps = B.K;
     for (int j = 0; j < B.K; ++j) {
-      // w = H v; partial Re<v, w>
+      // h = H v; partial Re<v, h>
+      C h[RPT];
       double ap = 0.0;
-      // the row loop is warp-uniform (the shuffles below need all 32 lanes):
-      // each warp takes 4 consecutive rows per pass, one per 8-lane group
-      for (int i0 = (tid >> 5) * (32 / kRowLanes); i0 < D; i0 += kGroups) {
-        const int i = i0 + group % (32 / kRowLanes);
-        double ar = 0.0, ai = 0.0;
-        const int e0 = i < D ? rp[i] + lane8 : 0;
-        const int e1 = i < D ? rp[i + 1] : 0;
-        for (int e = e0; e < e1; e += kRowLanes) {
-          const double2 h = val[e];
-          const C x = v[col[e]];
-          ar += h.x * static_cast<double>(x.x) - h.y * static_cast<double>(x.y);
-          ai += h.x * static_cast<double>(x.y) + h.y * static_cast<double>(x.x);
-        }
 #pragma unroll
-        for (int o = kRowLanes / 2; o > 0; o >>= 1) {
-          ar += __shfl_xor_sync(0xffffffffu, ar, o);
-          ai += __shfl_xor_sync(0xffffffffu, ai, o);
+      for (int q = 0; q < RPT; ++q) {
+        const int i = tid + q * NT;
+        if (i >= D) continue;
+        const uint32_t* e = A.ent + B.ent_off + i;
+        const C xi = v[i];
+        double ar = 0.0, ai = 0.0;
+        int n = len[q];
+        auto add = [&](uint32_t w) {
+          const double2 c = coef[(w >> 12) & 0x3FF];
+          const double ratio = s_ratio[w >> 22];
+          const C x = v[w & 0xFFF];
+          const double cr = __dmul_rn(c.x, ratio), ci = __dmul_rn(c.y, ratio);
+          ar += cr * static_cast<double>(x.x) - ci * static_cast<double>(x.y);
+          ai += cr * static_cast<double>(x.y) + ci * static_cast<double>(x.x);
+        };
+        for (; n >= 4; n -= 4, e += 4 * static_cast<int64_t>(D)) {
+          const uint32_t w0 = __ldg(e), w1 = __ldg(e + D), w2 = __ldg(e + 2 * D), w3 = __ldg(e + 3 * D);
+          add(w0);
+          add(w1);
+          add(w2);
+          add(w3);
         }
-        if (lane8 == 0 && i < D) {
-          const C xi = v[i];
-          ar += diag[i] * static_cast<double>(xi.x);
-          ai += diag[i] * static_cast<double>(xi.y);
-          const C wi = CT<T>::make(ar, ai);
-          w[i] = wi;
-          ap += static_cast<double>(xi.x) * static_cast<double>(wi.x) +
-                static_cast<double>(xi.y) * static_cast<double>(wi.y);
-        }
+        for (; n > 0; --n, e += D) add(__ldg(e));
+        ar += dg[q] * static_cast<double>(xi.x);
+        ai += dg[q] * static_cast<double>(xi.y);
+        h[q] = CT<T>::make(ar, ai);
+        ap += static_cast<double>(xi.x) * static_cast<double>(h[q].x) +
+              static_cast<double>(xi.y) * static_cast<double>(h[q].y);
       }
-      const double alpha = cta_sum(ap, red);  // also orders the writes of w before the update
-      // w -= alpha v + beta_prev vp; partial |w|^2
+      const double alpha = cta_sum<NW>(ap, red[0]);
+      // h -= alpha v + beta_prev vp; partial |h|^2
       double np = 0.0;
-      for (int i = tid; i < D; i += kSmallThreads) {
-        const C hi = w[i], xi = v[i], pi = vp[i];
-        const C ri = CT<T>::make(static_cast<double>(hi.x) - alpha * static_cast<double>(xi.x) -
-                                     beta_prev * static_cast<double>(pi.x),
-                                 static_cast<double>(hi.y) - alpha * static_cast<double>(xi.y) -
-                                     beta_prev * static_cast<double>(pi.y));
-        w[i] = ri;
-        np += static_cast<double>(ri.x) * static_cast<double>(ri.x) +
-              static_cast<double>(ri.y) * static_cast<double>(ri.y);
+#pragma unroll
+      for (int q = 0; q < RPT; ++q) {
+        const int i = tid + q * NT;
+        if (i >= D) continue;
+        const C xi = v[i], pi = vp[i];
+        h[q] = CT<T>::make(static_cast<double>(h[q].x) - alpha * static_cast<double>(xi.x) -
+                               beta_prev * static_cast<double>(pi.x),
+                           static_cast<double>(h[q].y) - alpha * static_cast<double>(xi.y) -
+                               beta_prev * static_cast<double>(pi.y));
+        np += static_cast<double>(h[q].x) * static_cast<double>(h[q].x) +
+              static_cast<double>(h[q].y) * static_cast<double>(h[q].y);
       }
-      const double beta = sqrt(cta_sum(np, red));
-      if (tid == 0) alpha_all[B.ab_off + static_cast<int64_t>(j) * B.ld + r] = alpha;
+      const double beta = sqrt(cta_sum<NW>(np, red[1]));
+      if (tid == 0) A.alpha[B.ab_off + static_cast<int64_t>(j) * B.ld + r] = alpha;
       if (beta < 1e-12 || j + 1 == B.K) {  // uniform: every thread holds the same beta
         steps = j + 1;
         break;
       }
-      if (tid == 0) beta_all[B.ab_off + static_cast<int64_t>(j) * B.ld + r] = beta;
+      if (tid == 0) A.beta[B.ab_off + static_cast<int64_t>(j) * B.ld + r] = beta;
       const double inv = 1.0 / beta;
-      for (int i = tid; i < D; i += kSmallThreads) {
-        const C ri = w[i];
-        w[i] = CT<T>::make(static_cast<double>(ri.x) * inv, static_cast<double>(ri.y) * inv);
+#pragma unroll
+      for (int q = 0; q < RPT; ++q) {  // v_next replaces v_prev, which only this thread reads
+        const int i = tid + q * NT;
+        if (i < D) vp[i] = CT<T>::make(static_cast<double>(h[q].x) * inv, static_cast<double>(h[q].y) * inv);
       }
       __syncthreads();
-      C* tmp = vp;  // rotate: v_prev <- v, v <- w, w <- old v_prev
+      C* tmp = vp;
       vp = v;
-      v = w;
-      w = tmp;
+      v = tmp;
       beta_prev = beta;
     }
-    if (tid == 0) steps_all[B.steps_off + r] = steps;
-    __syncthreads();  // the next task overwrites the vectors
+    if (tid == 0) A.steps[B.steps_off + r] = steps;
   }
 }
 
-}  // namespace
+template <typename T, int NT, int RPT>
+void launch_small(Ctx& c, const SmallArgs& A, cudaStream_t st) {
+  const size_t smem = sizeof(double2) * 16 * A.nsite + static_cast<size_t>(2) * A.cap * sizeof(typename CT<T>::C);
+  auto kern = k_lanczos_small<T, NT, RPT>;
+  FTLM_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+  int per_sm = 0;
+  FTLM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, NT, smem));
+  if (per_sm < 1) throw Error(FTLM_ERR_CAPACITY, "small-block Lanczos does not fit on an SM");
+  const int grid = static_cast<int>(std::min<int64_t>(A.ntasks, static_cast<int64_t>(c.sm_count) * per_sm));
+  kern<<<grid, NT, smem, st>>>(A);
+  FTLM_LAUNCH_CHECK();
+  c.prof.kernel_launches += 1;
+}
 
-void run_small_ftlm_blocks(Ctx& c, const std::vector<std::pair<int, int>>& blocks) {
-  if (blocks.empty()) return;
-  const bool fp32 = c.opts.precision == FTLM_PREC_MIXED;
+template <typename T>
+void launch_class(Ctx& c, int cls, const SmallArgs& A, cudaStream_t st) {
+  if (cls == 0) launch_small<T, 256, 2>(c, A, st);
+  else if (cls == 1) launch_small<T, 512, 2>(c, A, st);
+  else launch_small<T, 1024, 4>(c, A, st);
+}
+
+void side_sync(Ctx& c) {
+  for (cudaStream_t s : c.side)
+    if (s) FTLM_CUDA(cudaStreamSynchronize(s));
+}
+
+// Room for `bytes` in a pooled buffer; the side streams are idle when it moves.
+void pool_room(Ctx& c, DBuf& b, size_t bytes) {
+  if (bytes <= b.cap) return;
+  side_sync(c);
+  b.ensure_keep(std::max(bytes, 2 * b.cap), c.stream);
+}
+
+// Lanczos of the blocks (rows in the sb_* arrays), one launch per size class,
+// on the next side stream when pooling, else on c.stream.
+void small_lanczos(Ctx& c, const std::vector<SmallBlockDesc>& blocks) {
   const int R = c.opts.samples;
-  struct Item {
-    int mx, my;
-    int64_t dim;
-    int K;
-    SmallBlockDesc d;
-  };
-  std::vector<Item> items;
-  int64_t rp_tot = 0, nz_tot = 0, dg_tot = 0, ab_tot = 0, st_tot = 0;
-  int ld = 1;  // alpha/beta row stride, as the sweep path uses for one sweep of R vectors
-  while (ld < std::max(R, fp32 ? 2 : 1)) ld <<= 1;
-  for (const auto& b : blocks) {
-    const int64_t D = c.block_dims.at(static_cast<size_t>(b.second * c.geom.lx + b.first));
-    if (D <= 0) continue;
-    if (D > kSmallMaxDim) throw Error(FTLM_ERR_ARG, "block too large for the small-block FTLM launch");
-    Item it{b.first, b.second, D, static_cast<int>(std::min<int64_t>(c.opts.lanczos_steps, D)), {}};
-    items.push_back(it);
-  }
-  if (items.empty()) return;
-  // CSR of every block into one arena (built block by block)
-  DBuf rp, cl, vl, dg;
-  std::vector<int64_t> nnz(items.size());
-  for (size_t i = 0; i < items.size(); ++i) {
-    Item& it = items[i];
-    it.d.rp_off = rp_tot;
-    it.d.diag_off = dg_tot;
-    it.d.ab_off = ab_tot;
-    it.d.steps_off = st_tot;
-    rp_tot += it.dim + 1;
-    dg_tot += it.dim;
-    ab_tot += static_cast<int64_t>(it.K) * ld;
-    st_tot += R;
-  }
-  for (size_t i = 0; i < items.size(); ++i) {
-    block_prepare(c, items[i].mx, items[i].my);
-    nnz[i] = block_csr_device(c, rp, cl, vl, dg);
-    items[i].d.nz_off = nz_tot;
-    nz_tot += std::max<int64_t>(nnz[i], 1);
-    // copy into the arenas right away (the per-block buffers are rebuilt next)
-    c.sb_rp.ensure_keep(sizeof(int32_t) * rp_tot, c.stream);
-    c.sb_col.ensure_keep(sizeof(int32_t) * nz_tot, c.stream);
-    c.sb_val.ensure_keep(sizeof(double2) * nz_tot, c.stream);
-    c.sb_diag.ensure_keep(sizeof(double) * dg_tot, c.stream);
-    const Item& it = items[i];
-    FTLM_CUDA(cudaMemcpyAsync(c.sb_rp.as<int32_t>() + it.d.rp_off, rp.p, sizeof(int32_t) * (it.dim + 1),
-                              cudaMemcpyDeviceToDevice, c.stream));
-    if (nnz[i] > 0) {
-      FTLM_CUDA(cudaMemcpyAsync(c.sb_col.as<int32_t>() + it.d.nz_off, cl.p, sizeof(int32_t) * nnz[i],
-                                cudaMemcpyDeviceToDevice, c.stream));
-      FTLM_CUDA(cudaMemcpyAsync(c.sb_val.as<double2>() + it.d.nz_off, vl.p, sizeof(double2) * nnz[i],
-                                cudaMemcpyDeviceToDevice, c.stream));
-    }
-    FTLM_CUDA(cudaMemcpyAsync(c.sb_diag.as<double>() + it.d.diag_off, dg.p, sizeof(double) * it.dim,
-                              cudaMemcpyDeviceToDevice, c.stream));
-    FTLM_CUDA(cudaStreamSynchronize(c.stream));  // rp/cl/vl/dg are rebuilt for the next block
-  }
-  rp.release();
-  cl.release();
-  vl.release();
-  dg.release();
-  // start vectors: reference Gaussian ones from the host, Philox on the device
-  const bool ref_start = c.opts.start_vector == FTLM_START_REF_GAUSSIAN;
-  std::vector<double> hstart;
-  int64_t start_tot = 0;
-  for (Item& it : items) {
-    it.d.seed = block_seed(c.opts.seed, c.sec.n_up, c.sec.n_dn, it.mx, it.my);
-    it.d.dim = static_cast<int32_t>(it.dim);
-    it.d.K = it.K;
-    it.d.ld = ld;
-    it.d.pad = 0;
-    it.d.start_off = ref_start ? start_tot : -1;
-    if (ref_start) start_tot += static_cast<int64_t>(R) * it.dim;
-  }
-  if (ref_start) {
-    hstart.resize(2 * static_cast<size_t>(start_tot));
-    for (const Item& it : items)
-      reference_start_vectors(it.d.seed, 0, R, it.dim, hstart.data() + 2 * it.d.start_off);
-    c.host_start.ensure(sizeof(double) * hstart.size());
-    FTLM_CUDA(cudaMemcpyAsync(c.host_start.p, hstart.data(), sizeof(double) * hstart.size(), cudaMemcpyHostToDevice,
-                              c.stream));
-    c.prof.h2d_bytes += static_cast<int64_t>(sizeof(double) * hstart.size());
-  }
-  // tasks, largest block first
-  std::vector<int> order(items.size());
+  const bool fp32 = c.opts.precision == FTLM_PREC_MIXED;
+  // tasks by size class, largest block first within one
+  std::vector<int> order(blocks.size());
   std::iota(order.begin(), order.end(), 0);
-  std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return items[a].dim > items[b].dim; });
+  std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return blocks[a].dim > blocks[b].dim; });
   std::vector<int2> tasks;
-  tasks.reserve(items.size() * R);
-  int64_t dmax = 0;
-  for (int b : order) {
-    dmax = std::max(dmax, items[b].dim);
-    for (int r = 0; r < R; ++r) tasks.push_back(make_int2(b, r));
+  tasks.reserve(blocks.size() * R);
+  int first[4] = {0, 0, 0, 0}, cap[3] = {1, 1, 1};
+  for (int cls = 2; cls >= 0; --cls) {
+    for (int b : order) {
+      const int d = blocks[b].dim;
+      if ((d > 1024 ? 2 : d > 512 ? 1 : 0) != cls) continue;
+      cap[cls] = std::max(cap[cls], d);
+      for (int r = 0; r < R; ++r) tasks.push_back(make_int2(b, r));
+    }
+    first[3 - cls] = static_cast<int>(tasks.size());
   }
-  std::vector<SmallBlockDesc> desc(items.size());
-  for (size_t i = 0; i < items.size(); ++i) desc[i] = items[i].d;
-  c.sb_meta.ensure(sizeof(int2) * tasks.size() + sizeof(SmallBlockDesc) * desc.size() + 64);
-  int2* d_tasks = c.sb_meta.as<int2>();
-  SmallBlockDesc* d_desc = reinterpret_cast<SmallBlockDesc*>(
-      (reinterpret_cast<uintptr_t>(d_tasks + tasks.size()) + 15) & ~static_cast<uintptr_t>(15));
+  const size_t tbytes = (sizeof(int2) * tasks.size() + 15) / 16 * 16, dbytes = sizeof(SmallBlockDesc) * blocks.size();
+  pool_room(c, c.sb_meta, static_cast<size_t>(c.sb_meta_used) + tbytes + dbytes);
+  char* meta = c.sb_meta.as<char>() + c.sb_meta_used;
+  c.sb_meta_used += static_cast<int64_t>((tbytes + dbytes + 15) / 16 * 16);
+  int2* d_tasks = reinterpret_cast<int2*>(meta);
+  SmallBlockDesc* d_desc = reinterpret_cast<SmallBlockDesc*>(meta + tbytes);
   FTLM_CUDA(cudaMemcpyAsync(d_tasks, tasks.data(), sizeof(int2) * tasks.size(), cudaMemcpyHostToDevice, c.stream));
-  FTLM_CUDA(cudaMemcpyAsync(d_desc, desc.data(), sizeof(SmallBlockDesc) * desc.size(), cudaMemcpyHostToDevice,
-                            c.stream));
-  c.lz_alpha.ensure(sizeof(double) * ab_tot);
-  c.lz_beta.ensure(sizeof(double) * ab_tot);
-  FTLM_CUDA(cudaMemsetAsync(c.lz_alpha.p, 0, sizeof(double) * ab_tot, c.stream));
-  FTLM_CUDA(cudaMemsetAsync(c.lz_beta.p, 0, sizeof(double) * ab_tot, c.stream));
-  c.sb_steps.ensure(sizeof(int32_t) * st_tot);
-  // one persistent launch
+  FTLM_CUDA(cudaMemcpyAsync(d_desc, blocks.data(), dbytes, cudaMemcpyHostToDevice, c.stream));
+  SmallArgs A{};
+  A.nsite = c.geom.n;
+  A.blocks = d_desc;
+  A.ent = c.sb_ent.as<uint32_t>();
+  A.cnt = c.sb_cnt.as<int32_t>();
+  A.diag = c.sb_diag.as<double>();
+  A.phase = c.pack.phase.as<double>();
+  A.start = c.sb_start.as<double2>();
+  A.alpha = c.sb_alpha.as<double>();
+  A.beta = c.sb_beta.as<double>();
+  A.steps = c.sb_steps.as<int32_t>();
+  std::copy(c.geom.amp_re, c.geom.amp_re + 8, A.amp_re);
+  std::copy(c.geom.amp_im, c.geom.amp_im + 8, A.amp_im);
+  std::copy(c.geom.sqrt_deg, c.geom.sqrt_deg + 65, A.sqrt_deg);
+  A.ratios = small_ratios(c.geom.n);
+  cudaStream_t st = c.stream;
+  if (c.spectra_defer && !c.timing) {
+    cudaStream_t& s = c.side[c.side_next];
+    c.side_next = (c.side_next + 1) % Ctx::kSide;
+    if (!s) FTLM_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
+    if (!c.side_ev) FTLM_CUDA(cudaEventCreateWithFlags(&c.side_ev, cudaEventDisableTiming));
+    FTLM_CUDA(cudaEventRecord(c.side_ev, c.stream));
+    FTLM_CUDA(cudaStreamWaitEvent(s, c.side_ev, 0));
+    st = s;
+  }
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   if (c.timing) {
     FTLM_CUDA(cudaEventCreate(&e0));
     FTLM_CUDA(cudaEventCreate(&e1));
     FTLM_CUDA(cudaEventRecord(e0, c.stream));
   }
-  const int cap = static_cast<int>(dmax);
-  const size_t smem = static_cast<size_t>(3) * cap * (fp32 ? sizeof(float2) : sizeof(double2));
-  int per_sm = 1;
-  if (fp32) {
-    FTLM_CUDA(cudaFuncSetAttribute(k_lanczos_small<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   static_cast<int>(std::max<size_t>(smem, 1))));
-    FTLM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_lanczos_small<float>, kSmallThreads, smem));
-  } else {
-    FTLM_CUDA(cudaFuncSetAttribute(k_lanczos_small<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   static_cast<int>(std::max<size_t>(smem, 1))));
-    FTLM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_lanczos_small<double>, kSmallThreads, smem));
+  for (int cls = 2; cls >= 0; --cls) {
+    A.tasks = d_tasks + first[2 - cls];
+    A.ntasks = first[3 - cls] - first[2 - cls];
+    A.cap = cap[cls];
+    if (A.ntasks == 0) continue;
+    if (fp32) launch_class<float>(c, cls, A, st);
+    else launch_class<double>(c, cls, A, st);
   }
-  if (per_sm < 1) throw Error(FTLM_ERR_CAPACITY, "small-block Lanczos does not fit on an SM");
-  const int grid = static_cast<int>(std::min<int64_t>(static_cast<int64_t>(tasks.size()),
-                                                      static_cast<int64_t>(c.sm_count) * per_sm));
-  const double2* start = ref_start ? c.host_start.as<double2>() : nullptr;
-  if (fp32)
-    k_lanczos_small<float><<<grid, kSmallThreads, smem, c.stream>>>(
-        static_cast<int>(tasks.size()), d_tasks, d_desc, c.sb_rp.as<int32_t>(), c.sb_col.as<int32_t>(),
-        c.sb_val.as<double2>(), c.sb_diag.as<double>(), start, c.lz_alpha.as<double>(), c.lz_beta.as<double>(),
-        c.sb_steps.as<int32_t>(), cap);
-  else
-    k_lanczos_small<double><<<grid, kSmallThreads, smem, c.stream>>>(
-        static_cast<int>(tasks.size()), d_tasks, d_desc, c.sb_rp.as<int32_t>(), c.sb_col.as<int32_t>(),
-        c.sb_val.as<double2>(), c.sb_diag.as<double>(), start, c.lz_alpha.as<double>(), c.lz_beta.as<double>(),
-        c.sb_steps.as<int32_t>(), cap);
-  FTLM_LAUNCH_CHECK();
-  c.prof.kernel_launches += 1;
   if (c.timing) {
     FTLM_CUDA(cudaEventRecord(e1, c.stream));
     FTLM_CUDA(cudaEventSynchronize(e1));
@@ -337,49 +322,139 @@ void run_small_ftlm_blocks(Ctx& c, const std::vector<std::pair<int, int>>& block
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
   }
-  if (c.spectra_defer) {
-    // Lanczos coefficients into the pool; the Ritz stage runs for every
-    // pooled block of every sector in one launch when the pool is flushed
-    const int64_t add = static_cast<int64_t>(sizeof(double)) * 2 * ab_tot + static_cast<int64_t>(sizeof(int32_t)) * st_tot;
-    if (defer_pool_bytes(c) > 0 && defer_pool_bytes(c) + add > kDeferPoolBytes) flush_deferred(c);
-    const int64_t ab0 = c.defer_ab_used, st0 = c.defer_st_used;
-    c.defer_ab.ensure_keep(sizeof(double) * (ab0 + 2 * ab_tot), c.stream);
-    c.defer_st.ensure_keep(sizeof(int32_t) * (st0 + st_tot), c.stream);
-    FTLM_CUDA(cudaMemcpyAsync(c.defer_ab.as<double>() + ab0, c.lz_alpha.p, sizeof(double) * ab_tot,
-                              cudaMemcpyDeviceToDevice, c.stream));
-    FTLM_CUDA(cudaMemcpyAsync(c.defer_ab.as<double>() + ab0 + ab_tot, c.lz_beta.p, sizeof(double) * ab_tot,
-                              cudaMemcpyDeviceToDevice, c.stream));
-    FTLM_CUDA(cudaMemcpyAsync(c.defer_st.as<int32_t>() + st0, c.sb_steps.p, sizeof(int32_t) * st_tot,
-                              cudaMemcpyDeviceToDevice, c.stream));
-    c.defer_ab_used = ab0 + 2 * ab_tot;
-    c.defer_st_used = st0 + st_tot;
+}
+
+}  // namespace
+
+void small_join(Ctx& c) {
+  for (cudaStream_t s : c.side) {
+    if (!s) continue;
+    FTLM_CUDA(cudaEventRecord(c.side_ev, s));
+    FTLM_CUDA(cudaStreamWaitEvent(c.stream, c.side_ev, 0));
+  }
+}
+
+// The next blocks overwrite the arrays in c.stream's order, which small_join
+// has put behind the side streams.
+void small_rows_reset(Ctx& c) {
+  c.sb_ent_used = c.sb_row_used = c.sb_start_used = c.sb_ab_used = c.sb_st_used = c.sb_meta_used = 0;
+}
+
+RitzJob small_ritz_job(Ctx& c, const SmallBlockDesc& d, Spectrum* out) {
+  return RitzJob{c.opts.samples, c.opts.samples, d.ld, d.K, c.sb_alpha.as<double>() + d.ab_off,
+                 c.sb_beta.as<double>() + d.ab_off, c.sb_steps.as<int32_t>() + d.steps_off, out};
+}
+
+void run_small_ftlm_blocks(Ctx& c, const std::vector<std::pair<int, int>>& blocks) {
+  if (blocks.empty()) return;
+  const int R = c.opts.samples;
+  const bool ref_start = c.opts.start_vector == FTLM_START_REF_GAUSSIAN;
+  int ld = 1;  // alpha/beta row stride, as the sweep path uses for one sweep of R vectors
+  while (ld < std::max(R, c.opts.precision == FTLM_PREC_MIXED ? 2 : 1)) ld <<= 1;
+  const int64_t most = static_cast<int64_t>(c.geom.ndir) * (c.sec.n_up + c.sec.n_dn);  // hops of a row, at most
+  struct Item {
+    int mx, my;
+    SmallBlockDesc d;
+  };
+  std::vector<Item> items;
+  std::vector<PackItem> rows;
+  int64_t ent = 0, row = 0, start = 0, ab = 0, st = 0;
+  for (const auto& b : blocks) {
+    const int64_t D = c.block_dims.at(static_cast<size_t>(b.second * c.geom.lx + b.first));
+    if (D <= 0) continue;
+    if (D > kSmallMaxDim) throw Error(FTLM_ERR_ARG, "block too large for the small-block FTLM launch");
+    SmallBlockDesc d{};
+    d.dim = static_cast<int32_t>(D);
+    d.K = static_cast<int32_t>(std::min<int64_t>(c.opts.lanczos_steps, D));
+    d.ld = ld;
+    d.k = b.second * c.geom.lx + b.first;
+    d.seed = block_seed(c.opts.seed, c.sec.n_up, c.sec.n_dn, b.first, b.second);
+    d.ent_off = ent;
+    d.row_off = row;
+    d.ab_off = ab;
+    d.steps_off = st;
+    d.start_off = ref_start ? start : -1;
+    ent += D * most;
+    row += D;
+    ab += static_cast<int64_t>(d.K) * ld;
+    st += R;
+    if (ref_start) start += static_cast<int64_t>(R) * D;
+    items.push_back({b.first, b.second, d});
+  }
+  if (items.empty()) return;
+  const int64_t add = static_cast<int64_t>(sizeof(uint32_t)) * ent +
+                      static_cast<int64_t>(sizeof(int32_t) + sizeof(double)) * row +
+                      static_cast<int64_t>(sizeof(double2)) * start + static_cast<int64_t>(2 * sizeof(double)) * ab;
+  if (defer_pool_bytes(c) > 0 && defer_pool_bytes(c) + add > kDeferPoolBytes) flush_deferred(c);
+  for (Item& it : items) {
+    it.d.ent_off += c.sb_ent_used;
+    it.d.row_off += c.sb_row_used;
+    it.d.ab_off += c.sb_ab_used;
+    it.d.steps_off += c.sb_st_used;
+    if (ref_start) it.d.start_off += c.sb_start_used;
+    PackItem p{};
+    p.mx = it.mx;
+    p.my = it.my;
+    p.n = it.d.dim;
+    p.off = it.d.ent_off;
+    p.off2 = it.d.row_off;
+    rows.push_back(p);
+  }
+  pool_room(c, c.sb_ent, sizeof(uint32_t) * std::max<int64_t>(c.sb_ent_used + ent, 1));
+  pool_room(c, c.sb_cnt, sizeof(int32_t) * (c.sb_row_used + row));
+  pool_room(c, c.sb_diag, sizeof(double) * (c.sb_row_used + row));
+  pool_room(c, c.sb_alpha, sizeof(double) * (c.sb_ab_used + ab));
+  pool_room(c, c.sb_beta, sizeof(double) * (c.sb_ab_used + ab));
+  pool_room(c, c.sb_steps, sizeof(int32_t) * (c.sb_st_used + st));
+  FTLM_CUDA(cudaMemsetAsync(c.sb_alpha.as<double>() + c.sb_ab_used, 0, sizeof(double) * ab, c.stream));
+  FTLM_CUDA(cudaMemsetAsync(c.sb_beta.as<double>() + c.sb_ab_used, 0, sizeof(double) * ab, c.stream));
+  pack_entries(c, rows, c.sb_ent.as<uint32_t>(), c.sb_cnt.as<int32_t>(), c.sb_diag.as<double>());
+  // start vectors: reference Gaussian ones from the host, Philox on the device
+  if (ref_start) {
+    std::vector<double> h(2 * static_cast<size_t>(start));
+    for (const Item& it : items)
+      reference_start_vectors(it.d.seed, 0, R, it.d.dim, h.data() + 2 * (it.d.start_off - c.sb_start_used));
+    pool_room(c, c.sb_start, sizeof(double2) * (c.sb_start_used + start));
+    FTLM_CUDA(cudaMemcpyAsync(c.sb_start.as<double2>() + c.sb_start_used, h.data(), sizeof(double) * h.size(),
+                              cudaMemcpyHostToDevice, c.stream));
+    FTLM_CUDA(cudaStreamSynchronize(c.stream));
+    c.prof.h2d_bytes += static_cast<int64_t>(sizeof(double) * h.size());
+  }
+  c.sb_ent_used += ent;
+  c.sb_row_used += row;
+  c.sb_start_used += start;
+  c.sb_ab_used += ab;
+  c.sb_st_used += st;
+  std::vector<SmallBlockDesc> desc;
+  for (const Item& it : items) desc.push_back(it.d);
+  if (c.spectra_defer) {  // Ritz stage with those of the other sectors, at the flush
+    small_lanczos(c, desc);
     for (const Item& it : items) {
       Spectrum s;
       s.exact = false;
-      s.prefactor = static_cast<double>(it.dim);
+      s.prefactor = static_cast<double>(it.d.dim);
       s.particles = c.sec.n_up + c.sec.n_dn;
-      s.dim = it.dim;
-      s.pending_ritz = static_cast<int>(c.defer_ritz.size());
+      s.dim = it.d.dim;
+      s.pending_small = static_cast<int>(c.defer_small.size());
       c.spec[{it.mx, it.my}] = s;
-      c.defer_ritz.push_back(DeferRitz{c.sec.n_up, c.sec.n_dn, it.mx, it.my, R, ld, it.K, ab0 + it.d.ab_off,
-                                       ab0 + ab_tot + it.d.ab_off, st0 + it.d.steps_off, it.dim, c.sec_gen});
+      c.defer_small.push_back(DeferSmall{c.sec.n_up, c.sec.n_dn, it.mx, it.my, it.d, c.sec_gen});
     }
     return;
   }
+  struct Reset {  // the rows are this call's own, whether it succeeds or throws
+    Ctx& c;
+    ~Reset() { small_rows_reset(c); }
+  } reset{c};
+  small_lanczos(c, desc);
   // Ritz values and weights per block, then compaction into the spectra arena
   std::vector<Spectrum> spec(items.size());
   std::vector<RitzJob> jobs;
-  for (size_t i = 0; i < items.size(); ++i) {
-    const Item& it = items[i];
-    jobs.push_back(RitzJob{R, R, ld, it.K, c.lz_alpha.as<double>() + it.d.ab_off,
-                           c.lz_beta.as<double>() + it.d.ab_off, c.sb_steps.as<int32_t>() + it.d.steps_off,
-                           &spec[i]});
-  }
+  for (size_t i = 0; i < items.size(); ++i) jobs.push_back(small_ritz_job(c, desc[i], &spec[i]));
   ritz_stage_many(c, jobs);
   for (size_t i = 0; i < items.size(); ++i) {
-    spec[i].prefactor = static_cast<double>(items[i].dim);
+    spec[i].prefactor = static_cast<double>(items[i].d.dim);
     spec[i].particles = c.sec.n_up + c.sec.n_dn;
-    spec[i].dim = items[i].dim;
+    spec[i].dim = items[i].d.dim;
     c.spec[{items[i].mx, items[i].my}] = spec[i];
   }
 }

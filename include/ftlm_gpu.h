@@ -140,9 +140,10 @@ int ftlm_blocks_exact_batched(ftlm_ctx* ctx, const int32_t* mx, const int32_t* m
 /* Deferred block spectra across sectors (the reference solves each block as
  * its sector loop reaches it, main.cpp:1519-1534 with 847-911 and 996-1113).
  * With on != 0, ftlm_blocks_exact_batched only assembles the exact blocks'
- * dense matrices into a device pool, ftlm_blocks_ftlm_batched keeps the
- * Lanczos coefficients of its small blocks (<= FTLM_SMALL_BLOCK_MAX rows)
- * there instead of running their Ritz stage, and
+ * dense matrices into a device pool, ftlm_blocks_ftlm_batched starts the
+ * Lanczos runs of its small blocks (<= FTLM_SMALL_BLOCK_MAX rows) on a side
+ * stream and keeps their coefficients in the pool instead of running their
+ * Ritz stage, and
  * ftlm_thermo_accumulate_block of a pooled block is queued.
  * ftlm_spectra_flush diagonalises every pooled matrix, of any number of
  * sectors, in ONE launch of the dense solver and runs the Ritz stage of every
