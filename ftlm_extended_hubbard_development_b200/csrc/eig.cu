@@ -1,15 +1,17 @@
 // Exact block spectra on the GPU (diagonalize_block_exact, main.cpp:847-911).
 //
 // Every block of the list is assembled as a dense column-major Hermitian
-// matrix straight from its hop enumeration (the CSR's entries, summed in
-// the CSR's order, with no CSR stored and no host synchronisation between
-// blocks), symmetrised as (M + M^H)/2 like the
-// reference, then all matrices are diagonalised by ONE batched launch:
-// one CTA per matrix (largest first) reduces it to real symmetric
-// tridiagonal form with complex Householder reflections (trailing
-// rank-2 updates, coalesced along columns) and finds every eigenvalue
-// independently by Sturm-sequence bisection, one thread per eigenvalue,
-// which yields them sorted ascending. Eigenvalues only (jobz = 'N').
+// matrix straight from its hop enumeration (pack.cu: the CSR's entries,
+// summed in the CSR's order, with no CSR stored), symmetrised as (M + M^H)/2
+// like the reference, then all matrices are diagonalised by ONE launch:
+// complex Householder reduction to real symmetric tridiagonal form, then every
+// eigenvalue independently by Sturm-sequence multisection, four lanes per
+// eigenvalue, which yields them sorted ascending. Eigenvalues only (jobz =
+// 'N').
+//
+// The launch is a grid of clusters. The largest matrices are reduced by a whole
+// cluster each, the others by one CTA each (eig_plan chooses the cluster size
+// and where the line lies); both kinds are taken largest first from counters.
 #include <algorithm>
 #include <cfloat>
 #include <cmath>
@@ -21,31 +23,38 @@ namespace ftlm {
 
 namespace {
 
-constexpr int kEigThreads = 256;
-constexpr int kMaxDense = 7000;  // two complex work vectors in shared memory: 2*7000*16 B <= 227 KB
+constexpr int kEigThreads = 512;
+constexpr int kEigWarps = kEigThreads / 32;
+constexpr int kEigUnroll = 4;
+constexpr int kEigCols = 1;      // columns a warp updates at once (2: within 2%, slower on clusters of 8)
+constexpr int kMaxDense = 7000;
+constexpr size_t kEigMaxSmem = 200 * 1024;  // three complex work vectors per CTA, else in global memory
 
-__device__ double block_sum(double v, double* red) {
+// Fixed-order sum over the CTA, the same in every thread. Consecutive calls
+// alternate between the two halves of red.
+__device__ __forceinline__ double block_sum(double v, double (*red)[kEigWarps], int& flip) {
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  __syncthreads();
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+  double* r = red[flip];
+  flip ^= 1;
+  if ((threadIdx.x & 31) == 0) r[threadIdx.x >> 5] = v;
   __syncthreads();
   double s = 0.0;
-  for (int w = 0; w < kEigThreads / 32; ++w) s += red[w];
-  __syncthreads();
+#pragma unroll
+  for (int w = 0; w < kEigWarps; ++w) s += r[w];
   return s;
 }
 
-__device__ double block_minmax(double v, double* red, bool is_max) {
+__device__ __forceinline__ double block_minmax(double v, double (*red)[kEigWarps], int& flip, bool is_max) {
   for (int o = 16; o > 0; o >>= 1) {
     const double t = __shfl_xor_sync(0xffffffffu, v, o);
     v = is_max ? fmax(v, t) : fmin(v, t);
   }
+  double* r = red[flip];
+  flip ^= 1;
+  if ((threadIdx.x & 31) == 0) r[threadIdx.x >> 5] = v;
   __syncthreads();
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
-  __syncthreads();
-  double s = red[0];
-  for (int w = 1; w < kEigThreads / 32; ++w) s = is_max ? fmax(s, red[w]) : fmin(s, red[w]);
-  __syncthreads();
+  double s = r[0];
+  for (int w = 1; w < kEigWarps; ++w) s = is_max ? fmax(s, r[w]) : fmin(s, r[w]);
   return s;
 }
 
@@ -62,128 +71,260 @@ __device__ int sturm_count(int n, const double* d, const double* e2, double x, d
   return cnt;
 }
 
-// One CTA per matrix. work: per matrix 2*n doubles (d, e2) at woff.
-__global__ void __launch_bounds__(kEigThreads) k_dense_eig(int nmat, const int32_t* __restrict__ order,
-                                                          const int32_t* __restrict__ dims,
-                                                          const int64_t* __restrict__ aoff, double2* __restrict__ arena,
-                                                          const int64_t* __restrict__ eoff, double* __restrict__ evout,
-                                                          double* __restrict__ work, const int64_t* __restrict__ woff) {
-  extern __shared__ double2 sh[];
-  __shared__ double red[kEigThreads / 32];
-  for (int task = blockIdx.x; task < nmat; task += gridDim.x) {
-    const int mi = order[task];
-    const int n = dims[mi];
-    double2* A = arena + aoff[mi];
-    double* d = work + woff[mi];
-    double* e2 = d + n;
-    double2* v = sh;
-    double2* w = sh + n;
-    const int tid = threadIdx.x;
-    for (int k = 0; k + 2 < n; ++k) {
-      const int m = n - k - 1;
-      const int64_t base = (k + 1) + static_cast<int64_t>(k) * n;  // A[k+1][k]
-      double s2 = 0.0;
-      for (int i = tid; i < m; i += kEigThreads) {
-        const double2 x = A[base + i];
-        s2 += x.x * x.x + x.y * x.y;
-      }
-      const double alpha = sqrt(block_sum(s2, red));
-      if (tid == 0) d[k] = A[k + static_cast<int64_t>(k) * n].x;
-      if (alpha == 0.0) {
-        if (tid == 0) e2[k] = 0.0;
-        __syncthreads();
-        continue;
-      }
-      const double2 x0 = A[base];
-      const double ax0 = hypot(x0.x, x0.y);
-      const double phr = ax0 > 0.0 ? x0.x / ax0 : 1.0;
-      const double phi = ax0 > 0.0 ? x0.y / ax0 : 0.0;
-      for (int i = tid; i < m; i += kEigThreads) {
-        double2 x = A[base + i];
-        if (i == 0) {
-          x.x += phr * alpha;
-          x.y += phi * alpha;
-        }
-        v[i] = x;
-      }
-      const double tau = 1.0 / (alpha * (alpha + ax0));  // 2 / |v|^2
-      __syncthreads();
-      // p = tau * B v, B = A[k+1.., k+1..] (thread per row, columns in order)
-      const int64_t b0 = (k + 1) + static_cast<int64_t>(k + 1) * n;
-      double kr = 0.0;
-      for (int i = tid; i < m; i += kEigThreads) {
-        double pr = 0.0, pi = 0.0;
-        for (int j = 0; j < m; ++j) {
-          const double2 b = A[b0 + i + static_cast<int64_t>(j) * n];
-          const double2 vj = v[j];
-          pr += b.x * vj.x - b.y * vj.y;
-          pi += b.x * vj.y + b.y * vj.x;
-        }
-        pr *= tau;
-        pi *= tau;
-        w[i] = make_double2(pr, pi);
-        kr += v[i].x * pr + v[i].y * pi;  // Re(conj(v_i) p_i)
-      }
-      const double K = 0.5 * tau * block_sum(kr, red);
-      for (int i = tid; i < m; i += kEigThreads) {
-        w[i].x -= K * v[i].x;
-        w[i].y -= K * v[i].y;
-      }
-      __syncthreads();
-      // B -= v w^H + w v^H
-      for (int j = 0; j < m; ++j) {
-        const double2 vj = v[j], wj = w[j];
-        for (int i = tid; i < m; i += kEigThreads) {
-          const double2 vi = v[i], wi = w[i];
-          double2& b = A[b0 + i + static_cast<int64_t>(j) * n];
-          b.x -= (vi.x * wj.x + vi.y * wj.y) + (wi.x * vj.x + wi.y * vj.y);
-          b.y -= (vi.y * wj.x - vi.x * wj.y) + (wi.y * vj.x - wi.x * vj.y);
-        }
-      }
-      if (tid == 0) e2[k] = alpha * alpha;
-      __syncthreads();
-    }
-    if (tid == 0) {
-      if (n >= 2) {
-        d[n - 2] = A[(n - 2) + static_cast<int64_t>(n - 2) * n].x;
-        const double2 t = A[(n - 1) + static_cast<int64_t>(n - 2) * n];
-        e2[n - 2] = t.x * t.x + t.y * t.y;
-      }
-      d[n - 1] = A[(n - 1) + static_cast<int64_t>(n - 1) * n].x;
-      e2[n - 1] = 0.0;
-    }
-    __syncthreads();
-    // Gershgorin interval and bisection
-    double lo = DBL_MAX, hi = -DBL_MAX, emax = 0.0;
-    for (int i = tid; i < n; i += kEigThreads) {
-      const double el = i > 0 ? sqrt(e2[i - 1]) : 0.0;
-      const double er = i + 1 < n ? sqrt(e2[i]) : 0.0;
-      lo = fmin(lo, d[i] - el - er);
-      hi = fmax(hi, d[i] + el + er);
-      emax = fmax(emax, e2[i]);
-    }
-    lo = block_minmax(lo, red, false);
-    hi = block_minmax(hi, red, true);
-    emax = block_minmax(emax, red, true);
-    const double pivmin = DBL_MIN * fmax(1.0, emax);
-    const double span = fmax(fabs(lo), fabs(hi));
-    lo -= 4.0 * DBL_EPSILON * span + pivmin;
-    hi += 4.0 * DBL_EPSILON * span + pivmin;
-    double* ev = evout + eoff[mi];
-    for (int j = tid; j < n; j += kEigThreads) {
-      double a = lo, b = hi;
-      for (int it = 0; it < 128; ++it) {
-        const double mid = 0.5 * (a + b);
-        if (mid <= a || mid >= b) break;
-        if (b - a <= 2.0 * DBL_EPSILON * fmax(fabs(a), fabs(b))) break;
-        if (sturm_count(n, d, e2, mid, pivmin) > j) b = mid;
-        else a = mid;
-      }
-      ev[j] = 0.5 * (a + b);
-    }
+__device__ __forceinline__ void group_sync(bool cluster) {
+  if (cluster) {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  } else {
     __syncthreads();
   }
 }
+
+__device__ __forceinline__ double2 ld_cg(const double2* p) { return __ldcg(p); }
+
+// One matrix, by the nr CTAs of a group (a cluster, or one CTA with nr = 1).
+// work: d[n], e2[n], then two complex vectors p[2][n] through which the CTAs
+// exchange B v; v, w, u: this CTA's own complex work vectors.
+//
+// Step k reflects column k of the trailing matrix. The rank-2 update of step
+// k - 1 is applied while step k's product B v is formed, so the matrix is read
+// and written once per step: the update of column k alone gives the next
+// reflector u (every CTA computes it, from the same numbers in the same
+// order), then each warp takes its columns j, applies - v w^H - w v^H, stores
+// them, and adds up (B u)_j = sum_i conj(B_ij) u_i, which needs no other column.
+// One barrier per step, after which every CTA forms w from the whole product.
+// Columns stay with the same warp throughout. Bound: L2 traffic, 32 bytes per
+// trailing element and step, and 4-6 us of barriers and dependent sums per
+// step. Against one 256-thread CTA per matrix with B v and the update in
+// separate passes: 620 matrices up to 622 rows (4x2 ED curve) 325 -> 29 ms,
+// nine of 1764 rows 7625 -> 299 ms, nine of 336 rows 49 -> 3.3 ms.
+__device__ void dense_eig(int n, double2* __restrict__ A, double* __restrict__ work, double* __restrict__ ev,
+                          double2* v, double2* w, double2* u, int rank, int nr, double (*red)[kEigWarps], int& flip) {
+  double* d = work;
+  double* e2 = work + n;
+  double2* pbuf = reinterpret_cast<double2*>(work + 2 * n);
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int gwarp = rank * kEigWarps + (tid >> 5), nwarps = nr * kEigWarps;
+  const bool cluster = nr > 1;
+  for (int i = tid; i < n; i += kEigThreads) v[i] = w[i] = make_double2(0.0, 0.0);
+  __syncthreads();
+  for (int k = 0; k + 2 < n; ++k) {
+    const int m = n - k - 1;
+    const double2* col = A + k + static_cast<int64_t>(k) * n;  // A[k][k]
+    const double2 v0 = v[0], w0 = w[0];
+    // column k with the pending update, its norm
+    double s2 = 0.0;
+    for (int i = tid; i < m; i += kEigThreads) {
+      double2 x = ld_cg(col + 1 + i);
+      const double2 vi = v[i + 1], wi = w[i + 1];
+      x.x -= (vi.x * w0.x + vi.y * w0.y) + (wi.x * v0.x + wi.y * v0.y);
+      x.y -= (vi.y * w0.x - vi.x * w0.y) + (wi.y * v0.x - wi.x * v0.y);
+      u[i] = x;
+      s2 += x.x * x.x + x.y * x.y;
+    }
+    const double alpha = sqrt(block_sum(s2, red, flip));
+    if (rank == 0 && tid == 0) {
+      d[k] = ld_cg(col).x - 2.0 * (v0.x * w0.x + v0.y * w0.y);
+      e2[k] = alpha * alpha;
+    }
+    const double2 x0 = u[0];
+    const double ax0 = hypot(x0.x, x0.y);
+    const double tau = alpha > 0.0 ? 1.0 / (alpha * (alpha + ax0)) : 0.0;  // 2 / |u|^2; 0: nothing to reflect
+    __syncthreads();  // every thread has read u[0]
+    if (tid == 0) {
+      const double phr = ax0 > 0.0 ? x0.x / ax0 : 1.0;
+      const double phi = ax0 > 0.0 ? x0.y / ax0 : 0.0;
+      u[0] = make_double2(x0.x + phr * alpha, x0.y + phi * alpha);
+    }
+    __syncthreads();
+    // pending update of the columns behind, and their products with u
+    double2* p = pbuf + static_cast<int64_t>(k & 1) * n;
+    const int c0 = k + 1;
+    int g = (c0 / kEigCols) / nwarps * nwarps + gwarp;  // this warp's column groups: g = gwarp (mod nwarps)
+    if (g < c0 / kEigCols) g += nwarps;
+    for (; g * kEigCols < n; g += nwarps) {
+      double2* a[kEigCols];
+      double2 wj[kEigCols], vj[kEigCols], s[kEigCols];
+      bool on[kEigCols];
+#pragma unroll
+      for (int c = 0; c < kEigCols; ++c) {
+        const int cc = g * kEigCols + c;
+        on[c] = cc >= c0 && cc < n;
+        const int j = on[c] ? cc - c0 : 0;
+        a[c] = A + c0 + static_cast<int64_t>(on[c] ? cc : c0) * n;
+        wj[c] = w[j + 1];
+        vj[c] = v[j + 1];
+        s[c] = make_double2(0.0, 0.0);
+      }
+#pragma unroll kEigUnroll
+      for (int i = lane; i < m; i += 32) {
+        const double2 vi = v[i + 1], wi = w[i + 1], ui = u[i];
+#pragma unroll
+        for (int c = 0; c < kEigCols; ++c) {
+          if (!on[c]) continue;
+          double2 b = a[c][i];
+          b.x -= (vi.x * wj[c].x + vi.y * wj[c].y) + (wi.x * vj[c].x + wi.y * vj[c].y);
+          b.y -= (vi.y * wj[c].x - vi.x * wj[c].y) + (wi.y * vj[c].x - wi.x * vj[c].y);
+          a[c][i] = b;
+          s[c].x += b.x * ui.x + b.y * ui.y;
+          s[c].y += b.x * ui.y - b.y * ui.x;
+        }
+      }
+#pragma unroll
+      for (int c = 0; c < kEigCols; ++c) {
+        for (int o = 16; o > 0; o >>= 1) {
+          s[c].x += __shfl_xor_sync(0xffffffffu, s[c].x, o);
+          s[c].y += __shfl_xor_sync(0xffffffffu, s[c].y, o);
+        }
+        if (lane == 0 && on[c]) __stcg(p + (g * kEigCols + c - c0), make_double2(tau * s[c].x, tau * s[c].y));
+      }
+    }
+    group_sync(cluster);
+    // w = p - (tau/2)(u^H p) u; v <- u
+    double kr = 0.0;
+    for (int i = tid; i < m; i += kEigThreads) {
+      const double2 pi = ld_cg(p + i), ui = u[i];
+      w[i] = pi;
+      kr += ui.x * pi.x + ui.y * pi.y;
+    }
+    const double K = 0.5 * tau * block_sum(kr, red, flip);
+    for (int i = tid; i < m; i += kEigThreads) {
+      const double2 ui = u[i];
+      w[i] = make_double2(w[i].x - K * ui.x, w[i].y - K * ui.y);
+    }
+    double2* t = v;
+    v = u;
+    u = t;
+    __syncthreads();
+  }
+  if (rank == 0 && tid == 0) {  // the last 2x2 (or 1x1) with the pending update
+    const double2 v0 = v[0], w0 = w[0];
+    if (n >= 2) {
+      const double2* c = A + (n - 2) + static_cast<int64_t>(n - 2) * n;
+      const double2 v1 = v[1], w1 = w[1];
+      const double2 t = ld_cg(c + 1);
+      const double tr = t.x - ((v1.x * w0.x + v1.y * w0.y) + (w1.x * v0.x + w1.y * v0.y));
+      const double ti = t.y - ((v1.y * w0.x - v1.x * w0.y) + (w1.y * v0.x - w1.x * v0.y));
+      d[n - 2] = ld_cg(c).x - 2.0 * (v0.x * w0.x + v0.y * w0.y);
+      d[n - 1] = ld_cg(c + n + 1).x - 2.0 * (v1.x * w1.x + v1.y * w1.y);
+      e2[n - 2] = tr * tr + ti * ti;
+    } else {
+      d[0] = ld_cg(A).x;
+    }
+    e2[n - 1] = 0.0;
+  }
+  group_sync(cluster);
+  // tridiagonal matrix beside the CTA: d in v, e2 in w (as doubles)
+  double* ds = reinterpret_cast<double*>(v);
+  double* es = reinterpret_cast<double*>(w);
+  for (int i = tid; i < n; i += kEigThreads) {
+    ds[i] = __ldcg(d + i);
+    es[i] = __ldcg(e2 + i);
+  }
+  __syncthreads();
+  // Gershgorin interval and multisection
+  double lo = DBL_MAX, hi = -DBL_MAX, emax = 0.0;
+  for (int i = tid; i < n; i += kEigThreads) {
+    const double el = i > 0 ? sqrt(es[i - 1]) : 0.0;
+    const double er = i + 1 < n ? sqrt(es[i]) : 0.0;
+    lo = fmin(lo, ds[i] - el - er);
+    hi = fmax(hi, ds[i] + el + er);
+    emax = fmax(emax, es[i]);
+  }
+  lo = block_minmax(lo, red, flip, false);
+  hi = block_minmax(hi, red, flip, true);
+  emax = block_minmax(emax, red, flip, true);
+  const double pivmin = DBL_MIN * fmax(1.0, emax);
+  const double span = fmax(fabs(lo), fabs(hi));
+  lo -= 4.0 * DBL_EPSILON * span + pivmin;
+  hi += 4.0 * DBL_EPSILON * span + pivmin;
+  // four lanes per eigenvalue j count at the inner points of a fifth each: the
+  // j-th eigenvalue lies below the first point with more than j below it
+  const int sub = lane & 3;
+  const int quads = nr * kEigThreads / 4;
+  for (int j0 = 0; j0 < n; j0 += quads) {
+    const int j = j0 + (rank * kEigThreads + tid) / 4;
+    const bool real = j < n;
+    double a = lo, b = hi;
+    bool run = real;
+    for (int it = 0; it < 64; ++it) {
+      run = run && b - a > 2.0 * DBL_EPSILON * fmax(fabs(a), fabs(b));
+      const double x = a + (b - a) * (0.2 * (sub + 1));
+      const bool inside = x > a && x < b;
+      int above = 0;
+      if (run && inside) above = sturm_count(n, ds, es, x, pivmin) > j;
+      const unsigned ok = __ballot_sync(0xffffffffu, inside) >> (lane & ~3) & 15u;
+      const unsigned m = __ballot_sync(0xffffffffu, above) >> (lane & ~3) & 15u;
+      if (run && ok != 15u) {
+        // the interval no longer holds four inner points: finish by halves
+        const double mid = 0.5 * (a + b);
+        if (mid <= a || mid >= b) run = false;
+        else if (sturm_count(n, ds, es, mid, pivmin) > j) b = mid;
+        else a = mid;
+      } else if (run) {
+        const int f = m ? __ffs(m) - 1 : 4;  // counts grow with x: first point with more than j below
+        const double w5 = b - a;
+        const double na = f > 0 ? a + w5 * (0.2 * f) : a;
+        if (f < 4) b = a + w5 * (0.2 * (f + 1));
+        a = na;
+      }
+      if (!__any_sync(0xffffffffu, run)) break;
+    }
+    if (real && sub == 0) ev[j] = 0.5 * (a + b);
+  }
+  group_sync(cluster);  // the work vectors are free for the next matrix
+}
+
+struct EigArgs {
+  int nmat, nlarge;        // matrices, those taken by clusters (the first of `order`)
+  const int32_t* order;    // largest first
+  const int32_t* dims;
+  const int64_t* aoff;
+  const int64_t* eoff;
+  const int64_t* woff;
+  double2* arena;
+  double* evout;
+  double* work;
+  double2* vecs;           // per CTA three vectors of nmax, null: shared memory
+  int64_t nmax;
+  int* counters;           // [2], zeroed: next large, next small matrix
+  int* slots;              // [clusters][2]
+  int cluster;             // CTAs per cluster
+};
+
+__global__ void __launch_bounds__(kEigThreads) k_dense_eig(const __grid_constant__ EigArgs P) {
+  extern __shared__ double2 sh[];
+  __shared__ double red[2][kEigWarps];
+  __shared__ int s_next;
+  int flip = 0;
+  const int rank = blockIdx.x % P.cluster, tid = threadIdx.x;
+  double2* v = P.vecs ? P.vecs + static_cast<int64_t>(blockIdx.x) * 3 * P.nmax : sh;
+  double2* w = v + P.nmax;
+  double2* u = w + P.nmax;
+  // matrices of whole clusters: rank 0 takes the next one for all
+  int* slot = P.slots + 2 * (blockIdx.x / P.cluster);
+  for (int it = 0; P.nlarge > 0; ++it) {
+    if (rank == 0 && tid == 0) __stcg(slot + (it & 1), atomicAdd(P.counters, 1));
+    group_sync(true);
+    const int t = __ldcg(slot + (it & 1));
+    if (t >= P.nlarge) break;
+    const int mi = P.order[t];
+    dense_eig(P.dims[mi], P.arena + P.aoff[mi], P.work + P.woff[mi], P.evout + P.eoff[mi], v, w, u, rank, P.cluster,
+              red, flip);
+  }
+  // the rest, one CTA each
+  while (true) {
+    __syncthreads();
+    if (tid == 0) s_next = P.nlarge + atomicAdd(P.counters + 1, 1);
+    __syncthreads();
+    const int t = s_next;
+    if (t >= P.nmat) break;
+    const int mi = P.order[t];
+    dense_eig(P.dims[mi], P.arena + P.aoff[mi], P.work + P.woff[mi], P.evout + P.eoff[mi], v, w, u, 0, 1, red, flip);
+  }
+}
+
+constexpr int64_t kWorkPerRow = 6;  // doubles of dense_eig work space per row: d, e2, p[2] complex
 
 struct DenseItem {
   int mx, my;
@@ -201,7 +342,7 @@ std::vector<DenseItem> dense_items(Ctx& c, const std::vector<std::pair<int, int>
     if (n > kMaxDense) throw Error(FTLM_ERR_CAPACITY, "block too large for the dense exact solver: " + std::to_string(n));
     items.push_back({b.first, b.second, n, asz, wsz});
     asz += n * n;
-    wsz += 2 * n;
+    wsz += kWorkPerRow * n;
   }
   return items;
 }
@@ -220,8 +361,43 @@ void dense_fill(Ctx& c, const std::vector<DenseItem>& items, double2* arena, int
   pack_dense(c, rows, arena);
 }
 
+struct EigPlan {
+  int cluster, nlarge;
+};
+
+// Cluster size and number of matrices (the first of `order`) given to whole
+// clusters: those with the smallest modelled time. A column costs a CTA 4 us
+// of dependent sums, a cluster 6 us, and n^2 / cluster * 2.5e-4 us of memory
+// traffic (fitted to 336-row matrices: 20, 13 and 10 us a column on 2, 4 and 8
+// CTAs). One cluster size does not fit all: the exact blocks of a 4x2 curve up
+// to 256 rows take 4.4 ms on clusters of 2 and 10.9 on 8, nine matrices of
+// 1764 rows 986 ms on 2 and 299 on 8, the whole 4x2 ED curve 44, 30 and 39 ms
+// on 2, 4 and 8.
+EigPlan eig_plan(const std::vector<int32_t>& dims, const std::vector<int32_t>& order, int sms) {
+  auto cost = [](double n, int cs) { return n * ((cs > 1 ? 6.0 : 4.0) + n * n * 2.5e-4 / cs); };
+  std::vector<double> single(order.size() + 1, 0.0);  // [i]: the matrices from i on, one CTA each
+  for (size_t i = order.size(); i-- > 0;) single[i] = single[i + 1] + cost(dims[order[i]], 1);
+  auto phase = [](double sum, int slots, double most) { return std::max(sum / slots, most); };
+  EigPlan best{1, 0};
+  double t = phase(single[0], sms, cost(dims[order[0]], 1));
+  for (int cs = 2; cs <= 8; cs *= 2) {
+    double sum = 0.0;
+    for (size_t i = 0; i < order.size(); ++i) {
+      sum += cost(dims[order[i]], cs);
+      const bool rest = i + 1 < order.size();
+      const double tt = phase(sum, sms / cs, cost(dims[order[0]], cs)) +
+                        (rest ? phase(single[i + 1], sms, cost(dims[order[i + 1]], 1)) : 0.0);
+      if (tt < t) {
+        t = tt;
+        best = {cs, static_cast<int>(i + 1)};
+      }
+    }
+  }
+  return best;
+}
+
 // One k_dense_eig launch over matrices (dims, aoff into arena) writing the
-// eigenvalues at evout + eoff; largest matrix first, one CTA per matrix.
+// eigenvalues at evout + eoff; work: kWorkPerRow doubles per row.
 void dense_solve(Ctx& c, const std::vector<int32_t>& dims, const std::vector<int64_t>& aoff,
                  const std::vector<int64_t>& eoff, double2* arena, double* evout, double* work) {
   const size_t nb = dims.size();
@@ -229,33 +405,68 @@ void dense_solve(Ctx& c, const std::vector<int32_t>& dims, const std::vector<int
   std::vector<int32_t> order(nb);
   std::vector<int64_t> woff(nb);
   int64_t nmax = 0, wtot = 0;
+  EigArgs P{};
   for (size_t i = 0; i < nb; ++i) {
     woff[i] = wtot;
-    wtot += 2 * static_cast<int64_t>(dims[i]);
+    wtot += kWorkPerRow * static_cast<int64_t>(dims[i]);
     nmax = std::max<int64_t>(nmax, dims[i]);
   }
   std::iota(order.begin(), order.end(), 0);
   std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return dims[a] > dims[b]; });
-  const size_t i32bytes = ((sizeof(int32_t) * 2 * nb + 7) / 8) * 8;  // int64 arrays stay 8-byte aligned
+  const EigPlan plan = eig_plan(dims, order, c.sm_count);
+  P.cluster = plan.cluster;
+  P.nlarge = plan.nlarge;
+  // clusters: enough for the large matrices or one small one per CTA, at most one CTA per SM
+  const int want = std::max<int>(P.nlarge, static_cast<int>((nb - P.nlarge + P.cluster - 1) / P.cluster));
+  const int clusters = std::max(1, std::min(want, c.sm_count / P.cluster));
+  const size_t i32bytes = ((sizeof(int32_t) * (2 * nb + 2 + 2 * clusters) + 7) / 8) * 8;  // int64 arrays stay aligned
   c.dense_meta.ensure(i32bytes + sizeof(int64_t) * 3 * nb);
-  int32_t* d_order = c.dense_meta.as<int32_t>();
+  int32_t* d_ctr = c.dense_meta.as<int32_t>();
+  int32_t* d_order = d_ctr + 2 + 2 * clusters;
   int32_t* d_dims = d_order + nb;
   int64_t* d_aoff = reinterpret_cast<int64_t*>(c.dense_meta.as<char>() + i32bytes);
   int64_t* d_eoff = d_aoff + nb;
   int64_t* d_woff = d_eoff + nb;
+  FTLM_CUDA(cudaMemsetAsync(d_ctr, 0, sizeof(int32_t) * (2 + 2 * clusters), c.stream));
   FTLM_CUDA(cudaMemcpyAsync(d_order, order.data(), sizeof(int32_t) * nb, cudaMemcpyHostToDevice, c.stream));
   FTLM_CUDA(cudaMemcpyAsync(d_dims, dims.data(), sizeof(int32_t) * nb, cudaMemcpyHostToDevice, c.stream));
   FTLM_CUDA(cudaMemcpyAsync(d_aoff, aoff.data(), sizeof(int64_t) * nb, cudaMemcpyHostToDevice, c.stream));
   FTLM_CUDA(cudaMemcpyAsync(d_eoff, eoff.data(), sizeof(int64_t) * nb, cudaMemcpyHostToDevice, c.stream));
   FTLM_CUDA(cudaMemcpyAsync(d_woff, woff.data(), sizeof(int64_t) * nb, cudaMemcpyHostToDevice, c.stream));
   c.prof.h2d_bytes += static_cast<int64_t>(nb) * 32;
-  const size_t smem = sizeof(double2) * 2 * static_cast<size_t>(nmax);
-  if (smem > 48 * 1024)
-    FTLM_CUDA(cudaFuncSetAttribute(k_dense_eig, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-  const int grid = static_cast<int>(std::min<size_t>(nb, static_cast<size_t>(c.sm_count) * 4));
-  k_dense_eig<<<grid, kEigThreads, smem, c.stream>>>(static_cast<int>(nb), d_order, d_dims, d_aoff, arena, d_eoff,
-                                                     evout, work, d_woff);
-  FTLM_LAUNCH_CHECK();
+  P.nmat = static_cast<int>(nb);
+  P.order = d_order;
+  P.dims = d_dims;
+  P.aoff = d_aoff;
+  P.eoff = d_eoff;
+  P.woff = d_woff;
+  P.arena = arena;
+  P.evout = evout;
+  P.work = work;
+  P.nmax = std::max<int64_t>(nmax, 2);  // the reduction reads v[0], v[1] of any matrix
+  P.counters = d_ctr;
+  P.slots = d_ctr + 2;
+  size_t smem = sizeof(double2) * 3 * static_cast<size_t>(P.nmax);
+  if (smem > kEigMaxSmem) {
+    c.dense_vecs.ensure(smem * clusters * P.cluster);
+    P.vecs = c.dense_vecs.as<double2>();
+    smem = 0;
+  }
+  FTLM_CUDA(cudaFuncSetAttribute(k_dense_eig, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 static_cast<int>(std::max(smem, size_t(48) << 10))));
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(clusters * P.cluster);
+  cfg.blockDim = dim3(kEigThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = c.stream;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = P.cluster;
+  at.val.clusterDim.y = 1;
+  at.val.clusterDim.z = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  FTLM_CUDA(cudaLaunchKernelEx(&cfg, k_dense_eig, P));
   c.prof.kernel_launches += 1;
 }
 
@@ -378,7 +589,7 @@ void flush_deferred(Ctx& c) {
       etot += c.defer_items[i].n;
     }
     c.defer_ev.ensure(sizeof(double) * etot);
-    c.defer_work.ensure(sizeof(double) * 2 * etot);
+    c.defer_work.ensure(sizeof(double) * kWorkPerRow * etot);
     EventTimer t(c, c.prof.eig_ms);
     dense_solve(c, dims, aoff, eoff, c.defer_arena.as<double2>(), c.defer_ev.as<double>(), c.defer_work.as<double>());
     t.stop();

@@ -287,7 +287,7 @@ struct Ctx {
   DBuf vec_a, vec_b, vec_h, partial, lz_alpha, lz_beta, lz_scale, lz_state, host_start;
   DBuf ritz_tmp, ritz_out, ritz_meta, scan_tmp;
   // exact batch
-  DBuf dense_arena, dense_meta, dense_out;
+  DBuf dense_arena, dense_meta, dense_out, dense_vecs;
   // deferred block spectra (ftlm_spectra_defer): dense matrices of exact
   // blocks and rows of small FTLM blocks of any number of sectors, solved
   // together by flush_deferred, then the queued accumulations

@@ -47,6 +47,49 @@ def test_exact_blocks_of_a_sector(sector):
             assert np.abs(ev - O.block_exact(csr)).max() <= max(tol, 1e-14), (mx, my)
 
 
+# one size alone and several together: matrices of whole clusters (of 2, 4 and
+# 8 CTAs) beside matrices of one CTA
+@pytest.mark.parametrize("sector,count", [((3, 3, 2, 3), 1), ((3, 3, 2, 3), 9), ((4, 2, 3, 4), 3), ((4, 2, 2, 3), 8),
+                                          ((3, 3, 3, 3), 2), ((3, 3, 3, 4), 1)],
+                         ids=lambda x: "%dx%d_%d_%d" % x if isinstance(x, tuple) else "x%d" % x)
+def test_dense_solver_by_clusters(sector, count):
+    lx, ly, nu, nd = sector
+    m = model(lx, ly)
+    om = O.Model(**m.__dict__)
+    with pkg.Engine(m) as eng:
+        eng.spectra_defer(True)
+        eng.sector_prepare(1, 1)  # small matrices in the same launch
+        eng.blocks_exact_batched([(k % lx, k // lx) for k in range(lx * ly)])
+        eng.sector_prepare(nu, nd)
+        blocks = [(k % lx, k // lx) for k in range(count)]
+        eng.blocks_exact_batched(blocks)
+        for mx, my in blocks:
+            csr = O.block_csr(om, nu, nd, mx, my)
+            ev, _, _ = eng.block_spectrum(mx, my, exact=True)
+            rows = np.abs(csr.diag) + np.add.reduceat(np.abs(csr.val), csr.row_ptr[:-1])
+            assert np.all(np.diff(ev) >= 0)
+            assert np.abs(ev - O.block_exact(csr)).max() <= csr.dim * 2.0 ** -53 * rows.max() * 4, (mx, my)
+        eng.spectra_defer(False)
+
+
+def test_dense_solver_with_work_vectors_in_global_memory():
+    """4324 rows: three work vectors no longer fit in shared memory. Sum and
+    sum of squares of the eigenvalues against trace and Frobenius norm."""
+    m = model(7, 7)
+    csr = O.block_csr(O.Model(**m.__dict__), 0, 4, 1, 2)
+    with pkg.Engine(m) as eng:
+        eng.sector_prepare(0, 4)
+        ev, _, _ = eng.block_spectrum(1, 2, exact=True)
+    assert len(ev) == csr.dim > 4266 and np.all(np.diff(ev) >= 0)
+    row = np.repeat(np.arange(csr.dim), np.diff(csr.row_ptr))
+    import scipy.sparse as sp
+    h = sp.csr_matrix((csr.val, (row, csr.col)), shape=(csr.dim, csr.dim)) + sp.diags(csr.diag)
+    norm = abs(h).sum(1).max()
+    each = csr.dim * 2.0 ** -53 * norm  # per eigenvalue
+    assert abs(ev.sum() - h.diagonal().real.sum()) <= csr.dim * each
+    assert abs((ev ** 2).sum() - (abs(h).power(2)).sum()) <= 2 * csr.dim * norm * each
+
+
 # dims around 512 and 1024, and one far above
 FTLM = [(4, 2, 3, 4, 2, 0), (3, 3, 2, 5, 1, 1), (3, 3, 3, 3, 0, 0), (3, 3, 3, 4, 2, 2), (4, 3, 2, 4, 1, 2),
         (9, 5, 0, 4, 2, 1)]
