@@ -162,7 +162,6 @@ int ftlm_ctx_create(const ftlm_model* model, const ftlm_run_opts* opts, ftlm_ctx
   if (const char* rt = std::getenv("FTLM_HV_RETUNE")) c.hv_retune = std::string(rt) == "1";
   if (const char* sr = std::getenv("FTLM_SEG_ROWS")) c.seg_dynamic = std::string(sr) != "stride";
   if (const char* so = std::getenv("FTLM_SPLIT_OP")) c.split_stencil = std::string(so) != "fly";
-  if (const char* sr2 = std::getenv("FTLM_STN_ROWS")) c.stn_rows = std::string(sr2) != "0";
   if (const char* hm = std::getenv("FTLM_HV_MODE")) {
     const std::string m(hm);
     c.hv_mode = m == "list" ? ftlm::kSrcList : m == "fly" ? ftlm::kSrcFly : m == "split" ? ftlm::kSrcSplit : -1;
@@ -210,8 +209,8 @@ void ftlm_ctx_destroy(ftlm_ctx* ctx) {
                         &c.pack.act, &c.pack.act_list, &c.pack.dtab, &c.pack.aoff, &c.pack.nact, &c.pack.dims,
                         &c.pack.row_meta, &c.pack.row_dn, &c.pack.phase, &c.pack.items,
                         &c.scan_tmp, &c.dense_arena, &c.dense_meta, &c.dense_out, &c.dense_vecs, &c.spectra, &c.th_beta,
-                        &c.th_mu, &c.th_state, &c.hl_ptr, &c.hl_ent, &c.flip_map, &c.vec_xd, &c.vec_yd, &c.seg_counter, &c.stn_crb, &c.stn_rp, &c.stn_rp32, &c.stn_ent, &c.stn_cnt,
-                        &c.stn_rp4, &c.stn_row, &c.stn_ent4, &c.stn_deg, &c.stn_coef, &c.stn_seg, &c.stn_cls, &c.stn_diag,
+                        &c.th_mu, &c.th_state, &c.hl_ptr, &c.hl_ent, &c.flip_map, &c.vec_xd, &c.vec_yd, &c.seg_counter, &c.stn_crb, &c.stn_rp, &c.stn_ent, &c.stn_cnt,
+                        &c.stn_rp4, &c.stn_row, &c.stn_ent4, &c.stn_deg, &c.stn_coef, &c.stn_seg, &c.stn_cls, &c.stn_pos, &c.stn_diag,
                         &c.defer_arena, &c.defer_ev, &c.defer_work};
   for (auto* b : bufs) b->release();
   if (c.flipped) {
@@ -220,8 +219,8 @@ void ftlm_ctx_destroy(ftlm_ctx* ctx) {
                         &f.sec.d_star, &f.sec.d_hs, &f.sec.d_stab, &f.sec.d_chi, &f.sec.d_cidx, &f.sec.canon,
                         &f.sec.tmp_a, &f.sec.tmp_b, &f.sec.tmp_c, &f.sec.tmp_d, &f.sec.tmp_e, &f.blk.act,
                         &f.blk.act_list, &f.blk.aoff, &f.blk.dtab, &f.blk.row_meta, &f.blk.row_dn, &f.scan_tmp,
-                        &f.stn_crb, &f.stn_rp, &f.stn_rp32, &f.stn_ent, &f.stn_cnt,
-                        &f.stn_rp4, &f.stn_row, &f.stn_ent4, &f.stn_deg, &f.stn_coef, &f.stn_seg, &f.stn_cls, &f.stn_diag};
+                        &f.stn_crb, &f.stn_rp, &f.stn_ent, &f.stn_cnt,
+                        &f.stn_rp4, &f.stn_row, &f.stn_ent4, &f.stn_deg, &f.stn_coef, &f.stn_seg, &f.stn_cls, &f.stn_pos, &f.stn_diag};
     for (auto* b : fb) b->release();  // binom tables are the owner's
     c.flipped.reset();
   }
@@ -452,9 +451,13 @@ int ftlm_block_apply(ftlm_ctx* ctx, int32_t mx, int32_t my, int32_t nvec, const 
     ftlm::block_prepare(c, mx, my);
     const int64_t D = c.blk.dim;
     if (D == 0) return;
+    ftlm::HvSourceGuard guard{c};
+    c.prof.hv_source = ftlm::hv_select_source(c, ftlm::sweep_width(nvec, fp32), fp32);
+    const bool reorder = ftlm::sweep_pos(c) != nullptr;
+    if (reorder) NV = ftlm::sweep_width(nvec, fp32);
     const size_t esize = fp32 ? 8 : 16;
     const size_t bytes = static_cast<size_t>(D) * NV * esize;
-    c.vec_a.ensure(bytes);
+    c.vec_a.ensure(bytes + ftlm::kSweepPad);
     c.vec_h.ensure(bytes);
     // pack host [dim][nvec] FP64 complex into [dim][NV] of the working precision
     std::vector<char> h(bytes, 0);
@@ -471,10 +474,9 @@ int ftlm_block_apply(ftlm_ctx* ctx, int32_t mx, int32_t my, int32_t nvec, const 
           p[1] = im;
         }
       }
-    FTLM_CUDA(cudaMemcpyAsync(c.vec_a.p, h.data(), bytes, cudaMemcpyHostToDevice, c.stream));
+    FTLM_CUDA(cudaMemcpyAsync(reorder ? c.vec_h.p : c.vec_a.p, h.data(), bytes, cudaMemcpyHostToDevice, c.stream));
     c.prof.h2d_bytes += static_cast<int64_t>(bytes);
-    ftlm::HvSourceGuard guard{c};
-    c.prof.hv_source = ftlm::hv_select_source(c, NV, fp32);
+    if (reorder) ftlm::sweep_reorder(c, false, c.vec_h.p, c.vec_a.p, NV, fp32);
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     if (c.timing) {
       FTLM_CUDA(cudaEventCreate(&e0));
@@ -491,7 +493,8 @@ int ftlm_block_apply(ftlm_ctx* ctx, int32_t mx, int32_t my, int32_t nvec, const 
     if (c.timing) {
       FTLM_CUDA(cudaEventRecord(e1, c.stream));
     }
-    FTLM_CUDA(cudaMemcpyAsync(h.data(), c.vec_h.p, bytes, cudaMemcpyDeviceToHost, c.stream));
+    if (reorder) ftlm::sweep_reorder(c, true, c.vec_h.p, c.vec_a.p, NV, fp32);
+    FTLM_CUDA(cudaMemcpyAsync(h.data(), reorder ? c.vec_a.p : c.vec_h.p, bytes, cudaMemcpyDeviceToHost, c.stream));
     FTLM_CUDA(cudaStreamSynchronize(c.stream));
     c.prof.d2h_bytes += static_cast<int64_t>(bytes);
     if (c.timing) {

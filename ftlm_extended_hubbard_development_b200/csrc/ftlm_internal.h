@@ -255,20 +255,22 @@ struct Ctx {
   bool split_active = false;  // H*V runs as the two segment sweeps of split.cu
   std::unique_ptr<Ctx> flipped;  // tables of sector (N_down, N_up) when N_up != N_down
   DBuf flip_map;      // uint64 per row: flipped row | shift << 32 | sign << 38 (+ an error word)
-  int flip_for[4] = {-1, -1, -1, -1};  // (n_up, n_dn, mx, my) the flip map belongs to
+  int flip_for[5] = {-1, -1, -1, -1, -1};  // (n_up, n_dn, mx, my, stn_pos_seg) the flip map belongs to
   int64_t flip_gen = -1, sec_gen = 0;  // sector generation of the flip map / of the tables
   DBuf vec_xd, vec_yd;  // Lanczos vector and H*V output in the spin-flipped row order
   bool seg_dynamic = true;  // segment sweeps take rows from a shared counter (FTLM_SEG_ROWS=stride: grid-stride)
   DBuf seg_counter;         // the row counters of the two sweeps
   bool split_stencil = true;  // segment sweeps read the class stencils (FTLM_SPLIT_OP=fly: on-the-fly lookups)
-  bool stn_rows = true;       // narrow stencil sweeps run 8 lanes per row (FTLM_STN_ROWS=0: warp per row)
+  bool split_wide = false;    // the prepared sweeps are the stencil ones, their vectors in stn_pos order
   // class stencils of this context's prepared block (split.cu)
   bool stn_ok = false;
   int64_t stn_for[3] = {-1, -1, -1};  // (sector generation, mx, my) they belong to
-  DBuf stn_crb, stn_rp, stn_rp32, stn_ent, stn_cnt;
+  DBuf stn_crb, stn_rp, stn_ent, stn_cnt;
   DBuf stn_rp4, stn_row, stn_ent4, stn_deg, stn_coef;  // entries of the wide sweeps in runs of one coefficient
   DBuf stn_seg, stn_cls;           // segments by class, class list
-  DBuf stn_diag;                   // diagonal per row, in the sweeps' type
+  DBuf stn_pos;                    // position of every row in the sweeps' order,
+  int stn_pos_seg = 0;             // segments per group of that order (0: not built)
+  DBuf stn_diag;                   // diagonal per position, in the sweeps' type
   std::vector<int64_t> stn_classes;  // per class with rows: number of segments, rows per segment
   bool hv_rows = true;  // narrow sweeps on the hop list: 8 lanes per row (FTLM_HV_ROWS=0: warp per row)
   bool small_blocks = true;  // batched FTLM runs blocks <= kSmallMaxDim in one launch (FTLM_SMALL_BLOCKS=0: off)
@@ -376,15 +378,24 @@ void hv_tuned_store(Ctx& c, uint64_t key, int var);
 // the two flipped-order arrays for sweeps of nv vectors; false when they do
 // not fit in device memory.
 bool split_prepare(Ctx& c, int nv, bool fp32);
+// The prepared sweeps' row order for another number of vectors.
+void split_order(Ctx& c, int nv, bool fp32);
 // y = M x for x given in both row orders: out (this block's order, diagonal
 // included) and out_d (flipped order) such that M x = out + S^T out_d.
 // partial receives 2 x grid rows of fixed-point Re<s x, y> sums; returns
 // that row count.
 int hv_apply_split(Ctx& c, const void* in, const void* in_d, void* out, void* out_d, int nv, bool fp32,
                    const double* scale, fx128* partial);
-// Whether those sweeps leave y unscaled (the wide stencil kernel): the
-// Lanczos update then applies the scale.
-bool hv_split_unscaled(const Ctx& c, int nv, bool fp32);
+// Row order of the stencil sweeps' vectors (split.cu): position of every row of
+// the block, null where the active operator keeps the block order. Those sweeps
+// take any number of vectors (FP32: an even one), leave y unscaled (the Lanczos
+// update then applies the scale) and read up to kSweepPad bytes past the end of
+// their input vectors.
+const uint32_t* sweep_pos(const Ctx& c);
+constexpr size_t kSweepPad = 2048;
+inline int sweep_width(int nvec, bool fp32) { return fp32 ? (nvec + 1) / 2 * 2 : nvec; }
+// Vectors from block order to the sweeps' order, or back.
+void sweep_reorder(Ctx& c, bool to_block, const void* src, void* dst, int nv, bool fp32);
 int hv_split_max_grid(const Ctx& c);
 // x_D[p(q)] = conj(f_q) x[q];  y[q] += f_q y_D[p(q)].
 void flip_scatter(Ctx& c, const void* x, void* xd, int nv, bool fp32);

@@ -803,17 +803,22 @@ int hv_select_source(Ctx& c, int nv, bool fp32) {
   c.split_active = false;
   const int64_t D = c.blk.dim;
   int mode = c.hv_mode;
+  bool one_chunk = false;
   if (mode < 0) {
-    // measured on a 4x4 (8,8) block (FP32): split-spin sweeps fastest from 4
-    // vectors up (4.6 vs 7.8 ms per H*V at 4, 35 vs 56 at 128; 243 vs 282 ms at
-    // 16 on 6x3 (9,9)), the hop list's row kernel at one chunk per row
-    const bool one_chunk = nv == (fp32 ? 2 : 1);
-    if (D >= kSplitMinDim && !one_chunk) mode = kSrcSplit;
+    // The split-spin sweeps from 2^15 rows, at every width: on the stencils they
+    // take 2 FP32 vectors of 4x4 (6,6) in 0.28 ms per H*V, the hop list's row
+    // kernel in 1.56 (and the list takes 5.8 ms to build); without the stencils
+    // (more than 65536 down words) one-chunk rows stay on the hop list.
+    one_chunk = nv == (fp32 ? 2 : 1);
+    if (D >= kSplitMinDim) mode = kSrcSplit;
     else if (D >= (1 << 14) && nv <= (fp32 ? 32 : 16)) mode = kSrcList;
     else mode = kSrcFly;
   }
   if (mode == kSrcList && !hoplist_build(c)) mode = c.hv_mode < 0 && D >= kSplitMinDim ? kSrcSplit : kSrcFly;
-  if (mode == kSrcSplit && !split_prepare(c, nv, fp32)) mode = kSrcFly;
+  if (mode == kSrcSplit) {
+    if (!split_prepare(c, nv, fp32)) mode = kSrcFly;
+    else if (one_chunk && !c.split_wide && hoplist_build(c)) mode = kSrcList;
+  }
   c.hl_active = mode == kSrcList;
   c.split_active = mode == kSrcSplit;
   return mode;

@@ -61,17 +61,20 @@ __global__ void k_state_init(double* st, int NV, int nva) {
 
 // The per-CTA partials [ncta][NV] are summed by one CTA of kFinThreads
 // threads per 32 vectors: thread t takes vector t % VB of the rows t / VB,
-// t / VB + slots, ..., then the slots are added by halves. One thread per
+// t / VB + slots, ..., then the slots are added by halves (VB: a power of two). One thread per
 // vector walking all ncta (up to 1184) rows was a chain of dependent L2
 // loads: 80-150 us per launch against 5-8 us.
 constexpr int kFinThreads = 512;
 
+__device__ __forceinline__ int fin_width(int NV) { return NV >= 32 ? 32 : NV > 1 ? 2 << (31 - __clz(NV - 1)) : 1; }
+
 template <typename S>
 __device__ __forceinline__ S fin_sum(int NV, int ncta, const S* __restrict__ partial, S* sh) {
-  const int VB = min(NV, 32), slots = kFinThreads / VB;
+  const int VB = fin_width(NV), slots = kFinThreads / VB;
   const int v = blockIdx.x * VB + threadIdx.x % VB;
   S t = 0;
-  for (int b = threadIdx.x / VB; b < ncta; b += slots) t += partial[static_cast<int64_t>(b) * NV + v];
+  if (v < NV)
+    for (int b = threadIdx.x / VB; b < ncta; b += slots) t += partial[static_cast<int64_t>(b) * NV + v];
   sh[threadIdx.x] = t;
   for (int o = kFinThreads / 2; o >= VB; o >>= 1) {
     __syncthreads();
@@ -86,8 +89,8 @@ __global__ void __launch_bounds__(kFinThreads) k_alpha_fin(int NV, int ncta, con
                                                            double* __restrict__ st, double* __restrict__ alpha_j) {
   __shared__ fx128 sh[kFinThreads];
   const fx128 t = fin_sum(NV, ncta, partial, sh);
-  const int v = blockIdx.x * min(NV, 32) + threadIdx.x;
-  if (static_cast<int>(threadIdx.x) >= min(NV, 32)) return;
+  const int v = blockIdx.x * fin_width(NV) + threadIdx.x;
+  if (static_cast<int>(threadIdx.x) >= fin_width(NV) || v >= NV) return;
   const double s = fx_to_double(t);
   alpha_j[v] = s;
   st[S_CA * NV + v] = s * st[S_CUR * NV + v];
@@ -99,8 +102,8 @@ __global__ void __launch_bounds__(kFinThreads) k_beta_fin(int NV, int ncta, cons
                                                           int kdim) {
   __shared__ double sh[kFinThreads];
   const double s = fin_sum(NV, ncta, partial, sh);
-  const int v = blockIdx.x * min(NV, 32) + threadIdx.x;
-  if (static_cast<int>(threadIdx.x) >= min(NV, 32)) return;
+  const int v = blockIdx.x * fin_width(NV) + threadIdx.x;
+  if (static_cast<int>(threadIdx.x) >= fin_width(NV) || v >= NV) return;
   if (st[S_DONE * NV + v] != 0.0) {
     st[S_CUR * NV + v] = 0.0;
     st[S_PREV * NV + v] = 0.0;
@@ -141,7 +144,8 @@ __global__ void __launch_bounds__(kUpdThreads) k_update(int64_t nchunks, int NV,
   const int CPR = NV / VPL;
   __shared__ double red[kUpdThreads * 2];
   const int tid = threadIdx.x;
-  const int cv = tid % CPR;  // stride is a multiple of CPR, so fixed per thread
+  const int nt = static_cast<int>(blockDim.x);  // a multiple of CPR (update_threads), so cv is fixed per thread
+  const int cv = tid % CPR;
   double ca[VPL], cb[VPL], cy[VPL], acc[VPL];
 #pragma unroll
   for (int e = 0; e < VPL; ++e) {
@@ -150,8 +154,8 @@ __global__ void __launch_bounds__(kUpdThreads) k_update(int64_t nchunks, int NV,
     cb[e] = st[S_CB * NV + cv * VPL + e];
     acc[e] = 0.0;
   }
-  const int64_t stride = static_cast<int64_t>(gridDim.x) * kUpdThreads;
-  for (int64_t i = static_cast<int64_t>(blockIdx.x) * kUpdThreads + tid; i < nchunks; i += stride) {
+  const int64_t stride = static_cast<int64_t>(gridDim.x) * nt;
+  for (int64_t i = static_cast<int64_t>(blockIdx.x) * nt + tid; i < nchunks; i += stride) {
     const V h = y[i], x = wc[i], p = wp[i];
     int64_t fi_idx = 0;
     double fr = 1.0, fim = 0.0;
@@ -195,18 +199,23 @@ __global__ void __launch_bounds__(kUpdThreads) k_update(int64_t nchunks, int NV,
 #pragma unroll
   for (int e = 0; e < VPL; ++e) red[tid * VPL + e] = acc[e];
   __syncthreads();
-  for (int v = tid; v < NV; v += kUpdThreads) {
+  for (int v = tid; v < NV; v += nt) {
     const int c = v / VPL, e = v % VPL;
     double s = 0.0;
-    for (int t = c; t < kUpdThreads; t += CPR) s += red[t * VPL + e];
+    for (int t = c; t < nt; t += CPR) s += red[t * VPL + e];
     partial[static_cast<int64_t>(blockIdx.x) * NV + v] = s;
   }
 }
 
+// Threads per CTA of k_update: rows of CPR <= 128 chunks, whole rows per CTA.
+int update_threads(int CPR) { return kUpdThreads / CPR * CPR; }
+
 // Start vectors, production mode: uniform phase, |q_i|^2 = 1/dim.
-// Philox4x32-10 keyed by the block seed, counter (row, sample).
+// Philox4x32-10 keyed by the block seed, counter (row, sample). Written to
+// position pos[row] (null: row).
 template <typename T>
-__global__ void k_start_philox(int64_t dim, int NV, int nva, int sample0, uint64_t seed, typename VT<T>::V* __restrict__ out) {
+__global__ void k_start_philox(int64_t dim, int NV, int nva, int sample0, uint64_t seed,
+                               const uint32_t* __restrict__ pos, typename VT<T>::V* __restrict__ out) {
   using V = typename VT<T>::V;
   constexpr int VPL = VT<T>::VPL;
   const int CPR = NV / VPL;
@@ -231,14 +240,14 @@ __global__ void k_start_philox(int64_t dim, int NV, int nva, int sample0, uint64
     } else {
       o = make_double2(re[0], im[0]);
     }
-    out[i] = o;
+    out[pos ? static_cast<int64_t>(pos[row]) * CPR + c : i] = o;
   }
 }
 
-// Start vectors given per sample ([nva][dim] complex FP64) into [dim][NV].
+// Start vectors given per sample ([nva][dim] complex FP64) into [dim][NV], as k_start_philox.
 template <typename T>
 __global__ void k_start_gather(int64_t dim, int NV, int nva, const double2* __restrict__ src,
-                               typename VT<T>::V* __restrict__ out) {
+                               const uint32_t* __restrict__ pos, typename VT<T>::V* __restrict__ out) {
   using V = typename VT<T>::V;
   constexpr int VPL = VT<T>::VPL;
   const int CPR = NV / VPL;
@@ -260,7 +269,7 @@ __global__ void k_start_gather(int64_t dim, int NV, int nva, const double2* __re
     } else {
       o = z[0];
     }
-    out[i] = o;
+    out[pos ? static_cast<int64_t>(pos[row]) * CPR + c : i] = o;
   }
 }
 
@@ -585,18 +594,21 @@ void run_ftlm_block(Ctx& c, int n_up, int n_dn, int mx, int my, Spectrum& out, c
   // then streams 8 B per hop (few vectors share each lookup); large blocks
   // run the split-spin segment sweeps; the rest the on-the-fly kernel.
   HvSourceGuard guard{c};
-  const int src = hv_select_source(c, next_pow2(std::max(std::min(nvmax, R), fp32 ? 2 : 1)), fp32);
+  const int src = hv_select_source(c, sweep_width(std::min(nvmax, R), fp32), fp32);
   c.prof.hv_source = src;
   const bool split = src == kSrcSplit;
   const double nzh = c.timing ? static_cast<double>(src == kSrcList ? c.hl_nnz : block_nonzero_hops(c)) : 0.0;
   const FlipPhase fph = flip_phase(c);
   const uint64_t* fmap = split ? c.flip_map.as<uint64_t>() : nullptr;
+  const uint32_t* pos = sweep_pos(c);
   for (int s0 = 0; s0 < R; s0 += nvmax) {
     const int nva = std::min(nvmax, R - s0);
-    const int NV = next_pow2(std::max(nva, fp32 ? 2 : 1));
+    // the stencil sweeps take any width; the other operators powers of two
+    const int NV = pos ? sweep_width(nva, fp32) : next_pow2(std::max(nva, fp32 ? 2 : 1));
+    if (pos) split_order(c, NV, fp32);
     const size_t bytes = static_cast<size_t>(D) * NV * esize;
-    c.vec_a.ensure(bytes);
-    c.vec_b.ensure(bytes);
+    c.vec_a.ensure(bytes + kSweepPad);
+    c.vec_b.ensure(bytes + kSweepPad);
     c.vec_h.ensure(bytes);
     const int CPR = fp32 ? NV / 2 : NV;
     const int64_t nchunks = D * CPR;
@@ -616,21 +628,22 @@ void run_ftlm_block(Ctx& c, int n_up, int n_dn, int mx, int my, Spectrum& out, c
                                 cudaMemcpyHostToDevice, c.stream));
       c.prof.h2d_bytes += sizeof(double) * 2 * static_cast<int64_t>(nva) * D;
       if (fp32)
-        k_start_gather<float><<<sgrid, 256, 0, c.stream>>>(D, NV, nva, c.host_start.as<double2>(), c.vec_a.as<float4>());
+        k_start_gather<float><<<sgrid, 256, 0, c.stream>>>(D, NV, nva, c.host_start.as<double2>(), pos, c.vec_a.as<float4>());
       else
-        k_start_gather<double><<<sgrid, 256, 0, c.stream>>>(D, NV, nva, c.host_start.as<double2>(), c.vec_a.as<double2>());
+        k_start_gather<double><<<sgrid, 256, 0, c.stream>>>(D, NV, nva, c.host_start.as<double2>(), pos, c.vec_a.as<double2>());
     } else {
       if (fp32)
-        k_start_philox<float><<<sgrid, 256, 0, c.stream>>>(D, NV, nva, s0, bseed, c.vec_a.as<float4>());
+        k_start_philox<float><<<sgrid, 256, 0, c.stream>>>(D, NV, nva, s0, bseed, pos, c.vec_a.as<float4>());
       else
-        k_start_philox<double><<<sgrid, 256, 0, c.stream>>>(D, NV, nva, s0, bseed, c.vec_a.as<double2>());
+        k_start_philox<double><<<sgrid, 256, 0, c.stream>>>(D, NV, nva, s0, bseed, pos, c.vec_a.as<double2>());
     }
     FTLM_LAUNCH_CHECK();
     FTLM_CUDA(cudaMemsetAsync(c.vec_b.p, 0, bytes, c.stream));
     if (split) flip_scatter(c, c.vec_a.p, c.vec_xd.p, NV, fp32);
     const int hgrid = split ? hv_split_max_grid(c) : hv_grid(c, NV, fp32);
-    const int ugrid = std::max(1, std::min<int>(static_cast<int>((nchunks + kUpdThreads - 1) / kUpdThreads),
-                                                c.sm_count * 8));
+    const int uthr = update_threads(CPR);
+    const int ugrid = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>((nchunks + uthr - 1) / uthr,
+                                                                              int64_t(c.sm_count) * 8)));
     c.partial.ensure(std::max(sizeof(fx128) * hgrid, sizeof(double) * ugrid) * NV);
     c.lz_state.ensure(sizeof(double) * S_NFIELD * NV);
     double* st = c.lz_state.as<double>();
@@ -639,7 +652,7 @@ void run_ftlm_block(Ctx& c, int n_up, int n_dn, int mx, int my, Spectrum& out, c
     k_state_init<<<1, 128, 0, c.stream>>>(st, NV, nva);
     void* cur = c.vec_a.p;
     void* prev = c.vec_b.p;
-    const int unscaled = split && hv_split_unscaled(c, NV, fp32) ? 1 : 0;
+    const int unscaled = pos ? 1 : 0;
     for (int j = 0; j < K; ++j) {
       cudaEvent_t e0 = nullptr, e1 = nullptr;
       if (c.timing) {
@@ -661,21 +674,21 @@ void run_ftlm_block(Ctx& c, int n_up, int n_dn, int mx, int my, Spectrum& out, c
       if (fp32) {
         using V = float4;
         if (split)
-          k_update<float, true><<<ugrid, kUpdThreads, 0, c.stream>>>(
+          k_update<float, true><<<ugrid, uthr, 0, c.stream>>>(
               nchunks, NV, c.vec_h.as<V>(), static_cast<const V*>(cur), static_cast<V*>(prev), st,
               c.partial.as<double>(), c.vec_yd.as<V>(), c.vec_xd.as<V>(), fmap, fph, unscaled);
         else
-          k_update<float, false><<<ugrid, kUpdThreads, 0, c.stream>>>(
+          k_update<float, false><<<ugrid, uthr, 0, c.stream>>>(
               nchunks, NV, c.vec_h.as<V>(), static_cast<const V*>(cur), static_cast<V*>(prev), st,
               c.partial.as<double>(), nullptr, nullptr, nullptr, fph, 0);
       } else {
         using V = double2;
         if (split)
-          k_update<double, true><<<ugrid, kUpdThreads, 0, c.stream>>>(
+          k_update<double, true><<<ugrid, uthr, 0, c.stream>>>(
               nchunks, NV, c.vec_h.as<V>(), static_cast<const V*>(cur), static_cast<V*>(prev), st,
               c.partial.as<double>(), c.vec_yd.as<V>(), c.vec_xd.as<V>(), fmap, fph, unscaled);
         else
-          k_update<double, false><<<ugrid, kUpdThreads, 0, c.stream>>>(
+          k_update<double, false><<<ugrid, uthr, 0, c.stream>>>(
               nchunks, NV, c.vec_h.as<V>(), static_cast<const V*>(cur), static_cast<V*>(prev), st,
               c.partial.as<double>(), nullptr, nullptr, nullptr, fph, 0);
       }

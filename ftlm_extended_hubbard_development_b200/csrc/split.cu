@@ -29,6 +29,7 @@
 // shared.
 #include <algorithm>
 #include <cstring>
+#include <type_traits>
 
 #include "ftlm_internal.h"
 #include "hv_common.cuh"
@@ -323,21 +324,33 @@ struct CoefT<double> {
   using C = double2;
 };
 
-// One class of segments (equal stabiliser, hence equal stencil): its segments
-// are seg_ur[seg0 .. seg0 + nseg), `rows` rows each, stencil rows crb .. .
+// Row order of the stencil sweeps. All segments of a class share their stencil,
+// so the segments are taken in groups of S, S segments' vectors filling 64
+// chunks of 16 bytes (1 KB), and a group's rows are stored with the segment as
+// the fast index: position = base + g S rows + a S_g + s for row a of segment s
+// of group g (S_g = S but for the last group of a class). A hop then reads one
+// contiguous run of up to 1 KB for all segments of the group, whatever the
+// number of vectors, which need not be a power of two, and a group's rows stay
+// within a few MB, as one segment's do at 1 KB a row (interleaving a whole
+// class spread the gathers of a stencil row over all of the array: 5-7% slower
+// at 64 and 128 vectors). The vectors, the diagonal and the flip map of these
+// sweeps are kept in this order.
+//
+// One class of segments (equal stabiliser, hence equal stencil): `rows` rows
+// each, stencil rows crb ..., positions base ... .
 struct StnClass {
-  int32_t seg0, nseg, rows, c0;  // c0: trivial stabiliser
-  int64_t crb;
+  int32_t nseg, rows, c0, first;  // c0: trivial stabiliser; first: its segments in stn_seg
+  int64_t crb, base;
 };
+constexpr int kStnRun = 64;  // chunks of a full group's row
+inline int stn_group(int cpr) { return std::max(1, kStnRun / cpr); }
 
 // One sweep: y = diag * x + M_dn x over all segments of one row order.
 template <typename T>
 struct StnJob {
   const typename CT<T>::V* in;
   typename CT<T>::V* out;
-  const T* diag;  // per row, null: none
-  const int64_t* aoff;
-  const int32_t* seg_ur;
+  const T* diag;  // per position, null: none
   const int2* srow;  // per stencil row: first entry / 4, entries
   const uint4* ent;
   const typename CoefT<T>::C* coef;
@@ -345,23 +358,43 @@ struct StnJob {
   int32_t ncls;
   int32_t units;  // work units (below) of the job
 };
+// A group's stencil row, S_g cpr chunks, is cut into `parts` panels of at most
+// pw <= 32 LPL chunks, one per warp. A lane's chunks belong to the same vectors
+// in every panel of the same part.
+struct StnPanels {
+  int32_t cpr, seg, parts, pw;  // seg: S
+  __host__ __device__ __forceinline__ int64_t count(int64_t nseg) const { return (nseg + seg - 1) / seg * parts; }
+};
+inline StnPanels stn_panels(int cpr, int lanes) {
+  const int seg = stn_group(cpr), run = seg * cpr, parts = (run + lanes - 1) / lanes;
+  return {cpr, seg, parts, (run + parts - 1) / parts};
+}
 template <typename T>
 struct StnJobs {
   StnJob<T> j[2];
-  int32_t njobs;
+  int32_t njobs, nv, rows;  // rows per unit
+  StnPanels pan;
   typename CoefT<T>::C c0[kStnCoefs];  // class 0: +-amplitude of each direction
 };
 
+// Row `a` of a group whose rows are rowb bytes: one 32 x 32 + 64 bit multiply-add.
+template <typename V>
+__device__ __forceinline__ V* stn_at(V* p, uint32_t a, uint32_t rowb) {
+  using B = std::conditional_t<std::is_const_v<V>, const char, char>;
+  return reinterpret_cast<V*>(reinterpret_cast<B*>(p) + static_cast<uint64_t>(a) * rowb);
+}
+
 // N hops of a row (entries e): all gathers issued before the first FMA.
-template <typename T, int CPR, int G, int LPL, int N, bool C0>
+template <typename T, int LPL, int N, bool C0>
 __device__ __forceinline__ void stn_hops(const uint32_t* e, const StnJobs<T>& P, const typename CoefT<T>::C* coef,
-                                         const typename CT<T>::V* __restrict__ xs, typename CT<T>::V (&acc)[LPL]) {
+                                         const typename CT<T>::V* __restrict__ xs, uint32_t rowb,
+                                         typename CT<T>::V (&acc)[LPL]) {
   using V = typename CT<T>::V;
   V x[N][LPL];
 #pragma unroll
   for (int u = 0; u < N; ++u)
 #pragma unroll
-    for (int l = 0; l < LPL; ++l) x[u][l] = __ldg(xs + static_cast<uint64_t>(e[u] & 0xFFFFu) * CPR + l * G);
+    for (int l = 0; l < LPL; ++l) x[u][l] = __ldg(stn_at(xs, e[u] & 0xFFFFu, rowb) + l * 32);
   typename CoefT<T>::C c[N];
 #pragma unroll
   for (int u = 0; u < N; ++u) {
@@ -375,10 +408,10 @@ __device__ __forceinline__ void stn_hops(const uint32_t* e, const StnJobs<T>& P,
 }
 
 // All hops of a row, U (4 or 8) at a time, then the remainder.
-template <typename T, int CPR, int G, int LPL, int U, bool C0>
+template <typename T, int LPL, int U, bool C0>
 __device__ __forceinline__ void stn_row(const uint4* q, int left, const StnJobs<T>& P,
                                         const typename CoefT<T>::C* coef, const typename CT<T>::V* __restrict__ xs,
-                                        typename CT<T>::V (&acc)[LPL]) {
+                                        uint32_t rowb, typename CT<T>::V (&acc)[LPL]) {
   uint4 p = __ldg(q);
   if constexpr (U == 8) {
     while (left >= 8) {
@@ -386,20 +419,20 @@ __device__ __forceinline__ void stn_row(const uint4* q, int left, const StnJobs<
       const uint32_t e[8] = {p.x, p.y, p.z, p.w, p2.x, p2.y, p2.z, p2.w};
       q += 2;
       p = __ldg(q);
-      stn_hops<T, CPR, G, LPL, 8, C0>(e, P, coef, xs, acc);
+      stn_hops<T, LPL, 8, C0>(e, P, coef, xs, rowb, acc);
       left -= 8;
     }
   }
   while (left >= 4) {
     const uint32_t e[4] = {p.x, p.y, p.z, p.w};
     p = __ldg(++q);
-    stn_hops<T, CPR, G, LPL, 4, C0>(e, P, coef, xs, acc);
+    stn_hops<T, LPL, 4, C0>(e, P, coef, xs, rowb, acc);
     left -= 4;
   }
   const uint32_t e[3] = {p.x, p.y, p.z};
-  if (left == 1) stn_hops<T, CPR, G, LPL, 1, C0>(e, P, coef, xs, acc);
-  else if (left == 2) stn_hops<T, CPR, G, LPL, 2, C0>(e, P, coef, xs, acc);
-  else if (left == 3) stn_hops<T, CPR, G, LPL, 3, C0>(e, P, coef, xs, acc);
+  if (left == 1) stn_hops<T, LPL, 1, C0>(e, P, coef, xs, rowb, acc);
+  else if (left == 2) stn_hops<T, LPL, 2, C0>(e, P, coef, xs, rowb, acc);
+  else if (left == 3) stn_hops<T, LPL, 3, C0>(e, P, coef, xs, rowb, acc);
 }
 
 __device__ __forceinline__ void stn_finish(float4& y, const float4& x, float d, double* dot) {
@@ -418,57 +451,56 @@ __device__ __forceinline__ void stn_finish(double2& y, const double2& x, double 
 
 // The segment sweeps on the class stencils, one launch for both row orders.
 //
-// All segments of a class have the same stencil, so a warp takes one stencil
-// row for 32/G segments at once (G lanes of LPL 16-byte chunks per segment):
-// the row's entries are warp-uniform (one broadcast load per four hops, no
-// shuffles, no divergence, no partial sums to fold) whatever the sweep's
-// width. A work unit is kStnRows stencil rows, kStnLane apart, of one group of
-// segments; kStnLane consecutive units cover kStnLane * kStnRows consecutive
-// rows. A CTA takes one unit per warp, consecutive ones, from a shared counter,
-// so at any moment its warps are on neighbouring rows, which share gather
-// targets (hops among the low sites stay within a few hundred rows): a quarter
-// of the gathered sectors hit L1.
+// A warp takes a panel of a stencil row (32 lanes of LPL 16-byte chunks, 512 LPL
+// contiguous bytes per hop): the row's entries are warp-uniform (one broadcast
+// load per four hops, no shuffles, no divergence, no partial sums to fold). A
+// work unit is kStnRows stencil rows, kStnLane apart, of one panel;
+// kStnLane consecutive units cover kStnLane * kStnRows consecutive rows. A CTA
+// takes one unit per warp, consecutive ones, from a shared counter, so at any
+// moment its warps are on neighbouring rows, which share gather targets (hops
+// among the low sites stay within a few hundred rows): a quarter of the
+// gathered sectors hit L1. Lanes past the end of a panel load what follows it
+// (the arrays end in kSweepPad spare bytes) and drop the result.
 //
-// Bound: the L1 data pipe (68% busy) and L2 reads (12.5 TB/s) together; a hop
-// costs 4 LPL + 1 cycles of the pipe for 512 LPL bytes. Per H*V, both sweeps,
-// against one warp per row with shuffled entries and one launch per sweep:
-// 4x4 (8,8) k=0 128 FP32 vectors 34.8 -> 22.3 ms, 64 vectors 20.5 -> 11.1,
-// 6x3 (5,5) 16 vectors 5.27 -> 1.78, 4x4 (4,4) 8 FP64 vectors 0.283 -> 0.119,
-// 4x4 (5,6) 128 FP64 vectors 11.7 -> 7.4 (17-20 TB/s of gathered bytes).
+// Bound: waits for gathered lines at 16-24 warps per SM (L1 67% busy with 30%
+// hits, L2 50%; 17-20 TB/s of gathered bytes). Per H*V, both sweeps, against the
+// same kernel on one short row per segment (the row order of the block):
+// 6x3 (5,5) 16 FP32 vectors 1.90 -> 1.64 ms, 4x4 (4,4) 5 FP64 vectors (then
+// padded to 8) 0.111 -> 0.086, 4x4 (6,6) 2 FP32 vectors 0.28 against 1.56 of the
+// hop list; 4x4 (8,8) 64 vectors 11.6 -> 11.3, 4x4 (5,5) 128 vectors unchanged.
 //
 // y is NOT scaled (the Lanczos update applies the scale of the unnormalised
-// vectors). The dot terms Re<x, y> of a unit are summed in FP64 in row order,
-// scaled by scale^2 and added as 128-bit integers: neither the grid, the CTA
-// shape nor the assignment of units changes the sum.
-constexpr int kStnRows = 8;
+// vectors). The dot terms Re<x, y> of a unit are summed in FP64 in row order
+// per segment and vector, scaled by scale^2 and added as 128-bit integers:
+// neither the grid, the panels nor the assignment of units changes the sum.
 constexpr int kStnLane = 8;
-// Units of one group of segments of `rows` rows.
-__host__ __device__ __forceinline__ unsigned int stn_chunks(int64_t rows) {
-  const int64_t full = rows / (kStnLane * kStnRows), rest = rows % (kStnLane * kStnRows);
+// Units of one group of segments of `rows` rows, `per` rows a unit.
+__host__ __device__ __forceinline__ unsigned int stn_chunks(int64_t rows, int per) {
+  const int64_t full = rows / (kStnLane * per), rest = rows % (kStnLane * per);
   return static_cast<unsigned int>(full * kStnLane + (rest < kStnLane ? rest : kStnLane));
 }
 
-template <typename T, int NV, int LPL, int U, int NT, int MINB>
+constexpr int kStnSlots = 128;  // dot terms of a warp: parts x 32 LPL chunks x vectors per chunk, at most
+
+template <typename T, int LPL, int U, int NT, int MINB>
 __global__ void __launch_bounds__(NT, MINB) k_hv_stn(const __grid_constant__ StnJobs<T> P,
                                                      const double* __restrict__ scale, fx128* __restrict__ partial,
                                                      unsigned int* __restrict__ next_item) {
   using V = typename CT<T>::V;
   constexpr int VPL = CT<T>::VPL;
-  constexpr int CPR = NV / VPL;
-  constexpr int G = CPR / LPL;   // lanes per segment
-  constexpr int RPW = 32 / G;    // segments per warp
   constexpr int NW = NT / 32;
-  __shared__ double s_dot[2][NW][RPW * NV];
+  __shared__ fx128 s_acc[NW][kStnSlots];
   __shared__ unsigned int s_item[2];
   const int tid = threadIdx.x;
   const int lane = tid & 31;
   const int wid = tid >> 5;
-  const int grp = lane / G;
-  const int sub = lane % G;
+  const int cpr = P.pan.cpr, parts = P.pan.parts, pw = P.pan.pw;
   const unsigned int total = static_cast<unsigned int>(P.j[0].units) + (P.njobs > 1 ? P.j[1].units : 0);
   const unsigned int nitems = (total + NW - 1) / NW;
-  fx128 facc = 0;  // column tid of the dot product
-  const double sc = scale && tid < NV ? scale[tid] : 1.0;
+  if (partial) {
+    for (int i = tid; i < NW * kStnSlots; i += NT) s_acc[i / kStnSlots][i % kStnSlots] = 0;
+    __syncthreads();
+  }
   int jb = 0, cl = 0;
   unsigned int cbase = 0;  // first unit of class cl of job jb
   unsigned int item = blockIdx.x;
@@ -481,11 +513,6 @@ __global__ void __launch_bounds__(NT, MINB) k_hv_stn(const __grid_constant__ Stn
     unsigned int nxt = item + gridDim.x;
     if (next_item && tid == 0) nxt = atomicAdd(next_item, 1u);
     const unsigned int unit = item * NW + wid;
-    double dot[LPL][VPL];
-#pragma unroll
-    for (int l = 0; l < LPL; ++l)
-#pragma unroll
-      for (int e = 0; e < VPL; ++e) dot[l][e] = 0.0;
     if (unit < total) {
       // units grow monotonically, so job and class only move forward
       unsigned int ju = unit;
@@ -499,24 +526,37 @@ __global__ void __launch_bounds__(NT, MINB) k_hv_stn(const __grid_constant__ Stn
       }
       const StnJob<T>& J = P.j[jb];
       StnClass C = J.cls[cl];
-      unsigned int nch = stn_chunks(C.rows);
-      unsigned int cu = nch * ((C.nseg + RPW - 1) / RPW);
+      unsigned int nch = stn_chunks(C.rows, P.rows);
+      unsigned int cu = nch * static_cast<unsigned int>(P.pan.count(C.nseg));
       while (ju >= cbase + cu) {
         cbase += cu;
         C = J.cls[++cl];
-        nch = stn_chunks(C.rows);
-        cu = nch * ((C.nseg + RPW - 1) / RPW);
+        nch = stn_chunks(C.rows, P.rows);
+        cu = nch * static_cast<unsigned int>(P.pan.count(C.nseg));
       }
       const unsigned int q = (ju - cbase) / nch;
       const int ch = static_cast<int>(ju - cbase - q * nch);
-      const int a0 = (ch / kStnLane) * (kStnLane * kStnRows) + ch % kStnLane;
-      const int si = static_cast<int>(q) * RPW + grp;
-      const bool ok = si < C.nseg;
-      const int64_t row0 = __ldg(J.aoff + __ldg(J.seg_ur + C.seg0 + (ok ? si : C.nseg - 1)));
-      const V* xs = J.in + row0 * CPR + sub;
-      V* ys = J.out + row0 * CPR + sub;
-      const int nr = min(kStnRows, (C.rows - a0 + kStnLane - 1) / kStnLane);
-      const int2 hp = __ldg(J.srow + C.crb + a0 + kStnLane * min(lane, nr - 1));
+      const int a0 = (ch / kStnLane) * (kStnLane * P.rows) + ch % kStnLane;
+      const int g = static_cast<int>(q) / parts, part = static_cast<int>(q) - g * parts;
+      const int nsg = min(P.pan.seg, C.nseg - g * P.pan.seg);  // segments of the group
+      const uint32_t rowb = static_cast<uint32_t>(nsg * cpr) * sizeof(V);  // bytes of its rows
+      const int c0 = part * pw;
+      const int here = min(pw, nsg * cpr - c0);  // none in the last parts of a short group
+      const int64_t gbase = C.base + static_cast<int64_t>(g) * P.pan.seg * C.rows;
+      const int64_t off = gbase * cpr + c0 + lane;
+      const V* xs = J.in + off;
+      V* ys = J.out + off;
+      const T* dg[LPL];
+#pragma unroll
+      for (int l = 0; l < LPL; ++l)
+        dg[l] = J.diag ? J.diag + gbase + min(c0 + l * 32 + lane, nsg * cpr - 1) / cpr : nullptr;
+      double dot[LPL][VPL];
+#pragma unroll
+      for (int l = 0; l < LPL; ++l)
+#pragma unroll
+        for (int e = 0; e < VPL; ++e) dot[l][e] = 0.0;
+      const int nr = here > 0 ? min(P.rows, (C.rows - a0 + kStnLane - 1) / kStnLane) : 0;
+      const int2 hp = __ldg(J.srow + C.crb + a0 + kStnLane * min(lane, max(nr, 1) - 1));
       for (int r = 0; r < nr; ++r) {
         const int a = a0 + r * kStnLane;
         const uint4* q4 = J.ent + __shfl_sync(0xffffffffu, hp.x, r);
@@ -524,187 +564,63 @@ __global__ void __launch_bounds__(NT, MINB) k_hv_stn(const __grid_constant__ Stn
         V acc[LPL];
 #pragma unroll
         for (int l = 0; l < LPL; ++l) vzero(acc[l]);
-        const T d = J.diag ? __ldg(J.diag + row0 + a) : T(0);
+        T d[LPL];
+#pragma unroll
+        for (int l = 0; l < LPL; ++l) d[l] = J.diag ? __ldg(dg[l] + a * nsg) : T(0);
         V xo[LPL];
 #pragma unroll
-        for (int l = 0; l < LPL; ++l) xo[l] = __ldg(xs + static_cast<int64_t>(a) * CPR + l * G);
-        if (C.c0) stn_row<T, CPR, G, LPL, U, true>(q4, left, P, J.coef, xs, acc);
-        else stn_row<T, CPR, G, LPL, U, false>(q4, left, P, J.coef, xs, acc);
+        for (int l = 0; l < LPL; ++l) xo[l] = __ldg(stn_at(xs, a, rowb) + l * 32);
+        if (C.c0) stn_row<T, LPL, U, true>(q4, left, P, J.coef, xs, rowb, acc);
+        else stn_row<T, LPL, U, false>(q4, left, P, J.coef, xs, rowb, acc);
 #pragma unroll
         for (int l = 0; l < LPL; ++l) {
-          stn_finish(acc[l], xo[l], d, dot[l]);
-          if (ok) st_stream(ys + static_cast<int64_t>(a) * CPR + l * G, acc[l]);
+          stn_finish(acc[l], xo[l], d[l], dot[l]);
+          if (l * 32 + lane < here) st_stream(stn_at(ys, a, rowb) + l * 32, acc[l]);
         }
       }
-      if (!ok)
+      if (partial) {
 #pragma unroll
         for (int l = 0; l < LPL; ++l)
+          if (l * 32 + lane < here) {
+            const int v = (c0 + l * 32 + lane) % cpr * VPL;
 #pragma unroll
-          for (int e = 0; e < VPL; ++e) dot[l][e] = 0.0;
-    }
-    if (partial) {
-#pragma unroll
-      for (int l = 0; l < LPL; ++l)
-#pragma unroll
-        for (int e = 0; e < VPL; ++e) s_dot[it & 1][wid][grp * NV + (l * G + sub) * VPL + e] = dot[l][e];
+            for (int e = 0; e < VPL; ++e) {
+              const double sc = scale ? __ldg(scale + v + e) : 1.0;
+              s_acc[wid][((part * LPL + l) * VPL + e) * 32 + lane] += fx_of(sc * (sc * dot[l][e]));
+            }
+          }
+      }
     }
     if (tid == 0) s_item[it & 1] = nxt;
     __syncthreads();
     item = s_item[it & 1];
-    if (partial && tid < NV) {
-#pragma unroll
-      for (int w = 0; w < NW; ++w)
-#pragma unroll
-        for (int g = 0; g < RPW; ++g) facc += fx_of(sc * (sc * s_dot[it & 1][w][g * NV + tid]));
-    }
   }
-  if (partial && tid < NV) partial[static_cast<int64_t>(blockIdx.x) * NV + tid] = facc;
-}
-
-// Narrow sweeps (rows of at most 4 chunks: <= 8 FP32 / 4 FP64 vectors) on the
-// class stencils: one warp per row leaves the row's dependent loads (meta ->
-// class, offset -> stencil row -> entries -> gathers) exposed, so 8 lanes
-// share a row and a warp works on 4 rows, each lane taking every 8th hop of
-// its row with kStnChunks 16-byte gathers in flight (kStnChunks / CPR hops);
-// shuffles fold the row. Same contract as k_hv_stn; rows are taken 4 at a
-// time from the shared counter.
-constexpr int kStnLanes = 8;
-constexpr int kStnChunks = 4;
-
-template <typename W, typename T, int NV>
-__global__ void __launch_bounds__(kHvThreads, 4) k_hv_stn_rows(const __grid_constant__ HvParams<W> P,
-                                                               const int64_t* __restrict__ crb,
-                                                               const int32_t* __restrict__ srp,
-                                                               const uint32_t* __restrict__ sent,
-                                                               const typename CT<T>::V* __restrict__ in,
-                                                               typename CT<T>::V* __restrict__ out,
-                                                               const double* __restrict__ scale,
-                                                               fx128* __restrict__ partial, int with_diag,
-                                                               unsigned long long* __restrict__ next_row) {
-  using V = typename CT<T>::V;
-  constexpr int VPL = CT<T>::VPL;
-  constexpr int CPR = NV / VPL;
-  static_assert(CPR >= 1 && CPR <= 4, "narrow sweeps only");
-  constexpr int kStnU = kStnChunks / CPR;  // hops in flight per lane
-  constexpr int kRows = 32 / kStnLanes;  // rows per warp
-  __shared__ double s_ph[2][64];
-  __shared__ double s_amp[2][8];
-  __shared__ double s_sq[65];
-  __shared__ fx128 s_acc[kHvWarps * kRows][NV];
-  const Geom& g = P.g;
-  const BlockView<W>& v = P.v;
-  const int tid = threadIdx.x;
-  for (int i = tid; i < 64; i += kHvThreads) {
-    s_ph[0][i] = v.phase_re[i];
-    s_ph[1][i] = v.phase_im[i];
-  }
-  if (tid < 8) {
-    s_amp[0][tid] = g.amp_re[tid];
-    s_amp[1][tid] = g.amp_im[tid];
-  }
-  if (tid < 65) s_sq[tid] = g.sqrt_deg[tid];
-  for (int i = tid; i < kHvWarps * kRows * NV; i += kHvThreads) s_acc[i / NV][i % NV] = 0;
+  if (!partial) return;
   __syncthreads();
-  const int lane = tid & 31;
-  const int wid = tid >> 5;
-  const int grp = lane / kStnLanes;
-  const int sub = lane % kStnLanes;
-  double sc[CPR][VPL];
-#pragma unroll
-  for (int l = 0; l < CPR; ++l)
-#pragma unroll
-    for (int e = 0; e < VPL; ++e) sc[l][e] = scale ? scale[l * VPL + e] : 1.0;
-  const int64_t nwarps = static_cast<int64_t>(gridDim.x) * kHvWarps;
-  int64_t rb = (static_cast<int64_t>(blockIdx.x) * kHvWarps + wid) * kRows;
-  unsigned long long pend = 0;  // lane 0: the next grab, in flight while this one is processed
-  if (next_row && lane == 0) pend = atomicAdd(next_row, static_cast<unsigned long long>(kRows));
-  while (true) {
-    if (next_row) {
-      rb = static_cast<int64_t>(__shfl_sync(0xffffffffu, pend, 0));
-      if (lane == 0 && rb < v.dim) pend = atomicAdd(next_row, static_cast<unsigned long long>(kRows));
-    }
-    if (rb >= v.dim) break;  // warp-uniform
-    const int64_t row = rb + grp;
-    const bool ok = row < v.dim;
-    uint32_t meta = 0;
-    int64_t seg = 0;
-    int h0 = 0, h1 = 0;
-    if (ok) {
-      meta = __ldg(v.row_meta + row);
-      const uint32_t ur = meta & 0x3FFFFFFu;
-      seg = __ldg(v.aoff + ur);
-      const int64_t cr = __ldg(crb + __ldg(v.ur_class + ur)) + (row - seg);
-      h0 = __ldg(srp + cr);
-      h1 = __ldg(srp + cr + 1);
-    }
-    const double inv_s = 1.0 / s_sq[static_cast<int>(meta >> 26) + 1];
-    V acc[CPR];
-#pragma unroll
-    for (int l = 0; l < CPR; ++l) vzero(acc[l]);
-    for (int q0 = h0 + sub; q0 < h1; q0 += kStnLanes * kStnU) {
-      uint32_t e[kStnU];
-#pragma unroll
-      for (int u = 0; u < kStnU; ++u) {
-        const int q = q0 + u * kStnLanes;
-        e[u] = q < h1 ? __ldg(sent + q) : 0xFFFFFFFFu;
-      }
-      V x[kStnU][CPR];
-      T cr_[kStnU], ci[kStnU];
-#pragma unroll
-      for (int u = 0; u < kStnU; ++u) {
-        cr_[u] = 0;
-        ci[u] = 0;
-#pragma unroll
-        for (int l = 0; l < CPR; ++l) vzero(x[u][l]);
-        if (e[u] != 0xFFFFFFFFu) {
-          const int64_t col = seg + static_cast<int64_t>(e[u] & 0xFFFFu);
-          const int dir = static_cast<int>((e[u] >> 16) & 7);
-          const int p = static_cast<int>((e[u] >> 19) & 1);
-          const int shift = static_cast<int>((e[u] >> 20) & 63);
-          const int deg_t = static_cast<int>((e[u] >> 26) & 63) + 1;
-          const double ar = p ? -s_amp[0][dir] : s_amp[0][dir];
-          const double ai = p ? -s_amp[1][dir] : s_amp[1][dir];
-          const double pr = s_ph[0][shift], pi = s_ph[1][shift];
-          const double ratio = s_sq[deg_t] * inv_s;
-          cr_[u] = static_cast<T>((ar * pr - ai * pi) * ratio);
-          ci[u] = static_cast<T>((ar * pi + ai * pr) * ratio);
-#pragma unroll
-          for (int l = 0; l < CPR; ++l) x[u][l] = ld_stream(in + col * CPR + l);
-        }
-      }
-#pragma unroll
-      for (int u = 0; u < kStnU; ++u)
-#pragma unroll
-        for (int l = 0; l < CPR; ++l) cfma<T>(acc[l], cr_[u], ci[u], x[u][l]);
-    }
-#pragma unroll
-    for (int o = kStnLanes / 2; o > 0; o >>= 1)
-#pragma unroll
-      for (int l = 0; l < CPR; ++l) vadd(acc[l], shfl_xor_v(acc[l], o));
-    if (sub == 0 && ok) {
-      const uint32_t ur = meta & 0x3FFFFFFu;
-      const double diag = with_diag ? diag_energy(__ldg(v.ur_bits + ur), __ldg(v.row_dn + row), g) : 0.0;
-#pragma unroll
-      for (int l = 0; l < CPR; ++l) {
-        const V xr = ld_stream(in + row * CPR + l);
-        double dt2[VPL];
-        st_stream(out + row * CPR + l, finish_row(xr, acc[l], diag, sc[l], dt2));
-        if (partial) {
-#pragma unroll
-          for (int e2 = 0; e2 < VPL; ++e2) s_acc[wid * kRows + grp][l * VPL + e2] += fx_of(dt2[e2]);
-        }
-      }
-    }
-    if (!next_row) rb += nwarps * kRows;
+  for (int i = tid; i < kStnSlots; i += NT) {
+    fx128 t = s_acc[0][i];
+    for (int w = 1; w < NW; ++w) t += s_acc[w][i];
+    s_acc[0][i] = t;
   }
-  flush_dot<NV>(s_acc, partial);
+  __syncthreads();
+  for (int v = tid; v < P.nv; v += NT) {
+    const int e = v % VPL;
+    fx128 t = 0;
+    for (int c = v / VPL; c < P.pan.seg * cpr; c += cpr) {
+      const int part = c / pw, k = c - part * pw;
+      t += s_acc[0][((part * LPL + k / 32) * VPL + e) * 32 + k % 32];
+    }
+    partial[static_cast<int64_t>(blockIdx.x) * P.nv + v] = t;
+  }
 }
 
 // Flip map of every row q of block Pu: the flipped state (d, u) resolved in
-// the tables vd of sector (N_down, N_up): row p | shift << 32 | sign << 38.
+// the tables vd of sector (N_down, N_up): row p | shift << 32 | sign << 38,
+// both sides in the sweeps' row order (pos, pos_d; null: block order).
 template <typename W>
 __global__ void k_flip_map(const __grid_constant__ HvParams<W> Pu, const __grid_constant__ BlockView<W> vd,
-                           const uint64_t* __restrict__ binom, uint64_t* __restrict__ fmap, int* __restrict__ bad) {
+                           const uint64_t* __restrict__ binom, const uint32_t* __restrict__ pos,
+                           const uint32_t* __restrict__ pos_d, uint64_t* __restrict__ fmap, int* __restrict__ bad) {
   const BlockView<W>& v = Pu.v;
   for (int64_t q = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; q < v.dim;
        q += static_cast<int64_t>(gridDim.x) * blockDim.x) {
@@ -715,10 +631,11 @@ __global__ void k_flip_map(const __grid_constant__ HvParams<W> Pu, const __grid_
     int shift, sgn, deg;
     if (!resolve<W, uint64_t>(d, u, true, 0, vd, Pu.g, binom, col, shift, sgn, deg) || col < 0 || col >= vd.dim) {
       atomicAdd(bad, 1);
-      fmap[q] = 0;
+      fmap[pos ? pos[q] : q] = 0;
       continue;
     }
-    fmap[q] = static_cast<uint64_t>(col) | (static_cast<uint64_t>(shift) << 32) | (static_cast<uint64_t>(sgn) << 38);
+    if (pos_d) col = pos_d[col];
+    fmap[pos ? pos[q] : q] = static_cast<uint64_t>(col) | (static_cast<uint64_t>(shift) << 32) | (static_cast<uint64_t>(sgn) << 38);
   }
 }
 
@@ -762,19 +679,6 @@ void launch_seg_t(Ctx& c, Ctx& t, const void* in, void* out, const double* scale
   if constexpr (sizeof(W) == 4) P.v = view32(t);
   else P.v = view64(t);
   using V = typename CT<T>::V;
-  if (c.split_stencil && t.stn_ok) {
-    if constexpr (NV / CT<T>::VPL <= 4) {
-      if (c.stn_rows) {  // narrow rows: 8 lanes per row (no variants: the same kernel for every U, MINB)
-        k_hv_stn_rows<W, T, NV><<<static_cast<int>(std::min<int64_t>(
-                                      (t.blk.dim + 4 * kHvWarps - 1) / (4 * kHvWarps), int64_t(c.sm_count) * 4)),
-                                  kHvThreads, 0, c.stream>>>(
-            P, t.stn_crb.as<int64_t>(), t.stn_rp32.as<int32_t>(), t.stn_ent.as<uint32_t>(), static_cast<const V*>(in),
-            static_cast<V*>(out), scale, partial, with_diag ? 1 : 0, next_row);
-        return;
-      }
-    }
-    throw Error(FTLM_ERR_INTERNAL, "wide stencil sweeps are launched by launch_stn");
-  }
   const R* gb = sizeof(R) == 4 ? reinterpret_cast<const R*>(c.binom32.p) : reinterpret_cast<const R*>(c.binom.p);
   k_hv_seg<W, R, T, NV, U, MINB><<<grid, kHvThreads, 0, c.stream>>>(P, static_cast<const V*>(in), static_cast<V*>(out),
                                                                     scale, partial, gb, with_diag ? 1 : 0, next_row);
@@ -843,14 +747,18 @@ void launch_seg(Ctx& c, Ctx& t, int var, const void* in, void* out, int nv, bool
 }
 
 // ---- wide stencil sweeps
+// Stencil rows of a unit: more rows share more gathers in L1, fewer balance
+// better. 4x4 (8,8), 64 vectors (1.3 M units of 8 rows and 64 chunks): 16 rows
+// 11.3 ms per H*V, 8 rows 11.8, 32 rows 12.6; 6x3 (5,5), 16 vectors (130 k
+// units): 1.65, 1.63, 1.80; 4x4 (4,4), 5 FP64 vectors (4 k): 0.109, 0.087, 0.154.
+int stn_rows(int64_t dim, int cpr) { return dim * cpr >= (int64_t(1) << 27) ? 16 : 8; }
+
 template <typename T>
-StnJob<T> stn_job(Ctx& t, const void* in, void* out, bool with_diag, int rpw) {
+StnJob<T> stn_job(Ctx& t, const void* in, void* out, bool with_diag, const StnPanels& pan, int rows) {
   StnJob<T> j;
   j.in = static_cast<const typename CT<T>::V*>(in);
   j.out = static_cast<typename CT<T>::V*>(out);
   j.diag = with_diag ? t.stn_diag.as<T>() : nullptr;
-  j.aoff = t.blk.aoff.as<int64_t>();
-  j.seg_ur = t.stn_seg.as<int32_t>();
   j.srow = t.stn_row.as<int2>();
   j.ent = t.stn_ent4.as<uint4>();
   j.coef = t.stn_coef.as<typename CoefT<T>::C>();
@@ -858,7 +766,7 @@ StnJob<T> stn_job(Ctx& t, const void* in, void* out, bool with_diag, int rpw) {
   j.ncls = static_cast<int32_t>(t.stn_classes.size() / 2);
   int64_t units = 0;
   for (size_t k = 0; k + 1 < t.stn_classes.size(); k += 2)
-    units += stn_chunks(t.stn_classes[k + 1]) * ((t.stn_classes[k] + rpw - 1) / rpw);
+    units += stn_chunks(t.stn_classes[k + 1], rows) * pan.count(t.stn_classes[k]);
   j.units = static_cast<int32_t>(units);
   return j;
 }
@@ -870,11 +778,13 @@ struct StnSweep {  // the two sweeps of one H*V: block order (with the diagonal)
   int n;
 };
 
-template <typename T, int NV, int LPL, int U, int NT, int MINB>
-int launch_stn_t(Ctx& c, const StnSweep& w, const double* scale, fx128* partial, unsigned int* counter) {
-  constexpr int RPW = 32 / (NV / CT<T>::VPL / LPL);
+template <typename T, int LPL, int U, int NT, int MINB>
+int launch_stn_t(Ctx& c, const StnSweep& w, int nv, const double* scale, fx128* partial, unsigned int* counter) {
   StnJobs<T> P;
   P.njobs = w.n;
+  P.nv = nv;
+  P.pan = stn_panels(nv / CT<T>::VPL, 32 * LPL);
+  P.rows = stn_rows(c.blk.dim, nv / CT<T>::VPL);
   for (int k = 0; k < kStnCoefs; ++k) {  // shift 0 (phase 1), ratio 1
     const double sg = k & 1 ? -1.0 : 1.0;
     P.c0[k].x = static_cast<T>(sg * c.geom.amp_re[k / 2]);
@@ -882,56 +792,34 @@ int launch_stn_t(Ctx& c, const StnSweep& w, const double* scale, fx128* partial,
   }
   int64_t units = 0;
   for (int i = 0; i < w.n; ++i) {
-    P.j[i] = stn_job<T>(*w.t[i], w.in[i], w.out[i], i == 0, RPW);
+    P.j[i] = stn_job<T>(*w.t[i], w.in[i], w.out[i], i == 0, P.pan, P.rows);
     units += P.j[i].units;
   }
   const int64_t items = (units + NT / 32 - 1) / (NT / 32);
   const int grid = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(items, int64_t(c.sm_count) * MINB)));
   // the rest of the SM's 228 KB serves as L1, where most of the gather reuse is
-  constexpr size_t kSmem = 2 * sizeof(double) * NT * LPL * CT<T>::VPL + 2048;
+  constexpr size_t kSmem = sizeof(fx128) * NT / 32 * kStnSlots + 2048;
   constexpr int kCarve = static_cast<int>((kSmem * MINB * 100 + 228 * 1024 - 1) / (228 * 1024));
-  FTLM_CUDA(cudaFuncSetAttribute(k_hv_stn<T, NV, LPL, U, NT, MINB>, cudaFuncAttributePreferredSharedMemoryCarveout,
+  FTLM_CUDA(cudaFuncSetAttribute(k_hv_stn<T, LPL, U, NT, MINB>, cudaFuncAttributePreferredSharedMemoryCarveout,
                                  kCarve));
-  k_hv_stn<T, NV, LPL, U, NT, MINB><<<grid, NT, 0, c.stream>>>(P, scale, partial, counter);
+  k_hv_stn<T, LPL, U, NT, MINB><<<grid, NT, 0, c.stream>>>(P, scale, partial, counter);
   return grid;
 }
 
 // Variants: chunks per lane (more amortise the entry load, fewer leave
 // registers for warps), gathers in flight, CTA shape. All sum a row's hops in
-// the same order. Fastest on B200: 1 or 4 for rows of 256 bytes and more, 2 or
-// 3 below.
-template <typename T, int NV>
-int launch_stn_var(Ctx& c, int var, const StnSweep& w, const double* scale, fx128* partial, unsigned int* nr) {
-  constexpr int CPR = NV / CT<T>::VPL;
-  constexpr int L0 = CPR > 32 ? CPR / 32 : 1;
-  constexpr int L1 = CPR >= 16 && CPR <= 32 ? 2 : L0;
+// the same order, and the same dot terms.
+template <typename T>
+int launch_stn_var(Ctx& c, int var, const StnSweep& w, int nv, const double* scale, fx128* partial, unsigned int* nr) {
   switch (var) {
-    case 0: return launch_stn_t<T, NV, L1, 4, 256, 3>(c, w, scale, partial, nr);
-    case 1: return launch_stn_t<T, NV, L1, 8, 256, 2>(c, w, scale, partial, nr);
-    case 2: return launch_stn_t<T, NV, L0, 8, 256, 3>(c, w, scale, partial, nr);
-    case 3: return launch_stn_t<T, NV, L0, 4, 256, 4>(c, w, scale, partial, nr);
-    case 4: return launch_stn_t<T, NV, L1, 8, 512, 1>(c, w, scale, partial, nr);
+    case 0: return launch_stn_t<T, 2, 4, 256, 3>(c, w, nv, scale, partial, nr);
+    case 1: return launch_stn_t<T, 2, 8, 256, 2>(c, w, nv, scale, partial, nr);
+    case 2: return launch_stn_t<T, 1, 8, 256, 3>(c, w, nv, scale, partial, nr);
+    case 3: return launch_stn_t<T, 1, 4, 256, 4>(c, w, nv, scale, partial, nr);
+    case 4: return launch_stn_t<T, 2, 8, 256, 3>(c, w, nv, scale, partial, nr);
     default: break;
   }
   throw Error(FTLM_ERR_ARG, "bad H*V kernel variant");
-}
-
-template <typename T>
-int launch_stn_nv(Ctx& c, int var, const StnSweep& w, int nv, const double* scale, fx128* partial, unsigned int* nr) {
-  switch (nv) {
-    case 1:
-      if constexpr (sizeof(T) == 8) return launch_stn_var<T, 1>(c, var, w, scale, partial, nr);
-      break;
-    case 2: return launch_stn_var<T, 2>(c, var, w, scale, partial, nr);
-    case 4: return launch_stn_var<T, 4>(c, var, w, scale, partial, nr);
-    case 8: return launch_stn_var<T, 8>(c, var, w, scale, partial, nr);
-    case 16: return launch_stn_var<T, 16>(c, var, w, scale, partial, nr);
-    case 32: return launch_stn_var<T, 32>(c, var, w, scale, partial, nr);
-    case 64: return launch_stn_var<T, 64>(c, var, w, scale, partial, nr);
-    case 128: return launch_stn_var<T, 128>(c, var, w, scale, partial, nr);
-    default: break;
-  }
-  throw Error(FTLM_ERR_ARG, "unsupported vectors per sweep: " + std::to_string(nv));
 }
 
 // Returns the grid, which is the number of rows of dot partials.
@@ -942,15 +830,10 @@ int launch_stn(Ctx& c, int var, const StnSweep& w, int nv, bool fp32, const doub
     nr = c.seg_counter.as<unsigned int>();
     FTLM_CUDA(cudaMemsetAsync(nr, 0, sizeof(unsigned int), c.stream));
   }
-  const int grid = fp32 ? launch_stn_nv<float>(c, var, w, nv, scale, partial, nr)
-                        : launch_stn_nv<double>(c, var, w, nv, scale, partial, nr);
+  const int grid = fp32 ? launch_stn_var<float>(c, var, w, nv, scale, partial, nr)
+                        : launch_stn_var<double>(c, var, w, nv, scale, partial, nr);
   FTLM_LAUNCH_CHECK();
   return grid;
-}
-
-// Whether sweeps of nv vectors over block c run the wide stencil kernel.
-bool stn_wide(const Ctx& c, int nv, bool fp32) {
-  return c.split_stencil && c.stn_ok && !(c.stn_rows && (fp32 ? nv / 2 : nv) <= 4);
 }
 
 int seg_grid(const Ctx& c, int var) {
@@ -985,12 +868,6 @@ Ctx& flipped_tables(Ctx& c) {
   block_prepare(f, c.blk.mx, c.blk.my);
   if (f.blk.dim != c.blk.dim) throw Error(FTLM_ERR_INTERNAL, "spin-flipped block has another dimension");
   return f;
-}
-
-__global__ void k_rp_narrow(const int64_t* __restrict__ in, int32_t* __restrict__ out, int64_t n) {
-  for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < n;
-       i += static_cast<int64_t>(gridDim.x) * blockDim.x)
-    out[i] = static_cast<int32_t>(in[i]);
 }
 
 // ---- entries of the wide sweeps
@@ -1097,6 +974,22 @@ bool stn_wide_build(Ctx& c, Ctx& t, int64_t rows) {
   return true;
 }
 
+// Position of every row of the block in the sweeps' order, S segments a group.
+__global__ void k_stn_pos(const StnClass* __restrict__ cls, int ncls, int S, int64_t dim,
+                          const int32_t* __restrict__ seg_ur, const int64_t* __restrict__ aoff,
+                          uint32_t* __restrict__ pos) {
+  for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < dim;
+       i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+    int c = 0;
+    while (c + 1 < ncls && cls[c + 1].base <= i) ++c;
+    const StnClass C = cls[c];
+    const int64_t at = i - C.base, full = static_cast<int64_t>(S) * C.rows;
+    const int g = static_cast<int>(at / full);
+    const uint32_t in = static_cast<uint32_t>(at - g * full), nsg = min(S, C.nseg - g * S), a = in / nsg;
+    pos[aoff[seg_ur[C.first + g * S + (in - a * nsg)]] + a] = static_cast<uint32_t>(i);
+  }
+}
+
 // Class stencils of the prepared block of tables t (its own sector and
 // block); false when a class has more than kStencilMaxRows rows.
 template <typename W>
@@ -1134,11 +1027,14 @@ bool stencil_build_t(Ctx& c, Ctx& t) {
   std::vector<int64_t> at(first.begin(), first.end() - 1);
   for (int64_t u = 0; u < S.nur; ++u) seg[at[S.h_ur_class[u]]++] = static_cast<int32_t>(u);
   std::vector<StnClass> cls;
+  int64_t base = 0;
   t.stn_classes.clear();
   for (int k = 0; k < S.nclass; ++k) {
     const int64_t nseg = first[k + 1] - first[k], nrow = crb[k + 1] - crb[k];
     if (nseg == 0 || nrow == 0) continue;
-    cls.push_back({static_cast<int32_t>(first[k]), static_cast<int32_t>(nseg), static_cast<int32_t>(nrow), k == 0 ? 1 : 0, crb[k]});
+    cls.push_back({static_cast<int32_t>(nseg), static_cast<int32_t>(nrow), k == 0 ? 1 : 0,
+                   static_cast<int32_t>(first[k]), crb[k], base});
+    base += nseg * nrow;
     t.stn_classes.push_back(nseg);
     t.stn_classes.push_back(nrow);
   }
@@ -1146,23 +1042,21 @@ bool stencil_build_t(Ctx& c, Ctx& t) {
   t.stn_cls.ensure(sizeof(StnClass) * std::max<size_t>(cls.size(), 1));
   FTLM_CUDA(cudaMemcpyAsync(t.stn_seg.p, seg.data(), sizeof(int32_t) * seg.size(), cudaMemcpyHostToDevice, c.stream));
   FTLM_CUDA(cudaMemcpyAsync(t.stn_cls.p, cls.data(), sizeof(StnClass) * cls.size(), cudaMemcpyHostToDevice, c.stream));
-  // row offsets as int32 for the sweeps (fewer registers per row)
-  t.stn_rp32.ensure(sizeof(int32_t) * (rows + 1));
-  k_rp_narrow<<<grid_rows(rows + 1, 256), 256, 0, c.stream>>>(t.stn_rp.as<int64_t>(), t.stn_rp32.as<int32_t>(),
-                                                             rows + 1);
+  if (base != B.dim) throw Error(FTLM_ERR_INTERNAL, "stencil classes do not cover the block");
   FTLM_LAUNCH_CHECK();
   FTLM_CUDA(cudaStreamSynchronize(c.stream));
-  c.prof.kernel_launches += 6;
+  c.prof.kernel_launches += 5;
   return true;
 }
 
-// Diagonal energy of every row of the prepared block, in the sweeps' type.
+// Diagonal energy of every row of the prepared block, in the sweeps' type and order.
 template <typename W, typename T>
-__global__ void k_row_diag(const __grid_constant__ HvParams<W> P, T* __restrict__ diag) {
+__global__ void k_row_diag(const __grid_constant__ HvParams<W> P, const uint32_t* __restrict__ pos,
+                           T* __restrict__ diag) {
   const BlockView<W>& v = P.v;
   for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < v.dim;
        i += static_cast<int64_t>(gridDim.x) * blockDim.x)
-    diag[i] = static_cast<T>(diag_energy(v.ur_bits[v.row_meta[i] & 0x3FFFFFFu], v.row_dn[i], P.g));
+    diag[pos[i]] = static_cast<T>(diag_energy(v.ur_bits[v.row_meta[i] & 0x3FFFFFFu], v.row_dn[i], P.g));
 }
 
 template <typename W>
@@ -1174,10 +1068,10 @@ void row_diag_build(Ctx& c) {
   const int64_t D = c.blk.dim;
   if (c.opts.precision == FTLM_PREC_MIXED) {
     c.stn_diag.ensure(sizeof(float) * D);
-    k_row_diag<W, float><<<grid_rows(D, 256), 256, 0, c.stream>>>(P, c.stn_diag.as<float>());
+    k_row_diag<W, float><<<grid_rows(D, 256), 256, 0, c.stream>>>(P, c.stn_pos.as<uint32_t>(), c.stn_diag.as<float>());
   } else {
     c.stn_diag.ensure(sizeof(double) * D);
-    k_row_diag<W, double><<<grid_rows(D, 256), 256, 0, c.stream>>>(P, c.stn_diag.as<double>());
+    k_row_diag<W, double><<<grid_rows(D, 256), 256, 0, c.stream>>>(P, c.stn_pos.as<uint32_t>(), c.stn_diag.as<double>());
   }
   FTLM_LAUNCH_CHECK();
   c.prof.kernel_launches += 1;
@@ -1188,12 +1082,26 @@ void row_diag_build(Ctx& c) {
 void stencil_prepare(Ctx& c, Ctx& t) {
   const int64_t key[3] = {t.sec_gen, t.blk.mx, t.blk.my};
   if (std::memcmp(key, t.stn_for, sizeof key) == 0) return;
+  t.stn_pos_seg = 0;
   t.stn_ok = c.wide ? stencil_build_t<uint64_t>(c, t) : stencil_build_t<uint32_t>(c, t);
-  if (t.stn_ok && &t == &c) {
+  std::memcpy(t.stn_for, key, sizeof key);
+}
+
+// Positions of the block's rows (and the diagonal in that order) for groups of S segments.
+void order_prepare(Ctx& c, Ctx& t, int S) {
+  if (t.stn_pos_seg == S) return;
+  const int64_t D = t.blk.dim;
+  t.stn_pos.ensure(sizeof(uint32_t) * std::max<int64_t>(D, 1));
+  k_stn_pos<<<grid_rows(D, 256), 256, 0, c.stream>>>(t.stn_cls.as<StnClass>(), static_cast<int>(t.stn_classes.size() / 2),
+                                                     S, D, t.stn_seg.as<int32_t>(), t.blk.aoff.as<int64_t>(),
+                                                     t.stn_pos.as<uint32_t>());
+  FTLM_LAUNCH_CHECK();
+  c.prof.kernel_launches += 1;
+  if (&t == &c) {
     if (c.wide) row_diag_build<uint64_t>(c);
     else row_diag_build<uint32_t>(c);
   }
-  std::memcpy(t.stn_for, key, sizeof key);
+  t.stn_pos_seg = S;
 }
 
 template <typename W>
@@ -1212,7 +1120,10 @@ void flip_map_build_t(Ctx& c, Ctx& f) {
   c.flip_map.ensure(sizeof(uint64_t) * std::max<int64_t>(D, 1) + 64);
   int* bad = reinterpret_cast<int*>(c.flip_map.as<uint64_t>() + D);
   FTLM_CUDA(cudaMemsetAsync(bad, 0, sizeof(int), c.stream));
-  k_flip_map<W><<<grid_rows(D, 128), 128, 0, c.stream>>>(P, vd, c.binom.as<uint64_t>(), c.flip_map.as<uint64_t>(), bad);
+  const uint32_t* pos = c.split_wide ? c.stn_pos.as<uint32_t>() : nullptr;
+  const uint32_t* pos_d = c.split_wide ? f.stn_pos.as<uint32_t>() : nullptr;
+  k_flip_map<W><<<grid_rows(D, 128), 128, 0, c.stream>>>(P, vd, c.binom.as<uint64_t>(), pos, pos_d,
+                                                         c.flip_map.as<uint64_t>(), bad);
   FTLM_LAUNCH_CHECK();
   int hbad = 0;
   FTLM_CUDA(cudaMemcpyAsync(&hbad, bad, sizeof(int), cudaMemcpyDeviceToHost, c.stream));
@@ -1230,41 +1141,57 @@ FlipPhase flip_phase(const Ctx& c) {
   return ph;
 }
 
+void split_order(Ctx& c, int nv, bool fp32) {
+  Ctx& f = c.sec.n_up == c.sec.n_dn ? c : *c.flipped;
+  const int S = c.split_wide ? stn_group(fp32 ? nv / 2 : nv) : 0;
+  if (S) {
+    order_prepare(c, c, S);
+    if (&f != &c) order_prepare(c, f, S);
+  }
+  const int key[5] = {c.sec.n_up, c.sec.n_dn, c.blk.mx, c.blk.my, S};
+  if (std::memcmp(key, c.flip_for, sizeof key) == 0 && c.flip_gen == c.sec_gen) return;
+  if (c.wide) flip_map_build_t<uint64_t>(c, f);
+  else flip_map_build_t<uint32_t>(c, f);
+  std::memcpy(c.flip_for, key, sizeof key);
+  c.flip_gen = c.sec_gen;
+}
+
 bool split_prepare(Ctx& c, int nv, bool fp32) {
   const int64_t D = c.blk.dim;
   if (D <= 0) return false;
   if (D > 0x7fffffffLL) return false;  // the flip map keeps 32-bit rows
-  // memory: two extra vector arrays (flipped x and y) and the 8-byte map
+  // memory: two extra vector arrays (flipped x and y), the 8-byte map, and per
+  // row two positions and the diagonal
   const size_t esize = fp32 ? 8 : 16;
-  const size_t vec = static_cast<size_t>(D) * nv * esize;
-  const size_t need = 2 * vec + sizeof(uint64_t) * D;
-  const size_t have = c.vec_xd.cap + c.vec_yd.cap + c.flip_map.cap;
+  int pow2 = fp32 ? 2 : 1;  // the on-the-fly sweeps' width
+  while (pow2 < nv) pow2 <<= 1;
+  const size_t vec = static_cast<size_t>(D) * pow2 * esize;
+  const size_t need = 2 * vec + (sizeof(uint64_t) + 2 * sizeof(uint32_t) + esize / 2) * D;
+  const size_t have = c.vec_xd.cap + c.vec_yd.cap + c.flip_map.cap + c.stn_pos.cap + c.stn_diag.cap;
   size_t free_b = 0, total_b = 0;
   FTLM_CUDA(cudaMemGetInfo(&free_b, &total_b));
   if (need > have && need + (size_t(2) << 30) > free_b + have) return false;  // keep 2 GiB headroom
-  const int key[4] = {c.sec.n_up, c.sec.n_dn, c.blk.mx, c.blk.my};
   Ctx& f = flipped_tables(c);
-  if (std::memcmp(key, c.flip_for, sizeof key) != 0 || c.flip_gen != c.sec_gen) {
-    if (c.wide) flip_map_build_t<uint64_t>(c, f);
-    else flip_map_build_t<uint32_t>(c, f);
-    std::memcpy(c.flip_for, key, sizeof key);
-    c.flip_gen = c.sec_gen;
-  }
+  c.split_wide = false;
   if (c.split_stencil) {
     stencil_prepare(c, c);
     if (&f != &c) stencil_prepare(c, f);
+    c.split_wide = c.stn_ok && f.stn_ok;
   }
-  c.vec_xd.ensure(vec);
-  c.vec_yd.ensure(vec);
+  split_order(c, nv, fp32);
+  const size_t used = static_cast<size_t>(D) * (c.split_wide ? nv : pow2) * esize;
+  c.vec_xd.ensure(used + kSweepPad);
+  c.vec_yd.ensure(used);
   return true;
 }
 
 int seg_variant(Ctx& c, const void* in, void* out, int nv, bool fp32) {
   if (c.hv_forced >= 0 && c.hv_forced < kSegVariants) return c.hv_forced;
-  if (c.split_stencil && c.stn_ok && c.stn_rows && (fp32 ? nv / 2 : nv) <= 4) return 0;  // k_hv_stn_rows: no variants
-  const uint64_t key = static_cast<uint64_t>((c.wide ? 1 : 0) | 4 | (c.split_stencil && c.stn_ok ? 8 : 0)) |
+  int width = 1;  // the wide sweeps take any number of vectors: one measurement per power of two
+  while (width < nv) width <<= 1;
+  const uint64_t key = static_cast<uint64_t>((c.wide ? 1 : 0) | 4 | (c.split_wide ? 8 : 0)) |
                        (static_cast<uint64_t>(fp32 ? 1 : 0) << 4) |
-                       (static_cast<uint64_t>(nv) << 8) |
+                       (static_cast<uint64_t>(width) << 8) |
                        (static_cast<uint64_t>(hv_size_class(c.blk.dim)) << 20) |
                        (static_cast<uint64_t>(c.device) << 32);
   int best = -1;
@@ -1274,7 +1201,7 @@ int seg_variant(Ctx& c, const void* in, void* out, int nv, bool fp32) {
   FTLM_CUDA(cudaEventCreate(&e0));
   FTLM_CUDA(cudaEventCreate(&e1));
   // best of 3 single-launch timings per variant, variants interleaved
-  const bool wide = stn_wide(c, nv, fp32);
+  const bool wide = c.split_wide;
   const StnSweep one{{&c, nullptr}, {in, nullptr}, {out, nullptr}, 1};
   auto run = [&](int v) {
     if (wide) launch_stn(c, v, one, nv, fp32, nullptr, nullptr);
@@ -1311,7 +1238,7 @@ int hv_apply_split(Ctx& c, const void* in, const void* in_d, void* out, void* ou
   Ctx& f = flipped_tables(c);
   const int var = seg_variant(c, in, out, nv, fp32);
   c.prof.hv_variant = var;
-  if (stn_wide(c, nv, fp32)) {
+  if (c.split_wide) {
     const StnSweep both{{&c, &f}, {in, in_d}, {out, out_d}, 2};
     const int rows = launch_stn(c, var, both, nv, fp32, scale, partial);
     c.prof.kernel_launches += 1;
@@ -1326,7 +1253,28 @@ int hv_apply_split(Ctx& c, const void* in, const void* in_d, void* out, void* ou
   return 2 * grid;
 }
 
-bool hv_split_unscaled(const Ctx& c, int nv, bool fp32) { return stn_wide(c, nv, fp32); }
+// dst[pos[q]] = src[q], or dst[q] = src[pos[q]], for every 16-byte chunk.
+template <typename V>
+__global__ void k_reorder(int64_t dim, int CPR, bool gather, const uint32_t* __restrict__ pos,
+                          const V* __restrict__ src, V* __restrict__ dst) {
+  const int64_t n = dim * CPR;
+  for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < n;
+       i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+    const int64_t row = i / CPR, j = static_cast<int64_t>(pos[row]) * CPR + (i - row * CPR);
+    if (gather) dst[i] = src[j];
+    else dst[j] = src[i];
+  }
+}
+
+void sweep_reorder(Ctx& c, bool to_block, const void* src, void* dst, int nv, bool fp32) {
+  const int CPR = fp32 ? nv / 2 : nv;
+  k_reorder<float4><<<grid_rows(c.blk.dim * CPR, 256), 256, 0, c.stream>>>(
+      c.blk.dim, CPR, to_block, c.stn_pos.as<uint32_t>(), static_cast<const float4*>(src), static_cast<float4*>(dst));
+  FTLM_LAUNCH_CHECK();
+  c.prof.kernel_launches += 1;
+}
+
+const uint32_t* sweep_pos(const Ctx& c) { return c.split_active && c.split_wide ? c.stn_pos.as<uint32_t>() : nullptr; }
 
 int hv_split_max_grid(const Ctx& c) { return 2 * c.sm_count * 4; }
 

@@ -80,3 +80,25 @@ def test_lanczos_coefficients_do_not_depend_on_the_variant(monkeypatch, prec):
             got.append(eng.block_lanczos(1, 2))
     for a, b, s in got[1:]:
         assert np.array_equal(a, got[0][0]) and np.array_equal(b, got[0][1]) and np.array_equal(s, got[0][2])
+
+
+@pytest.mark.parametrize("prec,tol", [(E.PREC_FP64, 1e-11), (E.PREC_MIXED, 2e-4)], ids=["fp64", "mixed"])
+def test_vectors_per_sweep_do_not_change_the_coefficients(monkeypatch, prec, tol):
+    """The row order of the sweeps depends on their width, and the last sweep
+    of a block is narrower than the others: 21 vectors in one sweep, in 16 + 5,
+    in 7 + 7 + 7 and singly give the same alpha and beta up to the rounding of
+    the update (u times the amplification of 6 steps, below 1e5 u here)."""
+    monkeypatch.setenv("FTLM_HV_MODE", "split")
+    monkeypatch.setenv("FTLM_HV_VARIANT", "1")
+    got = {}
+    for batch in (21, 16, 7, 1):
+        opts = pkg.RunOpts(samples=21, lanczos_steps=6, exact_block_threshold=0, precision=prec,
+                           batch_vectors=batch, start_vector=E.START_PHILOX_PHASE)
+        with pkg.Engine(model(4, 4), opts) as eng:
+            eng.sector_prepare(3, 2)
+            got[batch] = eng.block_lanczos(1, 2)
+    a, b, s = got[21]
+    for batch in (16, 7, 1):
+        assert np.array_equal(got[batch][2], s)
+        assert np.abs(got[batch][0] - a).max() <= tol * np.abs(a).max(), batch
+        assert np.abs(got[batch][1] - b).max() <= tol * np.abs(b).max(), batch
