@@ -209,7 +209,7 @@ void ftlm_ctx_destroy(ftlm_ctx* ctx) {
                         &c.pack.act, &c.pack.act_list, &c.pack.dtab, &c.pack.aoff, &c.pack.nact, &c.pack.dims,
                         &c.pack.row_meta, &c.pack.row_dn, &c.pack.phase, &c.pack.items,
                         &c.scan_tmp, &c.dense_arena, &c.dense_meta, &c.dense_out, &c.dense_vecs, &c.spectra, &c.th_beta,
-                        &c.th_mu, &c.th_state, &c.hl_ptr, &c.hl_ent, &c.flip_map, &c.vec_xd, &c.vec_yd, &c.seg_counter, &c.stn_crb, &c.stn_rp, &c.stn_ent, &c.stn_cnt,
+                        &c.th_mu, &c.th_state, &c.hl_ptr, &c.hl_ent, &c.flip_map, &c.vec_xd, &c.vec_yd, &c.seg_counter, &c.gauss_jobs, &c.stn_crb, &c.stn_rp, &c.stn_ent, &c.stn_cnt,
                         &c.stn_rp4, &c.stn_row, &c.stn_ent4, &c.stn_deg, &c.stn_coef, &c.stn_seg, &c.stn_cls, &c.stn_pos, &c.stn_diag,
                         &c.defer_arena, &c.defer_ev, &c.defer_work};
   for (auto* b : bufs) b->release();

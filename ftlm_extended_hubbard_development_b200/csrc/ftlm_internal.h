@@ -260,6 +260,7 @@ struct Ctx {
   DBuf vec_xd, vec_yd;  // Lanczos vector and H*V output in the spin-flipped row order
   bool seg_dynamic = true;  // segment sweeps take rows from a shared counter (FTLM_SEG_ROWS=stride: grid-stride)
   DBuf seg_counter;         // the row counters of the two sweeps
+  DBuf gauss_jobs;          // Gaussian start vectors to draw
   bool split_stencil = true;  // segment sweeps read the class stencils (FTLM_SPLIT_OP=fly: on-the-fly lookups)
   bool split_wide = false;    // the prepared sweeps are the stencil ones, their vectors in stn_pos order
   // class stencils of this context's prepared block (split.cu)
@@ -453,7 +454,15 @@ void thermo_read(Ctx& c, double* emin, double* z, double* n, double* n2);
 
 // Seeds and reference start vectors (main.cpp:514-533, 1015-1025)
 uint64_t block_seed(uint64_t seed, int n_up, int n_dn, int mx, int my);
-void reference_start_vectors(uint64_t bseed, int sample0, int nva, int64_t dim, double* out);
+// Reference Gaussian start vectors on c.stream (start.cu): the vector of `seed`
+// to out[off .. off + dim), unit norm.
+struct GaussJob {
+  uint64_t seed;
+  int64_t dim, off;
+};
+void gaussian_starts(Ctx& c, const std::vector<GaussJob>& jobs, double2* out);
+// Seed of sample `sample` of the block with seed bseed (main.cpp:1015).
+uint64_t sample_seed(uint64_t bseed, int sample);
 // Nonzero-amplitude hops with active targets in the prepared block (the
 // h_nz * dim of the H*V byte model).
 int64_t block_nonzero_hops(Ctx& c);

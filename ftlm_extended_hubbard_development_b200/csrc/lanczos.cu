@@ -17,9 +17,6 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
-#include <atomic>
-#include <random>
-#include <thread>
 
 #include "ftlm_internal.h"
 #include "hv_common.cuh"
@@ -406,38 +403,7 @@ uint64_t block_seed(uint64_t seed, int n_up, int n_dn, int mx, int my) {  // mai
   return mix_u64(s);
 }
 
-// Reference start vectors (main.cpp:1015-1025): libstdc++ mt19937_64 and
-// normal_distribution; g++ evaluates Complex(normal(rng), normal(rng))
-// right to left, so each element is (second draw, first draw).
-void reference_start_vectors(uint64_t bseed, int sample0, int nva, int64_t dim, double* out) {
-  auto work = [&](int v) {
-    std::mt19937_64 rng(mix_u64(bseed ^ static_cast<uint64_t>(sample0 + v)));
-    std::normal_distribution<double> normal(0.0, 1.0);
-    double* q = out + 2 * static_cast<int64_t>(v) * dim;
-    double n2 = 0.0;
-    for (int64_t i = 0; i < dim; ++i) {
-      const double first = normal(rng);
-      const double second = normal(rng);
-      q[2 * i] = second;
-      q[2 * i + 1] = first;
-      n2 += second * second + first * first;
-    }
-    const double nrm = std::sqrt(n2);
-    for (int64_t i = 0; i < 2 * dim; ++i) q[i] /= nrm;
-  };
-  const unsigned hw = std::max(1u, std::thread::hardware_concurrency());
-  if (nva == 1 || dim < 4096 || hw == 1) {
-    for (int v = 0; v < nva; ++v) work(v);
-    return;
-  }
-  std::vector<std::thread> th;
-  std::atomic<int> next{0};
-  for (unsigned t = 0; t < std::min<unsigned>(hw, static_cast<unsigned>(nva)); ++t)
-    th.emplace_back([&] {
-      for (int v = next++; v < nva; v = next++) work(v);
-    });
-  for (auto& t : th) t.join();
-}
+uint64_t sample_seed(uint64_t bseed, int sample) { return mix_u64(bseed ^ static_cast<uint64_t>(sample)); }
 
 int64_t spectra_alloc(Ctx& c, int64_t count) {
   const int64_t need = c.spectra_used + count;
@@ -587,7 +553,6 @@ void run_ftlm_block(Ctx& c, int n_up, int n_dn, int mx, int my, Spectrum& out, c
   FTLM_CUDA(cudaMemsetAsync(c.lz_beta.p, 0, sizeof(double) * static_cast<size_t>(nsweep) * K * ld, c.stream));
   c.ritz_tmp.ensure(sizeof(int32_t) * (R + 8));
   int32_t* steps_all = c.ritz_tmp.as<int32_t>();
-  std::vector<double> hstart;
   std::vector<std::pair<cudaEvent_t, cudaEvent_t>> evs;
   double hv_bytes = 0.0, hv_hops = 0.0, hv_min_bytes = 0.0;
   // Operator source: the cached hop list pays one lookup pass per block and
@@ -615,18 +580,16 @@ void run_ftlm_block(Ctx& c, int n_up, int n_dn, int mx, int my, Spectrum& out, c
     const int sgrid = static_cast<int>(std::min<int64_t>((nchunks + 255) / 256, static_cast<int64_t>(c.sm_count) * 16));
     // start vectors into vec_a
     if (host_start || c.opts.start_vector == FTLM_START_REF_GAUSSIAN) {
-      const double* src = nullptr;
-      if (host_start) {
-        src = host_start + 2 * static_cast<int64_t>(s0) * D;
-      } else {
-        hstart.resize(2 * static_cast<size_t>(nva) * D);
-        reference_start_vectors(bseed, s0, nva, D, hstart.data());
-        src = hstart.data();
-      }
       c.host_start.ensure(sizeof(double) * 2 * static_cast<size_t>(nva) * D);
-      FTLM_CUDA(cudaMemcpyAsync(c.host_start.p, src, sizeof(double) * 2 * static_cast<size_t>(nva) * D,
-                                cudaMemcpyHostToDevice, c.stream));
-      c.prof.h2d_bytes += sizeof(double) * 2 * static_cast<int64_t>(nva) * D;
+      if (host_start) {
+        FTLM_CUDA(cudaMemcpyAsync(c.host_start.p, host_start + 2 * static_cast<int64_t>(s0) * D,
+                                  sizeof(double) * 2 * static_cast<size_t>(nva) * D, cudaMemcpyHostToDevice, c.stream));
+        c.prof.h2d_bytes += sizeof(double) * 2 * static_cast<int64_t>(nva) * D;
+      } else {
+        std::vector<GaussJob> jobs;
+        for (int v = 0; v < nva; ++v) jobs.push_back({sample_seed(bseed, s0 + v), D, static_cast<int64_t>(v) * D});
+        gaussian_starts(c, jobs, c.host_start.as<double2>());
+      }
       if (fp32)
         k_start_gather<float><<<sgrid, 256, 0, c.stream>>>(D, NV, nva, c.host_start.as<double2>(), pos, c.vec_a.as<float4>());
       else

@@ -409,16 +409,13 @@ void run_small_ftlm_blocks(Ctx& c, const std::vector<std::pair<int, int>>& block
   FTLM_CUDA(cudaMemsetAsync(c.sb_alpha.as<double>() + c.sb_ab_used, 0, sizeof(double) * ab, c.stream));
   FTLM_CUDA(cudaMemsetAsync(c.sb_beta.as<double>() + c.sb_ab_used, 0, sizeof(double) * ab, c.stream));
   pack_entries(c, rows, c.sb_ent.as<uint32_t>(), c.sb_cnt.as<int32_t>(), c.sb_diag.as<double>());
-  // start vectors: reference Gaussian ones from the host, Philox on the device
-  if (ref_start) {
-    std::vector<double> h(2 * static_cast<size_t>(start));
+  if (ref_start) {  // Philox start vectors are drawn by the Lanczos launch
+    std::vector<GaussJob> jobs;
     for (const Item& it : items)
-      reference_start_vectors(it.d.seed, 0, R, it.d.dim, h.data() + 2 * (it.d.start_off - c.sb_start_used));
+      for (int r = 0; r < R; ++r)
+        jobs.push_back({sample_seed(it.d.seed, r), it.d.dim, it.d.start_off + static_cast<int64_t>(r) * it.d.dim});
     pool_room(c, c.sb_start, sizeof(double2) * (c.sb_start_used + start));
-    FTLM_CUDA(cudaMemcpyAsync(c.sb_start.as<double2>() + c.sb_start_used, h.data(), sizeof(double) * h.size(),
-                              cudaMemcpyHostToDevice, c.stream));
-    FTLM_CUDA(cudaStreamSynchronize(c.stream));
-    c.prof.h2d_bytes += static_cast<int64_t>(sizeof(double) * h.size());
+    gaussian_starts(c, jobs, c.sb_start.as<double2>());
   }
   c.sb_ent_used += ent;
   c.sb_row_used += row;
