@@ -270,47 +270,39 @@ __global__ void k_start_gather(int64_t dim, int NV, int nva, const double2* __re
   }
 }
 
-// Strided view of one vector's work array (shared memory: stride 32, one
-// column per thread; global memory: stride 1, one row per thread).
-struct Col {
-  double* p;
-  int st;
-  __device__ __forceinline__ double& operator[](int i) const { return p[i * st]; }
-};
-
-// Implicit QL with shifts on every Lanczos tridiagonal (one thread per
-// random vector; k_tridiag_many serves all vectors of several blocks in one
-// launch, 32 vectors per CTA), tracking
-// the first row z of the eigenvector matrix; then an ascending sort.
+// Implicit QL with shifts on every Lanczos tridiagonal, tracking the first row z
+// of the eigenvector matrix; then an ascending sort. A warp per vector: the
+// recurrence runs on one lane, the others help to load and store. With a vector
+// per lane every lane waited for the longest QL iteration of its 32 (sweeps of
+// one warp diverge at every deflation): 5 vectors x 80 steps took 3.2 ms and 72
+// blocks of 32 x 120 took 10.7; now 1.0 and 4.2 (with ql_norm, ql.cuh). Bound: the
+// dependent chain of a rotation.
 // alpha/beta are [sweep][K][ld] (vector r = sweep r/nvmax, lane r%nvmax),
 // steps[r] the alphas taken. Outputs eigenvalues and z^2 * inv_r into [R][K]
-// rows. With smem != 0 the three work columns of the warp's 32 vectors live
-// in shared memory ([3][K][32]), otherwise in global memory.
-__device__ void tridiag_vector(int r, int t, int nvmax, int ld, int K, const double* __restrict__ alpha,
+// rows. The three work columns live in shared memory (sm, 3 K doubles) or, where
+// that does not hold them, in the output rows and escr.
+constexpr int kRitzWarps = 4;  // vectors per CTA
+
+__device__ void tridiag_vector(int r, int lane, int nvmax, int ld, int K, const double* __restrict__ alpha,
                                const double* __restrict__ beta, const int32_t* __restrict__ steps,
                                double* __restrict__ dout, double* __restrict__ zout, double* __restrict__ escr,
-                               double inv_r, int* __restrict__ status, double* sm, int smem) {
+                               double inv_r, int* __restrict__ status, double* sm) {
   const int n = steps[r];
   const int64_t base = (static_cast<int64_t>(r / nvmax) * K) * ld + r % nvmax;
-  Col d, z, e;
-  if (smem) {
-    d = {sm + t, 32};
-    z = {sm + 32 * K + t, 32};
-    e = {sm + 64 * K + t, 32};
-  } else {
-    d = {dout + static_cast<int64_t>(r) * K, 1};
-    z = {zout + static_cast<int64_t>(r) * K, 1};
-    e = {escr + static_cast<int64_t>(r) * K, 1};
-  }
-  for (int i = 0; i < n; ++i) {
+  double* dr = dout + static_cast<int64_t>(r) * K;
+  double* zr = zout + static_cast<int64_t>(r) * K;
+  double* d = sm ? sm : dr;
+  double* z = sm ? sm + K : zr;
+  double* e = sm ? sm + 2 * K : escr + static_cast<int64_t>(r) * K;
+  for (int i = lane; i < n; i += 32) {
     d[i] = alpha[base + static_cast<int64_t>(i) * ld];
     e[i] = i + 1 < n ? beta[base + static_cast<int64_t>(i) * ld] : 0.0;
     z[i] = i == 0 ? 1.0 : 0.0;
   }
-  if (!ql_first_row(n, d, z, e)) atomicExch(status, 1);
-  double* dr = dout + static_cast<int64_t>(r) * K;
-  double* zr = zout + static_cast<int64_t>(r) * K;
-  for (int i = 0; i < n; ++i) {
+  __syncwarp();
+  if (!ql_first_row<true>(n, d, z, e) && lane == 0) atomicExch(status, 1);
+  __syncwarp();
+  for (int i = lane; i < n; i += 32) {
     const double zi = z[i];
     dr[i] = d[i];
     zr[i] = zi * zi * inv_r;
@@ -318,7 +310,7 @@ __device__ void tridiag_vector(int r, int t, int nvmax, int ld, int K, const dou
 }
 
 // Several blocks' Ritz stages in one launch: CTA b belongs to the job j with
-// cta0[j] <= b < cta0[j+1] and serves that job's vectors 32(b-cta0[j]) ...
+// cta0[j] <= b < cta0[j+1] and serves that job's vectors kRitzWarps (b-cta0[j]) ...
 struct RitzJobDev {
   int R, nvmax, ld, K, cta0, pad;
   const double* alpha;
@@ -329,15 +321,20 @@ struct RitzJobDev {
   int* status;
 };
 
-__global__ void k_tridiag_many(int njobs, const RitzJobDev* __restrict__ jobs, int smem) {
+__global__ void __launch_bounds__(32 * kRitzWarps) k_tridiag_many(int njobs, const RitzJobDev* __restrict__ jobs,
+                                                                  int smem) {
   extern __shared__ double sm[];
   int j = 0;
-  while (j + 1 < njobs && jobs[j + 1].cta0 <= static_cast<int>(blockIdx.x)) ++j;
+  for (int hi = njobs - 1; j < hi;) {
+    const int mid = (j + hi + 1) / 2;
+    if (jobs[mid].cta0 <= static_cast<int>(blockIdx.x)) j = mid;
+    else hi = mid - 1;
+  }
   const RitzJobDev J = jobs[j];
-  const int r = (blockIdx.x - J.cta0) * blockDim.x + threadIdx.x;
+  const int w = threadIdx.x / 32, r = (blockIdx.x - J.cta0) * kRitzWarps + w;
   if (r >= J.R) return;
-  tridiag_vector(r, threadIdx.x, J.nvmax, J.ld, J.K, J.alpha, J.beta, J.steps, J.dout, J.zout, J.escr, 1.0 / J.R,
-                 J.status, sm, smem);
+  tridiag_vector(r, threadIdx.x % 32, J.nvmax, J.ld, J.K, J.alpha, J.beta, J.steps, J.dout, J.zout, J.escr, 1.0 / J.R,
+                 J.status, smem ? sm + static_cast<int64_t>(w) * 3 * smem : nullptr);
 }
 
 // Concatenate the per-vector spectra sample by sample (main.cpp:1097-1110).
@@ -470,19 +467,19 @@ void ritz_stage_many(Ctx& c, std::vector<RitzJob>& jobs) {
     d.w_out = d.ev_out + rk;
     d.total = totals + i;
     d.status = status + i;
-    ctas += (jb.R + 31) / 32;
+    ctas += (jb.R + kRitzWarps - 1) / kRitzWarps;
     kmax = std::max(kmax, jb.K);
     rmax = std::max(rmax, jb.R);
   }
   c.ritz_meta.ensure(sizeof(RitzJobDev) * nj);
   FTLM_CUDA(cudaMemcpyAsync(c.ritz_meta.p, dj.data(), sizeof(RitzJobDev) * nj, cudaMemcpyHostToDevice, c.stream));
-  const size_t tsmem = sizeof(double) * 3 * 32 * static_cast<size_t>(kmax);
+  const size_t tsmem = sizeof(double) * 3 * kRitzWarps * static_cast<size_t>(kmax);
   const int use_smem = tsmem <= 200 * 1024;
   if (use_smem && tsmem > 48 * 1024)
     FTLM_CUDA(cudaFuncSetAttribute(k_tridiag_many, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    static_cast<int>(tsmem)));
-  k_tridiag_many<<<ctas, 32, use_smem ? tsmem : 0, c.stream>>>(static_cast<int>(nj), c.ritz_meta.as<RitzJobDev>(),
-                                                              use_smem);
+  k_tridiag_many<<<ctas, 32 * kRitzWarps, use_smem ? tsmem : 0, c.stream>>>(
+      static_cast<int>(nj), c.ritz_meta.as<RitzJobDev>(), use_smem ? kmax : 0);
   k_compact_many<<<static_cast<int>(nj), 256, sizeof(int) * (rmax + 1), c.stream>>>(c.ritz_meta.as<RitzJobDev>());
   FTLM_LAUNCH_CHECK();
   c.prof.kernel_launches += 2;
