@@ -114,6 +114,36 @@ void check_k(Ctx& c, int mx, int my) {
 using ftlm::Ctx;
 using ftlm::Error;
 
+namespace ftlm {
+
+std::vector<DBuf*> table_bufs(Ctx& c) {
+  SectorTables& s = c.sec;
+  BlockTables& b = c.blk;
+  return {&s.ups, &s.dns, &s.up_info, &s.ur_bits, &s.ur_class, &s.ur_poff, &s.d_star, &s.d_hs, &s.d_stab, &s.d_chi,
+          &s.d_cidx, &s.canon, &s.tmp_a, &s.tmp_b, &s.tmp_c, &s.tmp_d, &s.tmp_e, &b.act, &b.act_list, &b.aoff,
+          &b.dtab, &b.row_meta, &b.row_dn, &c.scan_tmp, &c.stn_crb, &c.stn_rp, &c.stn_ent, &c.stn_cnt, &c.stn_rp4,
+          &c.stn_row, &c.stn_ent4, &c.stn_deg, &c.stn_coef, &c.stn_seg, &c.stn_cls, &c.stn_pos, &c.stn_diag};
+}
+
+namespace {
+
+std::vector<DBuf*> all_bufs(Ctx& c) {
+  std::vector<DBuf*> all = table_bufs(c);
+  for (DBuf* b :
+       {&c.binom, &c.binom32, &c.vec_a, &c.vec_b, &c.vec_h, &c.vec_xd, &c.vec_yd, &c.partial, &c.lz_alpha, &c.lz_beta,
+        &c.lz_scale, &c.lz_state, &c.host_start, &c.gauss_jobs, &c.ritz_tmp, &c.ritz_out, &c.ritz_meta, &c.sb_ent,
+        &c.sb_cnt, &c.sb_diag, &c.sb_start, &c.sb_meta, &c.sb_steps, &c.sb_alpha, &c.sb_beta, &c.pack.act,
+        &c.pack.act_list, &c.pack.dtab, &c.pack.aoff, &c.pack.nact, &c.pack.dims, &c.pack.row_meta, &c.pack.row_dn,
+        &c.pack.phase, &c.pack.items, &c.dense_arena, &c.dense_meta, &c.dense_out, &c.dense_vecs, &c.spectra,
+        &c.th_beta, &c.th_mu, &c.th_state, &c.hl_ptr, &c.hl_ent, &c.flip_map, &c.seg_counter,
+        &c.defer_arena, &c.defer_ev, &c.defer_work})
+    all.push_back(b);
+  return all;
+}
+
+}  // namespace
+}  // namespace ftlm
+
 extern "C" {
 
 int ftlm_abi_version(void) { return FTLM_ABI_VERSION; }
@@ -178,6 +208,7 @@ int ftlm_ctx_create(const ftlm_model* model, const ftlm_run_opts* opts, ftlm_ctx
     FTLM_CUDA(cudaSetDevice(c.device));
     FTLM_CUDA(cudaStreamCreateWithFlags(&c.stream, cudaStreamNonBlocking));
     FTLM_CUDA(cudaDeviceGetAttribute(&c.sm_count, cudaDevAttrMultiProcessorCount, c.device));
+    for (auto* b : ftlm::all_bufs(c)) b->arena = &c.arena;
     ftlm::setup_geometry(c);
     ftlm::setup_binom(c);
   } catch (const Error&) {
@@ -199,31 +230,12 @@ void ftlm_ctx_destroy(ftlm_ctx* ctx) {
       cudaStreamDestroy(s);
     }
   if (c.side_ev) cudaEventDestroy(c.side_ev);
-  ftlm::DBuf* bufs[] = {&c.binom, &c.binom32, &c.sec.ups, &c.sec.dns, &c.sec.up_info, &c.sec.ur_bits,
-                        &c.sec.ur_class, &c.sec.ur_poff, &c.sec.d_star, &c.sec.d_hs, &c.sec.d_stab,
-                        &c.sec.d_chi, &c.sec.d_cidx, &c.sec.canon, &c.sec.tmp_a, &c.sec.tmp_b, &c.sec.tmp_c,
-                        &c.sec.tmp_d, &c.sec.tmp_e, &c.blk.act, &c.blk.act_list, &c.blk.aoff, &c.blk.dtab,
-                        &c.blk.row_meta, &c.blk.row_dn, &c.vec_a, &c.vec_b, &c.vec_h, &c.partial,
-                        &c.lz_alpha, &c.lz_beta, &c.lz_scale, &c.lz_state, &c.host_start, &c.ritz_tmp, &c.ritz_out, &c.ritz_meta,
-                        &c.sb_ent, &c.sb_cnt, &c.sb_diag, &c.sb_start, &c.sb_meta, &c.sb_steps, &c.sb_alpha, &c.sb_beta,
-                        &c.pack.act, &c.pack.act_list, &c.pack.dtab, &c.pack.aoff, &c.pack.nact, &c.pack.dims,
-                        &c.pack.row_meta, &c.pack.row_dn, &c.pack.phase, &c.pack.items,
-                        &c.scan_tmp, &c.dense_arena, &c.dense_meta, &c.dense_out, &c.dense_vecs, &c.spectra, &c.th_beta,
-                        &c.th_mu, &c.th_state, &c.hl_ptr, &c.hl_ent, &c.flip_map, &c.vec_xd, &c.vec_yd, &c.seg_counter, &c.gauss_jobs, &c.stn_crb, &c.stn_rp, &c.stn_ent, &c.stn_cnt,
-                        &c.stn_rp4, &c.stn_row, &c.stn_ent4, &c.stn_deg, &c.stn_coef, &c.stn_seg, &c.stn_cls, &c.stn_pos, &c.stn_diag,
-                        &c.defer_arena, &c.defer_ev, &c.defer_work};
-  for (auto* b : bufs) b->release();
+  for (auto* b : ftlm::all_bufs(c)) b->release();
   if (c.flipped) {
-    ftlm::Ctx& f = *c.flipped;
-    ftlm::DBuf* fb[] = {&f.sec.ups, &f.sec.dns, &f.sec.up_info, &f.sec.ur_bits, &f.sec.ur_class, &f.sec.ur_poff,
-                        &f.sec.d_star, &f.sec.d_hs, &f.sec.d_stab, &f.sec.d_chi, &f.sec.d_cidx, &f.sec.canon,
-                        &f.sec.tmp_a, &f.sec.tmp_b, &f.sec.tmp_c, &f.sec.tmp_d, &f.sec.tmp_e, &f.blk.act,
-                        &f.blk.act_list, &f.blk.aoff, &f.blk.dtab, &f.blk.row_meta, &f.blk.row_dn, &f.scan_tmp,
-                        &f.stn_crb, &f.stn_rp, &f.stn_ent, &f.stn_cnt,
-                        &f.stn_rp4, &f.stn_row, &f.stn_ent4, &f.stn_deg, &f.stn_coef, &f.stn_seg, &f.stn_cls, &f.stn_pos, &f.stn_diag};
-    for (auto* b : fb) b->release();  // binom tables are the owner's
+    for (auto* b : ftlm::table_bufs(*c.flipped)) b->release();  // binom tables are the owner's
     c.flipped.reset();
   }
+  c.arena.release();
   if (c.stream) cudaStreamDestroy(c.stream);
   delete ctx;
 }

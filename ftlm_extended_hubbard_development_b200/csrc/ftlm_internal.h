@@ -30,42 +30,92 @@ struct Error : std::runtime_error {
 
 #define FTLM_LAUNCH_CHECK() FTLM_CUDA(cudaGetLastError())
 
+// Small device buffers of one context, cut from slabs that live as long as the
+// context. A curve on a small lattice creates about 70 buffers and grows them, and
+// a cudaMalloc and a cudaFree of each (which also wait for the device) took 0.1 to
+// 1 ms apiece, by host: 15-30% of a curve. A region that a growing buffer leaves
+// is not used again, so nothing waits for the kernels that still read it; sizes
+// double, so what is left behind stays below what is in use.
+//
+// Slabs grow from 256 KB (enough for the smallest calls, and cheap to get) to 64 MB.
+struct Arena {
+  static constexpr size_t kLast = size_t(64) << 20;
+  static constexpr size_t kMax = size_t(32) << 20;  // largest buffer taken from a slab
+  size_t first = size_t(256) << 10;  // the first slab's size
+  std::vector<void*> slabs;
+  size_t used = 0, size = 0;  // of the last slab
+  void* take(size_t bytes) {
+    bytes = (bytes + 255) / 256 * 256;
+    if (used + bytes > size) {
+      const size_t next = std::max(bytes, std::min(kLast, std::max(first, 4 * size)));
+      void* p = nullptr;
+      FTLM_CUDA(cudaMalloc(&p, next));
+      slabs.push_back(p);
+      size = next;
+      used = 0;
+    }
+    void* q = static_cast<char*>(slabs.back()) + used;
+    used += bytes;
+    return q;
+  }
+  void release() {
+    for (void* p : slabs) cudaFree(p);
+    slabs.clear();
+    used = size = 0;
+  }
+};
+
 // Grow-only device buffer owned by a context.
 struct DBuf {
   void* p = nullptr;
   size_t cap = 0;
+  Arena* arena = nullptr;  // where it is taken from up to Arena::kMax bytes
+  bool own = false;        // p is an allocation of its own
   void ensure(size_t bytes) {
     if (bytes <= cap) return;
-    // small buffers grow by doubling from 64 KB: a curve over many small
-    // sectors otherwise spends its time in cudaMalloc / cudaFree
-    if (bytes <= kSmallBytes) bytes = std::max(bytes, std::max(kFirstBytes, std::min(2 * cap, kSmallBytes)));
-    if (p) FTLM_CUDA(cudaFree(p));
-    p = nullptr;
-    cap = 0;
-    FTLM_CUDA(cudaMalloc(&p, bytes));
-    cap = bytes;
+    // small buffers grow by doubling, from 4 KB in a slab and 64 KB alone: a curve
+    // over many small sectors otherwise spends its time growing them
+    const size_t first = arena ? kFirstBytes / 16 : kFirstBytes;
+    if (bytes <= kSmallBytes) bytes = std::max(bytes, std::max(first, std::min(2 * cap, kSmallBytes)));
+    release();
+    get(bytes);
   }
   static constexpr size_t kFirstBytes = size_t(64) << 10, kSmallBytes = size_t(16) << 20;
   // Grows (by at least half) keeping the first `cap` bytes; stream-ordered copy.
   void ensure_keep(size_t bytes, cudaStream_t stream) {
     if (bytes <= cap) return;
-    const size_t want = std::max(bytes, std::max(cap + cap / 2, size_t(1) << 20));
-    void* q = nullptr;
-    FTLM_CUDA(cudaMalloc(&q, want));
-    if (p) {
-      FTLM_CUDA(cudaMemcpyAsync(q, p, cap, cudaMemcpyDeviceToDevice, stream));
-      FTLM_CUDA(cudaStreamSynchronize(stream));
-      FTLM_CUDA(cudaFree(p));
+    DBuf old = *this;
+    p = nullptr;
+    cap = 0;
+    try {
+      get(std::max(bytes, std::max(old.cap + old.cap / 2, arena ? size_t(64) << 10 : size_t(1) << 20)));
+    } catch (...) {
+      *this = old;
+      throw;
     }
-    p = q;
-    cap = want;
+    if (!old.p) return;
+    FTLM_CUDA(cudaMemcpyAsync(p, old.p, old.cap, cudaMemcpyDeviceToDevice, stream));
+    if (old.own) FTLM_CUDA(cudaStreamSynchronize(stream));
+    old.release();
   }
   template <typename T>
   T* as() const { return static_cast<T*>(p); }
   void release() {
-    if (p) cudaFree(p);
+    if (p && own) cudaFree(p);
     p = nullptr;
     cap = 0;
+  }
+
+ private:
+  void get(size_t bytes) {
+    if (arena && bytes <= Arena::kMax) {
+      p = arena->take(bytes);
+      own = false;
+    } else {
+      FTLM_CUDA(cudaMalloc(&p, bytes));
+      own = true;
+    }
+    cap = bytes;
   }
 };
 
@@ -242,6 +292,7 @@ struct FlipPhase {
 constexpr int64_t kSmallMaxDim = 4096;
 
 struct Ctx {
+  Arena arena;  // small buffers of this context and its spin-flipped companion
   ftlm_model model{};
   ftlm_run_opts opts{};
   Geom geom{};
@@ -463,6 +514,8 @@ struct GaussJob {
 void gaussian_starts(Ctx& c, const std::vector<GaussJob>& jobs, double2* out);
 // Seed of sample `sample` of the block with seed bseed (main.cpp:1015).
 uint64_t sample_seed(uint64_t bseed, int sample);
+// The buffers of a context's sector, block and stencil tables.
+std::vector<DBuf*> table_bufs(Ctx& c);
 // Nonzero-amplitude hops with active targets in the prepared block (the
 // h_nz * dim of the H*V byte model).
 int64_t block_nonzero_hops(Ctx& c);

@@ -406,6 +406,7 @@ int64_t spectra_alloc(Ctx& c, int64_t count) {
   const int64_t need = c.spectra_used + count;
   if (static_cast<size_t>(need) * sizeof(double) > c.spectra.cap) {
     DBuf n;
+    n.arena = c.spectra.arena;
     n.ensure(sizeof(double) * std::max<int64_t>(need * 2, 1 << 16));
     if (c.spectra_used > 0)
       FTLM_CUDA(cudaMemcpyAsync(n.p, c.spectra.p, sizeof(double) * c.spectra_used, cudaMemcpyDeviceToDevice, c.stream));
@@ -527,12 +528,14 @@ void run_ftlm_block(Ctx& c, int n_up, int n_dn, int mx, int my, Spectrum& out, c
     // 2 GiB to spare (wider sweeps cost less per vector at every width
     // measured); a large block counts the split sweeps' five arrays.
     size_t free_b = 0, total_b = 0;
-    FTLM_CUDA(cudaMemGetInfo(&free_b, &total_b));
     const size_t have = c.vec_a.cap + c.vec_b.cap + c.vec_h.cap + c.vec_xd.cap + c.vec_yd.cap;
     const size_t arrays = D >= kSplitMinDim ? 5 : 3;
     while (nvmax > 1) {
       const size_t nv = static_cast<size_t>(next_pow2(std::max(nvmax, fp32 ? 2 : 1)));
-      if (arrays * static_cast<size_t>(D) * nv * (fp32 ? 8 : 16) + (size_t(2) << 30) <= free_b + have) break;
+      const size_t need = arrays * static_cast<size_t>(D) * nv * (fp32 ? 8 : 16);
+      if (need <= have) break;
+      if (!total_b) FTLM_CUDA(cudaMemGetInfo(&free_b, &total_b));  // 0.1 ms and more: only where it decides
+      if (need + (size_t(2) << 30) <= free_b + have) break;
       nvmax = std::max(1, nvmax / 2);
     }
   }

@@ -30,6 +30,7 @@ struct ftlm_mlp {
   ftlm::DBuf data_x, data_t, data_m, batch_idx, batch_x, batch_t, batch_m, red, io;
   ftlm::DBuf perm, history;  // training order of one epoch; per-epoch loss sums
   ftlm::DBuf row_sum;        // sum of every training row's mask
+  ftlm::Arena arena;
   std::vector<ftlm::DBuf*> bufs() {
     return {&params, &grads, &adam_m, &adam_v, &act, &dact, &data_x, &data_t, &data_m, &batch_idx, &batch_x,
             &batch_t, &batch_m, &red, &io, &perm, &history, &row_sum};
@@ -721,6 +722,8 @@ int ftlm_mlp_create(int32_t n_in, int32_t width, int32_t depth, int32_t n_out, u
   try {
     FTLM_CUDA(cudaSetDevice(device));
     FTLM_CUDA(cudaStreamCreateWithFlags(&net->stream, cudaStreamNonBlocking));
+    net->arena.first = size_t(16) << 20;  // a training set and its batches
+    for (auto* b : net->bufs()) b->arena = &net->arena;
     net->params.ensure(sizeof(float) * off);
     net->grads.ensure(sizeof(float) * off);
     net->adam_m.ensure(sizeof(float) * off);
@@ -741,6 +744,7 @@ void ftlm_mlp_destroy(ftlm_mlp* net) {
   cudaSetDevice(net->device);
   if (net->stream) cudaStreamSynchronize(net->stream);
   for (auto* x : net->bufs()) x->release();
+  net->arena.release();
   if (net->stream) cudaStreamDestroy(net->stream);
   delete net;
 }

@@ -65,7 +65,7 @@ __global__ void k_scan_tile_offsets(int64_t* __restrict__ sums, int64_t ntiles, 
 }
 
 __global__ void k_scan_apply(const int32_t* __restrict__ in, int64_t n, const int64_t* __restrict__ offs,
-                             int64_t* __restrict__ out) {
+                             int64_t* __restrict__ out, int64_t* __restrict__ total) {
   __shared__ int64_t buf[kScanThreads];
   const int64_t base = static_cast<int64_t>(blockIdx.x) * kScanTile;
   int64_t loc[kScanItems];
@@ -83,7 +83,8 @@ __global__ void k_scan_apply(const int32_t* __restrict__ in, int64_t n, const in
     buf[threadIdx.x] += t;
     __syncthreads();
   }
-  const int64_t pre = offs[blockIdx.x] + buf[threadIdx.x] - s;
+  const int64_t pre = (offs ? offs[blockIdx.x] : 0) + buf[threadIdx.x] - s;
+  if (total && threadIdx.x == kScanThreads - 1) *total = pre + s;
   for (int i = 0; i < kScanItems; ++i) {
     const int64_t idx = base + static_cast<int64_t>(threadIdx.x) * kScanItems + i;
     if (idx < n) out[idx] = pre + loc[i];
@@ -601,14 +602,19 @@ int64_t scan_excl_i32_to_i64(Ctx& c, const int32_t* flags, int64_t* out, int64_t
   DBuf& tiles = c.scan_tmp;
   tiles.ensure(sizeof(int64_t) * (ntiles + 1));
   int64_t* ts = tiles.as<int64_t>();
-  k_scan_tiles<<<static_cast<unsigned>(ntiles), kScanThreads, 0, c.stream>>>(flags, n, ts);
-  k_scan_tile_offsets<<<1, kScanThreads, 0, c.stream>>>(ts, ntiles, ts + ntiles);
-  k_scan_apply<<<static_cast<unsigned>(ntiles), kScanThreads, 0, c.stream>>>(flags, n, ts, out);
+  if (ntiles == 1) {  // one launch for the short scans, 2-3 per sector, of a small lattice
+    k_scan_apply<<<1, kScanThreads, 0, c.stream>>>(flags, n, nullptr, out, ts + ntiles);
+    c.prof.kernel_launches += 1;
+  } else {
+    k_scan_tiles<<<static_cast<unsigned>(ntiles), kScanThreads, 0, c.stream>>>(flags, n, ts);
+    k_scan_tile_offsets<<<1, kScanThreads, 0, c.stream>>>(ts, ntiles, ts + ntiles);
+    k_scan_apply<<<static_cast<unsigned>(ntiles), kScanThreads, 0, c.stream>>>(flags, n, ts, out, nullptr);
+    c.prof.kernel_launches += 3;
+  }
   FTLM_LAUNCH_CHECK();
   int64_t total = 0;
   FTLM_CUDA(cudaMemcpyAsync(&total, ts + ntiles, sizeof(int64_t), cudaMemcpyDeviceToHost, c.stream));
   FTLM_CUDA(cudaStreamSynchronize(c.stream));
-  c.prof.kernel_launches += 3;
   return total;
 }
 

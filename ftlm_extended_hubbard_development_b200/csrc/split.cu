@@ -856,6 +856,7 @@ Ctx& flipped_tables(Ctx& c) {
     f.device = c.device;
     f.sm_count = c.sm_count;
     f.stream = c.stream;
+    for (DBuf* b : table_bufs(f)) b->arena = &c.arena;
     f.binom = c.binom;  // shared, owned by c
     f.binom32 = c.binom32;
   }
@@ -1168,9 +1169,11 @@ bool split_prepare(Ctx& c, int nv, bool fp32) {
   const size_t vec = static_cast<size_t>(D) * pow2 * esize;
   const size_t need = 2 * vec + (sizeof(uint64_t) + 2 * sizeof(uint32_t) + esize / 2) * D;
   const size_t have = c.vec_xd.cap + c.vec_yd.cap + c.flip_map.cap + c.stn_pos.cap + c.stn_diag.cap;
-  size_t free_b = 0, total_b = 0;
-  FTLM_CUDA(cudaMemGetInfo(&free_b, &total_b));
-  if (need > have && need + (size_t(2) << 30) > free_b + have) return false;  // keep 2 GiB headroom
+  if (need > have) {  // keep 2 GiB headroom
+    size_t free_b = 0, total_b = 0;
+    FTLM_CUDA(cudaMemGetInfo(&free_b, &total_b));
+    if (need + (size_t(2) << 30) > free_b + have) return false;
+  }
   Ctx& f = flipped_tables(c);
   c.split_wide = false;
   if (c.split_stencil) {
