@@ -411,7 +411,7 @@ int hv_grid(Ctx& c, int nv, bool fp32);
 // blocks); builds what it needs and sets c.hl_active / c.split_active. The
 // guard clears them again.
 enum { kSrcFly = 0, kSrcList = 1, kSrcSplit = 2 };
-constexpr int64_t kSplitMinDim = int64_t(1) << 15;
+constexpr int64_t kSplitMinDim = int64_t(1) << 15, kSplitMinDimFp64 = 12288;  // the latter for wide FP64 sweeps
 int hv_select_source(Ctx& c, int nv, bool fp32);
 struct HvSourceGuard {
   Ctx& c;

@@ -810,7 +810,10 @@ int hv_select_source(Ctx& c, int nv, bool fp32) {
     // kernel in 1.56 (and the list takes 5.8 ms to build); without the stencils
     // (more than 65536 down words) one-chunk rows stay on the hop list.
     one_chunk = nv == (fp32 ? 2 : 1);
-    if (D >= kSplitMinDim) mode = kSrcSplit;
+    // Wide FP64 sweeps gain from 12288 rows (40 steps, block set up included:
+    // 13805 rows 128 vectors 7.0 -> 6.2 ms, 32 vectors 3.4 -> 3.2; 19600 rows 11.9 ->
+    // 7.3 and 4.0 -> 3.5); narrow and FP32 ones do not (5 vectors 2.3 -> 2.4).
+    if (D >= kSplitMinDim || (D >= kSplitMinDimFp64 && !fp32 && nv >= 32)) mode = kSrcSplit;
     else if (D >= (1 << 14) && nv <= (fp32 ? 32 : 16)) mode = kSrcList;
     else mode = kSrcFly;
   }

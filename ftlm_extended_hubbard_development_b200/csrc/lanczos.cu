@@ -529,7 +529,7 @@ void run_ftlm_block(Ctx& c, int n_up, int n_dn, int mx, int my, Spectrum& out, c
     // measured); a large block counts the split sweeps' five arrays.
     size_t free_b = 0, total_b = 0;
     const size_t have = c.vec_a.cap + c.vec_b.cap + c.vec_h.cap + c.vec_xd.cap + c.vec_yd.cap;
-    const size_t arrays = D >= kSplitMinDim ? 5 : 3;
+    const size_t arrays = D >= kSplitMinDimFp64 ? 5 : 3;
     while (nvmax > 1) {
       const size_t nv = static_cast<size_t>(next_pow2(std::max(nvmax, fp32 ? 2 : 1)));
       const size_t need = arrays * static_cast<size_t>(D) * nv * (fp32 ? 8 : 16);
