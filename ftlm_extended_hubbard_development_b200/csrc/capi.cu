@@ -471,24 +471,42 @@ int ftlm_block_apply(ftlm_ctx* ctx, int32_t mx, int32_t my, int32_t nvec, const 
     const size_t bytes = static_cast<size_t>(D) * NV * esize;
     c.vec_a.ensure(bytes + ftlm::kSweepPad);
     c.vec_h.ensure(bytes);
-    // pack host [dim][nvec] FP64 complex into [dim][NV] of the working precision
-    std::vector<char> h(bytes, 0);
-    for (int64_t i = 0; i < D; ++i)
-      for (int v = 0; v < nvec; ++v) {
-        const double re = in[2 * (i * nvec + v)], im = in[2 * (i * nvec + v) + 1];
-        if (fp32) {
-          float* p = reinterpret_cast<float*>(h.data()) + 2 * (i * NV + v);
-          p[0] = static_cast<float>(re);
-          p[1] = static_cast<float>(im);
-        } else {
-          double* p = reinterpret_cast<double*>(h.data()) + 2 * (i * NV + v);
-          p[0] = re;
-          p[1] = im;
+    // Host [dim][nvec] FP64 complex to [dim][NV] of the working precision and the
+    // sweeps' row order, and back. The copies are the caller's own arrays and the
+    // GPU converts; what is as it is (FP64, no padding, block order) needs no
+    // conversion, and a few KB are converted on the host at some 4 ns an element,
+    // where two more launches would take longer (8 us). 4x4 (3,4), 16 vectors, 16 MB
+    // each way: 7.1 -> 5.5 ms, of which 2 are copies and the rest page faults of
+    // the caller's fresh arrays.
+    const int64_t elems = D * nvec;
+    const bool as_is = !fp32 && NV == nvec && !reorder;
+    const bool on_host = !as_is && !reorder && elems < ftlm::kHostConvert;
+    const size_t raw = sizeof(double) * 2 * static_cast<size_t>(elems);
+    std::vector<char> h;
+    if (as_is) {
+      FTLM_CUDA(cudaMemcpyAsync(c.vec_a.p, in, raw, cudaMemcpyHostToDevice, c.stream));
+      c.prof.h2d_bytes += static_cast<int64_t>(raw);
+    } else if (on_host) {
+      h.assign(bytes, 0);
+      for (int64_t i = 0; i < D; ++i)
+        for (int v = 0; v < nvec; ++v) {
+          const double re = in[2 * (i * nvec + v)], im = in[2 * (i * nvec + v) + 1];
+          if (fp32) {
+            float* p = reinterpret_cast<float*>(h.data()) + 2 * (i * NV + v);
+            p[0] = static_cast<float>(re);
+            p[1] = static_cast<float>(im);
+          } else {
+            double* p = reinterpret_cast<double*>(h.data()) + 2 * (i * NV + v);
+            p[0] = re;
+            p[1] = im;
+          }
         }
-      }
-    FTLM_CUDA(cudaMemcpyAsync(reorder ? c.vec_h.p : c.vec_a.p, h.data(), bytes, cudaMemcpyHostToDevice, c.stream));
-    c.prof.h2d_bytes += static_cast<int64_t>(bytes);
-    if (reorder) ftlm::sweep_reorder(c, false, c.vec_h.p, c.vec_a.p, NV, fp32);
+      FTLM_CUDA(cudaMemcpyAsync(c.vec_a.p, h.data(), bytes, cudaMemcpyHostToDevice, c.stream));
+      c.prof.h2d_bytes += static_cast<int64_t>(bytes);
+    } else {
+      ftlm::vectors_from_host(c, nvec, NV, fp32, in, c.vec_a.p);
+      c.prof.h2d_bytes += static_cast<int64_t>(raw);
+    }
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     if (c.timing) {
       FTLM_CUDA(cudaEventCreate(&e0));
@@ -505,10 +523,14 @@ int ftlm_block_apply(ftlm_ctx* ctx, int32_t mx, int32_t my, int32_t nvec, const 
     if (c.timing) {
       FTLM_CUDA(cudaEventRecord(e1, c.stream));
     }
-    if (reorder) ftlm::sweep_reorder(c, true, c.vec_h.p, c.vec_a.p, NV, fp32);
-    FTLM_CUDA(cudaMemcpyAsync(h.data(), reorder ? c.vec_a.p : c.vec_h.p, bytes, cudaMemcpyDeviceToHost, c.stream));
+    const size_t back_bytes = on_host ? bytes : raw;
+    if (as_is || on_host)
+      FTLM_CUDA(cudaMemcpyAsync(on_host ? static_cast<void*>(h.data()) : static_cast<void*>(out), c.vec_h.p, back_bytes,
+                                cudaMemcpyDeviceToHost, c.stream));
+    else
+      ftlm::vectors_to_host(c, nvec, NV, fp32, c.vec_h.p, out);
     FTLM_CUDA(cudaStreamSynchronize(c.stream));
-    c.prof.d2h_bytes += static_cast<int64_t>(bytes);
+    c.prof.d2h_bytes += static_cast<int64_t>(back_bytes);
     if (c.timing) {
       float ms = 0.f;
       FTLM_CUDA(cudaEventElapsedTime(&ms, e0, e1));
@@ -522,6 +544,7 @@ int ftlm_block_apply(ftlm_ctx* ctx, int32_t mx, int32_t my, int32_t nvec, const 
       c.prof.hv_hops += nzh * nvec;
       c.prof.hv_min_bytes += static_cast<double>(D) * (2.0 * nvec * s + 8.0);
     }
+    if (!on_host) return;
     for (int64_t i = 0; i < D; ++i)
       for (int v = 0; v < nvec; ++v) {
         if (fp32) {

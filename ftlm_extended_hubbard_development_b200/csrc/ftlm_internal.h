@@ -446,8 +446,13 @@ int hv_apply_split(Ctx& c, const void* in, const void* in_d, void* out, void* ou
 const uint32_t* sweep_pos(const Ctx& c);
 constexpr size_t kSweepPad = 2048;
 inline int sweep_width(int nvec, bool fp32) { return fp32 ? (nvec + 1) / 2 * 2 : nvec; }
-// Vectors from block order to the sweeps' order, or back.
-void sweep_reorder(Ctx& c, bool to_block, const void* src, void* dst, int nv, bool fp32);
+// Host vectors ([dim][nvec] complex FP64, block order) to [dim][NV] of the working
+// precision in the operator's row order, and back, kConvertChunk elements at a
+// time (256 MB on the device, whatever the block).
+void vectors_from_host(Ctx& c, int nvec, int NV, bool fp32, const double* in, void* vec);
+void vectors_to_host(Ctx& c, int nvec, int NV, bool fp32, const void* vec, double* out);
+constexpr int64_t kConvertChunk = int64_t(1) << 24;
+constexpr int64_t kHostConvert = 2048;  // elements below which the host converts
 int hv_split_max_grid(const Ctx& c);
 // x_D[p(q)] = conj(f_q) x[q];  y[q] += f_q y_D[p(q)].
 void flip_scatter(Ctx& c, const void* x, void* xd, int nv, bool fp32);

@@ -1164,11 +1164,16 @@ bool split_prepare(Ctx& c, int nv, bool fp32) {
   // memory: two extra vector arrays (flipped x and y), the 8-byte map, and per
   // row two positions and the diagonal
   const size_t esize = fp32 ? 8 : 16;
-  int pow2 = fp32 ? 2 : 1;  // the on-the-fly sweeps' width
+  // the on-the-fly sweeps take powers of two; the stencil ones, which nearly
+  // every lattice takes, as many as there are
+  int pow2 = fp32 ? 2 : 1;
   while (pow2 < nv) pow2 <<= 1;
-  const size_t vec = static_cast<size_t>(D) * pow2 * esize;
-  const size_t need = 2 * vec + (sizeof(uint64_t) + 2 * sizeof(uint32_t) + esize / 2) * D;
-  const size_t have = c.vec_xd.cap + c.vec_yd.cap + c.flip_map.cap + c.stn_pos.cap + c.stn_diag.cap;
+  const bool likely = c.split_stencil && std::max(c.sec.c_up, c.sec.c_dn) <= kStencilMaxRows;
+  const size_t vec = static_cast<size_t>(D) * (likely ? nv : pow2) * esize;
+  const bool two = c.sec.n_up != c.sec.n_dn;
+  const size_t need = 2 * vec + (sizeof(uint64_t) + (two ? 2 : 1) * sizeof(uint32_t) + esize / 2) * D;
+  const size_t have = c.vec_xd.cap + c.vec_yd.cap + c.flip_map.cap + c.stn_pos.cap + c.stn_diag.cap +
+                      (two && c.flipped ? c.flipped->stn_pos.cap : 0);
   if (need > have) {  // keep 2 GiB headroom
     size_t free_b = 0, total_b = 0;
     FTLM_CUDA(cudaMemGetInfo(&free_b, &total_b));
@@ -1256,25 +1261,70 @@ int hv_apply_split(Ctx& c, const void* in, const void* in_d, void* out, void* ou
   return 2 * grid;
 }
 
-// dst[pos[q]] = src[q], or dst[q] = src[pos[q]], for every 16-byte chunk.
-template <typename V>
-__global__ void k_reorder(int64_t dim, int CPR, bool gather, const uint32_t* __restrict__ pos,
-                          const V* __restrict__ src, V* __restrict__ dst) {
-  const int64_t n = dim * CPR;
+// vec[pos[q]][v] = raw[q - row0][v], zero for v >= nvec (pos null: q), for `rows`
+// rows from row0, one thread per element.
+template <typename T2>
+__global__ void k_vectors_in(int64_t row0, int64_t rows, int nvec, int NV, const uint32_t* __restrict__ pos,
+                             const double2* __restrict__ raw, T2* __restrict__ vec) {
+  const int64_t n = rows * NV;
   for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < n;
        i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const int64_t row = i / CPR, j = static_cast<int64_t>(pos[row]) * CPR + (i - row * CPR);
-    if (gather) dst[i] = src[j];
-    else dst[j] = src[i];
+    const int64_t row = i / NV, q = row0 + row;
+    const int v = static_cast<int>(i - row * NV);
+    T2 z{0, 0};
+    if (v < nvec) {
+      const double2 r = raw[row * nvec + v];
+      z.x = static_cast<decltype(z.x)>(r.x);
+      z.y = static_cast<decltype(z.x)>(r.y);
+    }
+    vec[(pos ? pos[q] : q) * NV + v] = z;
   }
 }
 
-void sweep_reorder(Ctx& c, bool to_block, const void* src, void* dst, int nv, bool fp32) {
-  const int CPR = fp32 ? nv / 2 : nv;
-  k_reorder<float4><<<grid_rows(c.blk.dim * CPR, 256), 256, 0, c.stream>>>(
-      c.blk.dim, CPR, to_block, c.stn_pos.as<uint32_t>(), static_cast<const float4*>(src), static_cast<float4*>(dst));
-  FTLM_LAUNCH_CHECK();
-  c.prof.kernel_launches += 1;
+template <typename T2>
+__global__ void k_vectors_out(int64_t row0, int64_t rows, int nvec, int NV, const uint32_t* __restrict__ pos,
+                              const T2* __restrict__ vec, double2* __restrict__ raw) {
+  const int64_t n = rows * nvec;
+  for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < n;
+       i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+    const int64_t row = i / nvec, q = row0 + row;
+    const T2 z = vec[(pos ? pos[q] : q) * NV + (i - row * nvec)];
+    raw[i] = make_double2(z.x, z.y);
+  }
+}
+
+// f(first row, rows) for the chunks of a block.
+template <typename F>
+void convert_chunks(Ctx& c, int nvec, F&& f) {
+  const int64_t D = c.blk.dim, step = std::max<int64_t>(1, kConvertChunk / nvec);
+  c.host_start.ensure(sizeof(double2) * static_cast<size_t>(std::min(D, step)) * nvec);
+  for (int64_t r = 0; r < D; r += step) f(r, std::min(step, D - r));
+}
+
+void vectors_from_host(Ctx& c, int nvec, int NV, bool fp32, const double* in, void* vec) {
+  convert_chunks(c, nvec, [&](int64_t r, int64_t rows) {
+    double2* raw = c.host_start.as<double2>();
+    FTLM_CUDA(cudaMemcpyAsync(raw, in + 2 * r * nvec, sizeof(double2) * rows * nvec, cudaMemcpyHostToDevice, c.stream));
+    const int grid = grid_rows(rows * NV, 256);
+    if (fp32) k_vectors_in<<<grid, 256, 0, c.stream>>>(r, rows, nvec, NV, sweep_pos(c), raw, static_cast<float2*>(vec));
+    else k_vectors_in<<<grid, 256, 0, c.stream>>>(r, rows, nvec, NV, sweep_pos(c), raw, static_cast<double2*>(vec));
+    FTLM_LAUNCH_CHECK();
+    c.prof.kernel_launches += 1;
+  });
+}
+
+void vectors_to_host(Ctx& c, int nvec, int NV, bool fp32, const void* vec, double* out) {
+  convert_chunks(c, nvec, [&](int64_t r, int64_t rows) {
+    double2* raw = c.host_start.as<double2>();
+    const int grid = grid_rows(rows * nvec, 256);
+    if (fp32)
+      k_vectors_out<<<grid, 256, 0, c.stream>>>(r, rows, nvec, NV, sweep_pos(c), static_cast<const float2*>(vec), raw);
+    else
+      k_vectors_out<<<grid, 256, 0, c.stream>>>(r, rows, nvec, NV, sweep_pos(c), static_cast<const double2*>(vec), raw);
+    FTLM_LAUNCH_CHECK();
+    FTLM_CUDA(cudaMemcpyAsync(out + 2 * r * nvec, raw, sizeof(double2) * rows * nvec, cudaMemcpyDeviceToHost, c.stream));
+    c.prof.kernel_launches += 1;
+  });
 }
 
 const uint32_t* sweep_pos(const Ctx& c) { return c.split_active && c.split_wide ? c.stn_pos.as<uint32_t>() : nullptr; }

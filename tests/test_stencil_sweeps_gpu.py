@@ -102,3 +102,26 @@ def test_vectors_per_sweep_do_not_change_the_coefficients(monkeypatch, prec, tol
         assert np.array_equal(got[batch][2], s)
         assert np.abs(got[batch][0] - a).max() <= tol * np.abs(a).max(), batch
         assert np.abs(got[batch][1] - b).max() <= tol * np.abs(b).max(), batch
+
+
+@pytest.mark.parametrize("prec", [E.PREC_FP64, E.PREC_MIXED], ids=["fp64", "mixed"])
+def test_host_vectors_of_every_size_are_the_same_vectors(monkeypatch, prec):
+    """Host vectors are converted on the host (few elements), on the device, and
+    there in several chunks (more than 2^24 elements: 4x4 (5,5), 1.19 M rows, 15
+    vectors). A vector's result does not depend on how it came: the same bits
+    alone and among others."""
+    monkeypatch.setenv("FTLM_HV_VARIANT", "1")
+    for (nu, nd), widths in {((2, 3)): (3, 16), ((3, 4)): (3, 7), ((5, 5)): (15,)}.items():
+        with pkg.Engine(model(4, 4), pkg.RunOpts(precision=prec)) as eng:
+            dim = int(eng.sector_prepare(nu, nd).block_dims[0])
+            for nvec in widths:
+                g = np.random.default_rng(nvec)
+                x = g.standard_normal((dim, nvec)) + 1j * g.standard_normal((dim, nvec))
+                y = eng.block_apply(0, 0, x)
+                for v in {0, nvec - 1}:
+                    alone = eng.block_apply(0, 0, np.ascontiguousarray(x[:, v:v + 1]))[:, 0]
+                    if dim >= 1 << 15:  # the same operator at every width
+                        assert np.array_equal(alone, y[:, v]), (nu, nd, nvec, v)
+                    else:
+                        tol = 1e-13 if prec == E.PREC_FP64 else 2e-6
+                        assert np.abs(alone - y[:, v]).max() <= tol * np.abs(y).max(), (nu, nd, nvec, v)
