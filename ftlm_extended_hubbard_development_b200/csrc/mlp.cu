@@ -165,8 +165,8 @@ __global__ void k_adam(int64_t n, float* __restrict__ p, const float* __restrict
 // leaving the SM; k_train_params forms every weight's gradient as one sum over
 // the batch and applies Adam to it in registers. Bound now: the chains of
 // dependent multiply-adds (K per layer, the batch per weight) and the shared
-// loads that feed them: 16 + 18 us a step there; 86 steps with copies and
-// allocations 35 -> 5.4 ms.
+// loads that feed them: 16 + 15 us a step there; 86 steps with copies and
+// allocations 35 -> 5.3 ms.
 
 constexpr int kTrMaxLayers = 17;
 constexpr int kTrThreads = 256;
@@ -394,7 +394,7 @@ __global__ void __launch_bounds__(kTrThreads) k_train_rows(const __grid_constant
 }
 
 constexpr int kTpTile = 16;      // outputs x inputs of a CTA
-constexpr int kTpThreads = 128;  // 1 output x 2 inputs per thread
+constexpr int kTpThreads = 256;  // one weight per thread
 constexpr int kTpRows = 128;     // batch rows per stage
 constexpr int kTpStages = 4;
 
@@ -467,36 +467,32 @@ __global__ void __launch_bounds__(kTpThreads) k_train_params(const __grid_consta
     cp_commit();
   };
   for (int st = 0; st < kTpStages - 1; ++st) load(st);
-  const int to = tid / 8, tj = tid % 8 * 2;
-  float g0 = 0.f, g1 = 0.f, gb = 0.f;
+  const int to = tid / kTpTile, tj = tid % kTpTile;
+  float g0 = 0.f, gb = 0.f;
   for (int st = 0; st < nst; ++st) {
     cp_wait(kTpStages - 2);
     __syncthreads();
     load(st + kTpStages - 1);
     const float* s = sm + st % kTpStages * kTpRows * 2 * kTpTile;
     const int nr = min(kTpRows, N.n - st * kTpRows);
-    // one warp per scheduler: the loads of 16 rows together, else each waits for its own
+    // two warps per scheduler: the loads of 16 rows together, else each waits for its own
     int r = 0;
     for (; r + 16 <= nr; r += 16) {
-      float a[16];
-      float2 b[16];
+      float a[16], b[16];
 #pragma unroll
       for (int u = 0; u < 16; ++u) {
         a[u] = s[(r + u) * 2 * kTpTile + to];
-        b[u] = *reinterpret_cast<const float2*>(s + (r + u) * 2 * kTpTile + kTpTile + tj);
+        b[u] = s[(r + u) * 2 * kTpTile + kTpTile + tj];
       }
 #pragma unroll
       for (int u = 0; u < 16; ++u) {
-        g0 = fmaf(a[u], b[u].x, g0);
-        g1 = fmaf(a[u], b[u].y, g1);
+        g0 = fmaf(a[u], b[u], g0);
         gb += a[u];
       }
     }
     for (; r < nr; ++r) {
       const float a = s[r * 2 * kTpTile + to];
-      const float2 b = *reinterpret_cast<const float2*>(s + r * 2 * kTpTile + kTpTile + tj);
-      g0 = fmaf(a, b.x, g0);
-      g1 = fmaf(a, b.y, g1);
+      g0 = fmaf(a, s[r * 2 * kTpTile + kTpTile + tj], g0);
       gb += a;
     }
   }
@@ -504,7 +500,6 @@ __global__ void __launch_bounds__(kTpThreads) k_train_params(const __grid_consta
   if (o >= fo) return;
   const int64_t w = N.w[l] + static_cast<int64_t>(o) * fi + i;
   if (i < fi) adam_update(A, g0, par + w, am + w, av + w);
-  if (i + 1 < fi) adam_update(A, g1, par + w + 1, am + w + 1, av + w + 1);
   if (i0 == 0 && tj == 0) adam_update(A, gb, par + N.b[l] + o, am + N.b[l] + o, av + N.b[l] + o);
 }
 
