@@ -310,7 +310,7 @@ def run_ours(args):
                          "frac": achieved / peak, "peak_kind": peak_kind,
                          "kernel": (["k_hv (on-the-fly multi-vector H*V)", "k_hv_list (cached hop list)",
                                      "k_hv_stn x2 (split-spin segment sweeps on the class stencils, both "
-                                     "row orders; k_hv_stn_rows at <= 4 chunks per row)"]
+                                     "row orders, one launch)"]
                                     [prof["hv_source"]] if prof["hv_source"] in (0, 1, 2) else "unknown"),
                          "kernel_variant": prof["hv_variant"],
                          "bytes_per_launch": bytes_per_launch,
