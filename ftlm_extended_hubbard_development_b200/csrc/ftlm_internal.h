@@ -37,21 +37,25 @@ struct Error : std::runtime_error {
 // is not used again, so nothing waits for the kernels that still read it; sizes
 // double, so what is left behind stays below what is in use.
 //
-// Slabs grow from 256 KB (enough for the smallest calls, and cheap to get) to 64 MB.
+// Slabs grow from 256 KB to 64 MB: what is held doubles up to 1 MB (small calls stay
+// with allocations the driver has at hand; a larger one takes it 0.4 ms), then each
+// is four times the last.
 struct Arena {
   static constexpr size_t kLast = size_t(64) << 20;
   static constexpr size_t kMax = size_t(32) << 20;  // largest buffer taken from a slab
   size_t first = size_t(256) << 10;  // the first slab's size
   std::vector<void*> slabs;
   size_t used = 0, size = 0;  // of the last slab
+  size_t held = 0;            // all slabs
   void* take(size_t bytes) {
     bytes = (bytes + 255) / 256 * 256;
     if (used + bytes > size) {
-      const size_t next = std::max(bytes, std::min(kLast, std::max(first, 4 * size)));
+      const size_t next = std::max(bytes, std::min(kLast, std::max(first, held < (size_t(1) << 20) ? held : 4 * size)));
       void* p = nullptr;
       FTLM_CUDA(cudaMalloc(&p, next));
       slabs.push_back(p);
       size = next;
+      held += next;
       used = 0;
     }
     void* q = static_cast<char*>(slabs.back()) + used;
@@ -61,7 +65,7 @@ struct Arena {
   void release() {
     for (void* p : slabs) cudaFree(p);
     slabs.clear();
-    used = size = 0;
+    used = size = held = 0;
   }
 };
 
