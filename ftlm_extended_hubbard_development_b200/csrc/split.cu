@@ -1208,7 +1208,9 @@ int seg_variant(Ctx& c, const void* in, void* out, int nv, bool fp32) {
   cudaEvent_t e0, e1;
   FTLM_CUDA(cudaEventCreate(&e0));
   FTLM_CUDA(cudaEventCreate(&e1));
-  // best of 3 single-launch timings per variant, variants interleaved
+  // best of several single-launch timings per variant, variants interleaved: of 3
+  // after a warm run, or of 2 for the stencil sweeps, whose times repeat to 1% (a
+  // few steps of 2 vectors cost less than 20 launches)
   const bool wide = c.split_wide;
   const StnSweep one{{&c, nullptr}, {in, nullptr}, {out, nullptr}, 1};
   auto run = [&](int v) {
@@ -1218,9 +1220,9 @@ int seg_variant(Ctx& c, const void* in, void* out, int nv, bool fp32) {
   float best_ms[kSegVariants];
   for (int v = 0; v < kSegVariants; ++v) {
     best_ms[v] = 1e30f;
-    run(v);  // warm
+    if (!wide) run(v);  // warm
   }
-  for (int rep = 0; rep < 3; ++rep)
+  for (int rep = 0; rep < (wide ? 2 : 3); ++rep)
     for (int v = 0; v < kSegVariants; ++v) {
       FTLM_CUDA(cudaEventRecord(e0, c.stream));
       run(v);
@@ -1236,7 +1238,7 @@ int seg_variant(Ctx& c, const void* in, void* out, int nv, bool fp32) {
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   c.prof.tune_runs += 1;
-  c.prof.kernel_launches += 4 * kSegVariants;
+  c.prof.kernel_launches += (wide ? 2 : 4) * kSegVariants;
   hv_tuned_store(c, key, best);
   return best;
 }
