@@ -1,8 +1,8 @@
 // Implicit QL with shifts on a symmetric tridiagonal matrix, tracking only
 // the first row of the eigenvector matrix (Golub-Welsch: the FTLM weights are
-// the squared first components), then an ascending insertion sort. One
-// thread per matrix. Shared by the engine's batched Ritz stage (lanczos.cu)
-// and the allocation-free entry point (noalloc.cu).
+// the squared first components), then an ascending insertion sort. A warp per
+// matrix in the engine's batched Ritz stage (lanczos.cu), a thread per matrix in
+// the allocation-free entry point (noalloc.cu).
 #pragma once
 
 namespace ftlm {
@@ -25,12 +25,15 @@ __device__ __forceinline__ void ql_norm(double f, double g, double& rr, double& 
 // d[0..n): diagonal, e[0..n-1): off-diagonal (e[n-1] = 0), z: first row of
 // the eigenvector matrix (1, 0, ..., 0 on entry). A is any indexable view of
 // doubles. Returns false when an eigenvalue needed more than 200 iterations.
-// WARP: the whole warp runs it on the same arrays (its lanes store equal values)
-// and looks for the next negligible off-diagonal 32 at a time.
+// WARP: called by all 32 lanes with the same arrays. The lanes look for the next
+// negligible off-diagonal 32 at a time; the sweeps and the sort, which read what
+// they have just written, run on lane 0 alone, and a __syncwarp stands between
+// every store and the other lanes' next loads (all lanes in step is not promised).
 template <bool WARP = false, typename A>
 __device__ __forceinline__ bool ql_first_row(int n, A d, A z, A e) {
   bool ok = true;
   const double eps = 2.220446049250313e-16;
+  const bool lead = !WARP || (threadIdx.x & 31) == 0;
   for (int l = 0; l < n; ++l) {
     int iter = 0;
     while (true) {
@@ -54,60 +57,69 @@ __device__ __forceinline__ bool ql_first_row(int n, A d, A z, A e) {
         ok = false;
         break;
       }
-      double g = (d[l + 1] - d[l]) / (2.0 * e[l]);
-      double rr = hypot(g, 1.0);
-      double dm = d[m];  // d[i + 1]
-      g = dm - d[l] + e[l] / (g + copysign(rr, g));
-      double s = 1.0, c = 1.0, p = 0.0, zm = z[m];  // zm: z[i + 1]
-      double en = e[m - 1], dn = d[m - 1], zn = z[m - 1];  // row i's, loaded one rotation ahead
-      bool underflow = false;
-      for (int i = m - 1; i >= l; --i) {
-        const double ei = en, di = dn, zi = zn;
-        if (i > l) {
-          en = e[i - 1];
-          dn = d[i - 1];
-          zn = z[i - 1];
+      if constexpr (WARP) __syncwarp();  // every lane has loaded
+      if (lead) {
+        double g = (d[l + 1] - d[l]) / (2.0 * e[l]);
+        double rr = hypot(g, 1.0);
+        double dm = d[m];  // d[i + 1]
+        g = dm - d[l] + e[l] / (g + copysign(rr, g));
+        double s = 1.0, c = 1.0, p = 0.0, zm = z[m];  // zm: z[i + 1]
+        double en = e[m - 1], dn = d[m - 1], zn = z[m - 1];  // row i's, loaded one rotation ahead
+        bool underflow = false;
+        for (int i = m - 1; i >= l; --i) {
+          const double ei = en, di = dn, zi = zn;
+          if (i > l) {
+            en = e[i - 1];
+            dn = d[i - 1];
+            zn = z[i - 1];
+          }
+          const double f = s * ei, b = c * ei;
+          double inv;
+          ql_norm(f, g, rr, inv);
+          e[i + 1] = rr;
+          if (rr == 0.0) {
+            d[i + 1] = dm - p;
+            z[i + 1] = zm;
+            e[m] = 0.0;
+            underflow = true;
+            break;
+          }
+          s = f * inv;
+          c = g * inv;
+          g = dm - p;
+          rr = (di - g) * s + 2.0 * c * b;
+          p = s * rr;
+          d[i + 1] = g + p;
+          g = c * rr - b;
+          z[i + 1] = s * zi + c * zm;
+          zm = c * zi - s * zm;
+          dm = di;
         }
-        const double f = s * ei, b = c * ei;
-        double inv;
-        ql_norm(f, g, rr, inv);
-        e[i + 1] = rr;
-        if (rr == 0.0) {
-          d[i + 1] = dm - p;
-          z[i + 1] = zm;
+        if (!underflow) {
+          d[l] = dm - p;
+          z[l] = zm;
+          e[l] = g;
           e[m] = 0.0;
-          underflow = true;
-          break;
         }
-        s = f * inv;
-        c = g * inv;
-        g = dm - p;
-        rr = (di - g) * s + 2.0 * c * b;
-        p = s * rr;
-        d[i + 1] = g + p;
-        g = c * rr - b;
-        z[i + 1] = s * zi + c * zm;
-        zm = c * zi - s * zm;
-        dm = di;
       }
-      if (underflow) continue;
-      d[l] = dm - p;
-      z[l] = zm;
-      e[l] = g;
-      e[m] = 0.0;
+      if constexpr (WARP) __syncwarp();
     }
   }
-  for (int i = 1; i < n; ++i) {  // insertion sort, ascending
-    const double dk = d[i], zk = z[i];
-    int j = i - 1;
-    while (j >= 0 && d[j] > dk) {
-      d[j + 1] = d[j];
-      z[j + 1] = z[j];
-      --j;
+  if constexpr (WARP) __syncwarp();
+  if (lead) {
+    for (int i = 1; i < n; ++i) {  // insertion sort, ascending
+      const double dk = d[i], zk = z[i];
+      int j = i - 1;
+      while (j >= 0 && d[j] > dk) {
+        d[j + 1] = d[j];
+        z[j + 1] = z[j];
+        --j;
+      }
+      d[j + 1] = dk;
+      z[j + 1] = zk;
     }
-    d[j + 1] = dk;
-    z[j + 1] = zk;
   }
+  if constexpr (WARP) __syncwarp();
   return ok;
 }
 
