@@ -452,8 +452,7 @@ void dense_solve(Ctx& c, const std::vector<int32_t>& dims, const std::vector<int
     P.vecs = c.dense_vecs.as<double2>();
     smem = 0;
   }
-  FTLM_CUDA(cudaFuncSetAttribute(k_dense_eig, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 static_cast<int>(std::max(smem, size_t(48) << 10))));
+  smem_limit(k_dense_eig, kEigMaxSmem);
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(clusters * P.cluster);
   cfg.blockDim = dim3(kEigThreads);

@@ -30,6 +30,16 @@ struct Error : std::runtime_error {
 
 #define FTLM_LAUNCH_CHECK() FTLM_CUDA(cudaGetLastError())
 
+// Lets `kernel` be launched with up to `most` bytes of dynamic shared memory. The
+// limit belongs to the function in the device, for all contexts and host threads,
+// so `most` is the same in every call: a limit set to one launch's size would refuse
+// a larger launch that another thread has just set it for. It does not affect
+// occupancy, which follows from the launch's own size.
+template <typename K>
+inline void smem_limit(K* kernel, size_t most) {
+  FTLM_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(most)));
+}
+
 // Small device buffers of one context, cut from slabs that live as long as the
 // context. A curve on a small lattice creates about 70 buffers and grows them, and
 // a cudaMalloc and a cudaFree of each (which also wait for the device) took 0.1 to

@@ -282,6 +282,7 @@ __global__ void k_start_gather(int64_t dim, int NV, int nva, const double2* __re
 // rows. The three work columns live in shared memory (sm, 3 K doubles) or, where
 // that does not hold them, in the output rows and escr.
 constexpr int kRitzWarps = 4;  // vectors per CTA
+constexpr size_t kRitzMaxSmem = 200 * 1024;
 
 __device__ void tridiag_vector(int r, int lane, int nvmax, int ld, int K, const double* __restrict__ alpha,
                                const double* __restrict__ beta, const int32_t* __restrict__ steps,
@@ -475,10 +476,8 @@ void ritz_stage_many(Ctx& c, std::vector<RitzJob>& jobs) {
   c.ritz_meta.ensure(sizeof(RitzJobDev) * nj);
   FTLM_CUDA(cudaMemcpyAsync(c.ritz_meta.p, dj.data(), sizeof(RitzJobDev) * nj, cudaMemcpyHostToDevice, c.stream));
   const size_t tsmem = sizeof(double) * 3 * kRitzWarps * static_cast<size_t>(kmax);
-  const int use_smem = tsmem <= 200 * 1024;
-  if (use_smem && tsmem > 48 * 1024)
-    FTLM_CUDA(cudaFuncSetAttribute(k_tridiag_many, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   static_cast<int>(tsmem)));
+  const int use_smem = tsmem <= kRitzMaxSmem;
+  if (use_smem && tsmem > 48 * 1024) smem_limit(k_tridiag_many, kRitzMaxSmem);
   k_tridiag_many<<<ctas, 32 * kRitzWarps, use_smem ? tsmem : 0, c.stream>>>(
       static_cast<int>(nj), c.ritz_meta.as<RitzJobDev>(), use_smem ? kmax : 0);
   k_compact_many<<<static_cast<int>(nj), 256, sizeof(int) * (rmax + 1), c.stream>>>(c.ritz_meta.as<RitzJobDev>());

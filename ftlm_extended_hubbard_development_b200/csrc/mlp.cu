@@ -613,7 +613,7 @@ bool train_net(const ftlm_mlp* net, int64_t n, TrainNet& N) {
 template <int R>
 void launch_train_rows(ftlm_mlp* m, const TrainNet& N, const int32_t* idx, float inv_count) {
   const size_t smem = train_smem(N, R);
-  FTLM_CUDA(cudaFuncSetAttribute(k_train_rows<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+  smem_limit(k_train_rows<R>, kTrSmem);
   FTLM_CUDA(cudaFuncSetAttribute(k_train_rows<R>, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
   k_train_rows<R><<<(N.n + R - 1) / R, kTrThreads, smem, m->stream>>>(
       N, m->params.as<float>(), idx, m->data_x.as<float>(), m->data_t.as<float>(), m->data_m.as<float>(), inv_count,
@@ -631,7 +631,7 @@ void train_step(ftlm_mlp* m, const TrainNet& N, const int32_t* idx, float count,
   for (int l = 0; l < N.nl; ++l)
     tiles += ((N.fo[l] + kTpTile - 1) / kTpTile) * ((N.fi[l] + kTpTile - 1) / kTpTile);
   constexpr size_t smem = sizeof(float) * kTpStages * kTpRows * 2 * kTpTile;
-  FTLM_CUDA(cudaFuncSetAttribute(k_train_params, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+  smem_limit(k_train_params, smem);
   FTLM_CUDA(cudaFuncSetAttribute(k_train_params, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
   k_train_params<<<tiles + 1, kTpThreads, smem, m->stream>>>(
       N, A, idx, m->data_x.as<float>(), m->act.as<float>(), m->dact.as<float>(), m->params.as<float>(),

@@ -215,7 +215,7 @@ template <typename T, int NT, int RPT>
 void launch_small(Ctx& c, const SmallArgs& A, cudaStream_t st) {
   const size_t smem = sizeof(double2) * 16 * A.nsite + static_cast<size_t>(2) * A.cap * sizeof(typename CT<T>::C);
   auto kern = k_lanczos_small<T, NT, RPT>;
-  FTLM_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+  smem_limit(kern, sizeof(double2) * 16 * 64 + static_cast<size_t>(2) * kSmallMaxDim * sizeof(typename CT<T>::C));
   int per_sm = 0;
   FTLM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, NT, smem));
   if (per_sm < 1) throw Error(FTLM_ERR_CAPACITY, "small-block Lanczos does not fit on an SM");
