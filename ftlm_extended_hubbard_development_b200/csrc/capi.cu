@@ -474,13 +474,11 @@ int ftlm_block_apply(ftlm_ctx* ctx, int32_t mx, int32_t my, int32_t nvec, const 
     // Host [dim][nvec] FP64 complex to [dim][NV] of the working precision and the
     // sweeps' row order, and back. The copies are the caller's own arrays and the
     // GPU converts; what is as it is (FP64, no padding, block order) needs no
-    // conversion, and a few KB are converted on the host at some 4 ns an element,
-    // where two more launches would take longer (8 us). 4x4 (3,4), 16 vectors, 16 MB
-    // each way: 7.1 -> 5.5 ms, of which 2 are copies and the rest page faults of
-    // the caller's fresh arrays.
+    // conversion, and few elements are converted on the host, where two more
+    // launches would take longer (host_convert).
     const int64_t elems = D * nvec;
     const bool as_is = !fp32 && NV == nvec && !reorder;
-    const bool on_host = !as_is && !reorder && elems < ftlm::kHostConvert;
+    const bool on_host = !as_is && !reorder && elems < ftlm::host_convert(fp32);
     const size_t raw = sizeof(double) * 2 * static_cast<size_t>(elems);
     std::vector<char> h;
     if (as_is) {

@@ -466,7 +466,12 @@ inline int sweep_width(int nvec, bool fp32) { return fp32 ? (nvec + 1) / 2 * 2 :
 void vectors_from_host(Ctx& c, int nvec, int NV, bool fp32, const double* in, void* vec);
 void vectors_to_host(Ctx& c, int nvec, int NV, bool fp32, const void* vec, double* out);
 constexpr int64_t kConvertChunk = int64_t(1) << 24;
-constexpr int64_t kHostConvert = 2048;  // elements below which the host converts
+// Elements below which the host converts. Whole calls, host against device (us):
+// mixed precision, 3136 elements 52 / 62, 6272 70 / 76, 14112 114 / 127, 16144 130 / 128,
+// 20180 169 / 147, 32288 218 / 200; FP64 with padding (3, 5, 7 ... vectors; else
+// nothing is converted), 198 elements 37 / 42, 2744 55 / 57, 4256 68 / 71, 5292 77 / 74,
+// 8820 113 / 87, 20180 216 / 147.
+inline int64_t host_convert(bool fp32) { return fp32 ? 16000 : 5000; }
 int hv_split_max_grid(const Ctx& c);
 // x_D[p(q)] = conj(f_q) x[q];  y[q] += f_q y_D[p(q)].
 void flip_scatter(Ctx& c, const void* x, void* xd, int nv, bool fp32);
