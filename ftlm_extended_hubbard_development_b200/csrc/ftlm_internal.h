@@ -444,6 +444,9 @@ void hv_tuned_store(Ctx& c, uint64_t key, int var);
 // the two flipped-order arrays for sweeps of nv vectors; false when they do
 // not fit in device memory.
 bool split_prepare(Ctx& c, int nv, bool fp32);
+// Whether the prepared sector's split sweeps run on the class stencils: known
+// before anything is built.
+bool split_stencils(const Ctx& c);
 // The prepared sweeps' row order for another number of vectors.
 void split_order(Ctx& c, int nv, bool fp32);
 // y = M x for x given in both row orders: out (this block's order, diagonal

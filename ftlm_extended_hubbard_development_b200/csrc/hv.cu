@@ -803,25 +803,23 @@ int hv_select_source(Ctx& c, int nv, bool fp32) {
   c.split_active = false;
   const int64_t D = c.blk.dim;
   int mode = c.hv_mode;
-  bool one_chunk = false;
   if (mode < 0) {
     // The split-spin sweeps from 2^15 rows, at every width: on the stencils they
     // take 2 FP32 vectors of 4x4 (6,6) in 0.28 ms per H*V, the hop list's row
     // kernel in 1.56 (and the list takes 5.8 ms to build); without the stencils
-    // (more than 65536 down words) one-chunk rows stay on the hop list.
-    one_chunk = nv == (fp32 ? 2 : 1);
+    // (more than 65536 down words) one-chunk rows stay on the hop list, and
+    // nothing of the sweeps is built.
+    const bool one_chunk = nv == (fp32 ? 2 : 1);
     // Wide FP64 sweeps gain from 12288 rows (40 steps, block set up included:
     // 13805 rows 128 vectors 7.0 -> 6.2 ms, 32 vectors 3.4 -> 3.2; 19600 rows 11.9 ->
     // 7.3 and 4.0 -> 3.5); narrow and FP32 ones do not (5 vectors 2.3 -> 2.4).
-    if (D >= kSplitMinDim || (D >= kSplitMinDimFp64 && !fp32 && nv >= 32)) mode = kSrcSplit;
+    if (D >= kSplitMinDim || (D >= kSplitMinDimFp64 && !fp32 && nv >= 32))
+      mode = one_chunk && !split_stencils(c) ? kSrcList : kSrcSplit;
     else if (D >= (1 << 14) && nv <= (fp32 ? 32 : 16)) mode = kSrcList;
     else mode = kSrcFly;
   }
   if (mode == kSrcList && !hoplist_build(c)) mode = c.hv_mode < 0 && D >= kSplitMinDim ? kSrcSplit : kSrcFly;
-  if (mode == kSrcSplit) {
-    if (!split_prepare(c, nv, fp32)) mode = kSrcFly;
-    else if (one_chunk && !c.split_wide && hoplist_build(c)) mode = kSrcList;
-  }
+  if (mode == kSrcSplit && !split_prepare(c, nv, fp32)) mode = kSrcFly;
   c.hl_active = mode == kSrcList;
   c.split_active = mode == kSrcSplit;
   return mode;

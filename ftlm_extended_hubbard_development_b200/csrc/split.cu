@@ -1157,6 +1157,11 @@ void split_order(Ctx& c, int nv, bool fp32) {
   c.flip_gen = c.sec_gen;
 }
 
+bool split_stencils(const Ctx& c) {
+  StnRatios R;
+  return c.split_stencil && std::max(c.sec.c_up, c.sec.c_dn) <= kStencilMaxRows && stn_ratios(c.geom.n, R);
+}
+
 bool split_prepare(Ctx& c, int nv, bool fp32) {
   const int64_t D = c.blk.dim;
   if (D <= 0) return false;
@@ -1168,8 +1173,7 @@ bool split_prepare(Ctx& c, int nv, bool fp32) {
   // every lattice takes, as many as there are
   int pow2 = fp32 ? 2 : 1;
   while (pow2 < nv) pow2 <<= 1;
-  const bool likely = c.split_stencil && std::max(c.sec.c_up, c.sec.c_dn) <= kStencilMaxRows;
-  const size_t vec = static_cast<size_t>(D) * (likely ? nv : pow2) * esize;
+  const size_t vec = static_cast<size_t>(D) * (split_stencils(c) ? nv : pow2) * esize;
   const bool two = c.sec.n_up != c.sec.n_dn;
   const size_t need = 2 * vec + (sizeof(uint64_t) + (two ? 2 : 1) * sizeof(uint32_t) + esize / 2) * D;
   const size_t have = c.vec_xd.cap + c.vec_yd.cap + c.flip_map.cap + c.stn_pos.cap + c.stn_diag.cap +

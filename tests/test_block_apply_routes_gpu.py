@@ -1,5 +1,6 @@
 """Which launches a block_apply call makes: few elements are converted on the host,
-many on the GPU, with equal results (the conversions round and order the same)."""
+many on the GPU, with equal results (the conversions round and order the same); one
+vector without stencils goes to the hop list and builds nothing of the split sweeps."""
 import numpy as np
 import pytest
 
@@ -45,3 +46,22 @@ def test_conversions(lx, ly, nu, nd, nvec, precision, launches):
             u = 2.0 ** -24 if precision == E.PREC_MIXED else 2.0 ** -53
             big = 60 * u * 8.0 * np.abs(x).max() * 8 * 16
             assert np.abs(one - y[:, v:v + width]).max() <= big
+
+
+@pytest.mark.parametrize("precision", [E.PREC_FP64, E.PREC_MIXED])
+def test_one_vector_without_stencils_builds_the_hop_list_only(precision, monkeypatch):
+    """4x4 (3,4), 63,700 rows: as many launches from a new engine as with the list forced
+    (the sweeps' tables of sector (4,3), flip map and order take about 30 more)."""
+    monkeypatch.setenv("FTLM_SPLIT_OP", "fly")
+    seen = []
+    for mode in ("", "list"):
+        if mode:
+            monkeypatch.setenv("FTLM_HV_MODE", mode)
+        with _engine(4, 4, precision) as eng:
+            dim = int(eng.sector_prepare(3, 4).block_dims[1])
+            x = np.random.default_rng(3).standard_normal((dim, 1)) + 0j
+            y, n = _call(eng, x)
+            seen.append((y, n, eng.profile()["hv_source"]))
+    assert [s[2] for s in seen] == [1, 1]
+    assert seen[0][1] == seen[1][1]
+    assert np.array_equal(seen[0][0], seen[1][0])
