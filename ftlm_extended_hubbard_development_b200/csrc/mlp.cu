@@ -618,6 +618,7 @@ void launch_train_rows(ftlm_mlp* m, const TrainNet& N, const int32_t* idx, float
   k_train_rows<R><<<(N.n + R - 1) / R, kTrThreads, smem, m->stream>>>(
       N, m->params.as<float>(), idx, m->data_x.as<float>(), m->data_t.as<float>(), m->data_m.as<float>(), inv_count,
       m->act.as<float>(), m->dact.as<float>(), m->red.as<float>());
+  FTLM_LAUNCH_CHECK();  // before the next attribute call, which clears a refused launch's error
 }
 
 void train_step(ftlm_mlp* m, const TrainNet& N, const int32_t* idx, float count, const Adam& A, float* loss) {
