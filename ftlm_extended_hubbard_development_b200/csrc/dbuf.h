@@ -47,9 +47,14 @@ struct Arena {
   void* take(size_t bytes) {
     bytes = (bytes + 255) / 256 * 256;
     if (used + bytes > size) {
-      const size_t next = std::max(bytes, std::min(kLast, std::max(first, held < (size_t(1) << 20) ? held : 4 * size)));
+      size_t next = std::max(bytes, std::min(kLast, std::max(first, held < (size_t(1) << 20) ? held : 4 * size)));
       void* p = nullptr;
-      FTLM_CUDA(cudaMalloc(&p, next));
+      if (next > bytes && cudaMalloc(&p, next) != cudaSuccess) {  // near full memory: what is asked, no more
+        cudaGetLastError();
+        p = nullptr;
+        next = bytes;
+      }
+      if (!p) FTLM_CUDA(cudaMalloc(&p, next));
       slabs.push_back(p);
       size = next;
       held += next;

@@ -27,3 +27,7 @@ def test_growing_in_small_steps_holds_a_bounded_amount(exe, how):
     are at most 2 (3) times the largest one, 32 MB, and slabs round up to 64 MB: below
     3 slabs and the buffer's own last allocation with its predecessor (2 x 60 MB)."""
     assert _run(exe, "grow", *how) <= (3 * 64 + 2 * 60) << 20
+
+
+def test_a_small_request_does_not_need_a_whole_slab(exe):
+    assert _run(exe, "full") == 1
