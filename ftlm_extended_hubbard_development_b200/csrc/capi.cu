@@ -463,14 +463,22 @@ int ftlm_block_apply(ftlm_ctx* ctx, int32_t mx, int32_t my, int32_t nvec, const 
     ftlm::block_prepare(c, mx, my);
     const int64_t D = c.blk.dim;
     if (D == 0) return;
-    ftlm::HvSourceGuard guard{c};
-    c.prof.hv_source = ftlm::hv_select_source(c, ftlm::sweep_width(nvec, fp32), fp32);
-    const bool reorder = ftlm::sweep_pos(c) != nullptr;
-    if (reorder) NV = ftlm::sweep_width(nvec, fp32);
     const size_t esize = fp32 ? 8 : 16;
-    const size_t bytes = static_cast<size_t>(D) * NV * esize;
-    c.vec_a.ensure(bytes + ftlm::kSweepPad);
-    c.vec_h.ensure(bytes);
+    size_t bytes = 0;
+    auto vectors = [&](int width) {
+      bytes = static_cast<size_t>(D) * width * esize;
+      c.vec_a.ensure(bytes + ftlm::kSweepPad);
+      c.vec_h.ensure(bytes);
+    };
+    // the vectors before the operator, which takes its own arrays only from what
+    // they leave; at the width of the stencil sweeps where those may be chosen
+    const int narrow = ftlm::sweep_width(nvec, fp32);
+    vectors(D >= ftlm::kSplitMinDimFp64 && ftlm::split_stencils(c) ? narrow : NV);
+    ftlm::HvSourceGuard guard{c};
+    c.prof.hv_source = ftlm::hv_select_source(c, narrow, fp32);
+    const bool reorder = ftlm::sweep_pos(c) != nullptr;
+    if (reorder) NV = narrow;
+    vectors(NV);
     // Host [dim][nvec] FP64 complex to [dim][NV] of the working precision and the
     // sweeps' row order, and back. The copies are the caller's own arrays and the
     // GPU converts; what is as it is (FP64, no padding, block order) needs no

@@ -1,5 +1,6 @@
 """Which launches a block_apply call makes: few elements are converted on the host,
-many on the GPU, with equal results (the conversions round and order the same); one
+many on the GPU, with equal results (the conversions round and order the same); near
+full memory the operator is chosen by what the vectors leave; one
 vector without stencils goes to the hop list and builds nothing of the split sweeps."""
 import numpy as np
 import pytest
@@ -65,3 +66,31 @@ def test_one_vector_without_stencils_builds_the_hop_list_only(precision, monkeyp
     assert [s[2] for s in seen] == [1, 1]
     assert seen[0][1] == seen[1][1]
     assert np.array_equal(seen[0][0], seen[1][0])
+
+
+def test_little_memory_falls_back():
+    """4x4 (8,8), 8 FP64 vectors, 1.33 GB an array: with 5.35 GB free the two vectors fit, but not
+    the split sweeps' two arrays, maps and 2 GiB of headroom beside them: the on-the-fly
+    kernel runs, and its H*V is that of the sweeps (60 hops of |x| <= 1 to FP64 rounding)."""
+    import torch
+    free = torch.cuda.mem_get_info()[0]
+    if free < 20 << 30:
+        pytest.skip("needs 20 GB of device memory")
+    out = []
+    for leave in (None, 5_350_000_000):
+        with _engine(4, 4, E.PREC_FP64) as eng:
+            dim = int(eng.sector_prepare(8, 8).block_dims[1])
+            x = np.cos(np.arange(dim * 8, dtype=np.float64).reshape(dim, 8) * 0.37) + 0j
+            hold = []
+            if leave:
+                fill = torch.cuda.mem_get_info()[0] - leave
+                while fill > 0:  # in pieces, so that no single one is refused
+                    n = min(fill, 8 << 30)
+                    hold.append(torch.empty(n, dtype=torch.uint8, device="cuda"))
+                    fill -= n
+            y = eng.block_apply(1, 0, x)
+            out.append((y[::97].copy(), eng.profile()["hv_source"]))
+            del hold
+            torch.cuda.empty_cache()
+    assert out[0][1] == 2 and out[1][1] == 0
+    assert np.abs(out[0][0] - out[1][0]).max() <= 60 * 2.0 ** -53 * 16 * 100
