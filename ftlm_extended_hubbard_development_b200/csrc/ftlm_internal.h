@@ -361,10 +361,10 @@ constexpr size_t kSweepPad = 2048;
 inline int sweep_width(int nvec, bool fp32) { return fp32 ? (nvec + 1) / 2 * 2 : nvec; }
 // Host vectors ([dim][nvec] complex FP64, block order) to [dim][NV] of the working
 // precision in the operator's row order, and back, kConvertChunk elements at a
-// time (256 MB on the device, whatever the block).
+// time (256 MB on the device, whatever the block; less where that does not fit).
 void vectors_from_host(Ctx& c, int nvec, int NV, bool fp32, const double* in, void* vec);
 void vectors_to_host(Ctx& c, int nvec, int NV, bool fp32, const void* vec, double* out);
-constexpr int64_t kConvertChunk = int64_t(1) << 24;
+constexpr int64_t kConvertChunk = int64_t(1) << 24, kConvertLeast = int64_t(1) << 16;
 // Elements below which the host converts. Whole calls, host against device (us):
 // mixed precision, 3136 elements 52 / 62, 6272 70 / 76, 14112 114 / 127, 16144 130 / 128,
 // 20180 169 / 147, 32288 218 / 200; FP64 with padding (3, 5, 7 ... vectors; else

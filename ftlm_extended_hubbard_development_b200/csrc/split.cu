@@ -1302,8 +1302,18 @@ __global__ void k_vectors_out(int64_t row0, int64_t rows, int nvec, int NV, cons
 // f(first row, rows) for the chunks of a block.
 template <typename F>
 void convert_chunks(Ctx& c, int nvec, F&& f) {
-  const int64_t D = c.blk.dim, step = std::max<int64_t>(1, kConvertChunk / nvec);
-  c.host_start.ensure(sizeof(double2) * static_cast<size_t>(std::min(D, step)) * nvec);
+  const int64_t D = c.blk.dim;
+  int64_t step = std::min(D, std::max<int64_t>(1, kConvertChunk / nvec));
+  while (true) {
+    try {
+      c.host_start.ensure(sizeof(double2) * static_cast<size_t>(step) * nvec);
+      break;
+    } catch (const Error&) {  // beside vectors that fill the memory: smaller chunks
+      if (step * nvec <= kConvertLeast) throw;
+      cudaGetLastError();
+      step = (step + 1) / 2;
+    }
+  }
   for (int64_t r = 0; r < D; r += step) f(r, std::min(step, D - r));
 }
 

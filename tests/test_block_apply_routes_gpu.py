@@ -68,6 +68,17 @@ def test_one_vector_without_stencils_builds_the_hop_list_only(precision, monkeyp
     assert np.array_equal(seen[0][0], seen[1][0])
 
 
+def _leave_free(bytes_free):
+    """Holds device memory so that `bytes_free` are left."""
+    import torch
+    hold, fill = [], torch.cuda.mem_get_info()[0] - bytes_free
+    while fill > 0:  # in pieces, so that no single one is refused
+        n = min(fill, 8 << 30)
+        hold.append(torch.empty(n, dtype=torch.uint8, device="cuda"))
+        fill -= n
+    return hold
+
+
 def test_little_memory_falls_back():
     """4x4 (8,8), 8 FP64 vectors, 1.33 GB an array: with 5.35 GB free the two vectors fit, but not
     the split sweeps' two arrays, maps and 2 GiB of headroom beside them: the on-the-fly
@@ -81,16 +92,29 @@ def test_little_memory_falls_back():
         with _engine(4, 4, E.PREC_FP64) as eng:
             dim = int(eng.sector_prepare(8, 8).block_dims[1])
             x = np.cos(np.arange(dim * 8, dtype=np.float64).reshape(dim, 8) * 0.37) + 0j
-            hold = []
-            if leave:
-                fill = torch.cuda.mem_get_info()[0] - leave
-                while fill > 0:  # in pieces, so that no single one is refused
-                    n = min(fill, 8 << 30)
-                    hold.append(torch.empty(n, dtype=torch.uint8, device="cuda"))
-                    fill -= n
+            hold = _leave_free(leave) if leave else []
             y = eng.block_apply(1, 0, x)
             out.append((y[::97].copy(), eng.profile()["hv_source"]))
             del hold
             torch.cuda.empty_cache()
     assert out[0][1] == 2 and out[1][1] == 0
     assert np.abs(out[0][0] - out[1][0]).max() <= 60 * 2.0 ** -53 * 16 * 100
+
+
+def test_less_memory_than_a_conversion_chunk(monkeypatch):
+    """4x4 (8,8), 8 FP32 vectors, 0.66 GB an array: with the two vectors, the block's tables
+    (0.15 GB) and 0.15 GB more there is no room for the 256 MB of a conversion chunk."""
+    import torch
+    monkeypatch.setenv("FTLM_HV_MODE", "fly")
+    if torch.cuda.mem_get_info()[0] < 20 << 30:
+        pytest.skip("needs 20 GB of device memory")
+    out = []
+    for short in (False, True):
+        with _engine(4, 4, E.PREC_MIXED) as eng:
+            dim = int(eng.sector_prepare(8, 8).block_dims[1])
+            x = np.cos(np.arange(dim * 8, dtype=np.float64).reshape(dim, 8) * 0.37) + 0j
+            hold = _leave_free(2 * dim * 8 * 8 + 300_000_000) if short else []
+            out.append(eng.block_apply(1, 0, x)[::97].copy())
+            del hold
+            torch.cuda.empty_cache()
+    assert np.array_equal(out[0], out[1])
