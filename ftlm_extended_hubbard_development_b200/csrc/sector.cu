@@ -13,6 +13,7 @@
 #include <cstring>
 
 #include "ftlm_internal.h"
+#include "strided.h"
 
 namespace ftlm {
 
@@ -371,13 +372,11 @@ __global__ void k_debug_relations(int64_t c_up, int64_t c_dn, const __grid_const
 template <typename W>
 W* wptr(const DBuf& b) { return b.as<W>(); }
 
-// Values of a scan over ncls classes of c_dn words at the class starts, in one
-// strided copy ([ncls + 1], the last one left to the caller).
+// Values of a scan over ncls classes of c_dn words at the class starts ([ncls + 1],
+// the last one left to the caller).
 std::vector<int64_t> class_bases(const int64_t* scan, int ncls, int64_t c_dn, cudaStream_t st) {
   std::vector<int64_t> base(ncls + 1, 0);
-  FTLM_CUDA(cudaMemcpy2DAsync(base.data(), sizeof(int64_t), scan, sizeof(int64_t) * c_dn, sizeof(int64_t), ncls,
-                              cudaMemcpyDeviceToHost, st));
-  FTLM_CUDA(cudaStreamSynchronize(st));
+  copy_strided(base.data(), scan, c_dn, ncls, st);
   return base;
 }
 
