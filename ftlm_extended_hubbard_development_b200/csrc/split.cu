@@ -384,8 +384,60 @@ __device__ __forceinline__ V* stn_at(V* p, uint32_t a, uint32_t rowb) {
   return reinterpret_cast<V*>(reinterpret_cast<B*>(p) + static_cast<uint64_t>(a) * rowb);
 }
 
-// N hops of a row (entries e): all gathers issued before the first FMA.
-template <typename T, int LPL, int N, bool C0>
+// Pairs of FP32 numbers in one register pair.
+__device__ __forceinline__ uint64_t pack2(float a, float b) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ float2 unpack2(uint64_t v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+// At most four hops, summed on their own, then added: acc += sum_u c[u] x[u].
+template <int LPL>
+__device__ __forceinline__ void stn_four(int n, const float2* c, const float4 (*x)[LPL], float4 (&acc)[LPL]) {
+#pragma unroll
+  for (int l = 0; l < LPL; ++l) {
+    // Re c (x.re, x.im) and Im c (x.re, x.im) of both vectors of a chunk: two
+    // multiply-adds a hop and vector, in pairs, where the complex product takes four
+    uint64_t r0 = 0, i0 = 0, r1 = 0, i1 = 0;
+#pragma unroll
+    for (int u = 0; u < n; ++u) {
+      const uint64_t cr = pack2(c[u].x, c[u].x), ci = pack2(c[u].y, c[u].y);
+      const uint64_t x0 = pack2(x[u][l].x, x[u][l].y), x1 = pack2(x[u][l].z, x[u][l].w);
+      r0 = fma2(cr, x0, r0);
+      i0 = fma2(ci, x0, i0);
+      r1 = fma2(cr, x1, r1);
+      i1 = fma2(ci, x1, i1);
+    }
+    const float2 a0 = unpack2(r0), b0 = unpack2(i0), a1 = unpack2(r1), b1 = unpack2(i1);
+    acc[l].x += a0.x - b0.y;
+    acc[l].y += a0.y + b0.x;
+    acc[l].z += a1.x - b1.y;
+    acc[l].w += a1.y + b1.x;
+  }
+}
+template <int LPL>
+__device__ __forceinline__ void stn_four(int n, const double2* c, const double2 (*x)[LPL], double2 (&acc)[LPL]) {
+#pragma unroll
+  for (int l = 0; l < LPL; ++l) {
+    double2 t = make_double2(0.0, 0.0);
+#pragma unroll
+    for (int u = 0; u < n; ++u) cfma<double>(t, c[u].x, c[u].y, x[u][l]);
+    vadd(acc[l], t);
+  }
+}
+
+// N hops of a row (entries e): all gathers issued before the first FMA. FOURS: summed
+// four at a time, else in a chain.
+template <typename T, int LPL, int N, bool C0, bool FOURS>
 __device__ __forceinline__ void stn_hops(const uint32_t* e, const StnJobs<T>& P, const typename CoefT<T>::C* coef,
                                          const typename CT<T>::V* __restrict__ xs, uint32_t rowb,
                                          typename CT<T>::V (&acc)[LPL]) {
@@ -401,14 +453,19 @@ __device__ __forceinline__ void stn_hops(const uint32_t* e, const StnJobs<T>& P,
     if constexpr (C0) c[u] = P.c0[e[u] >> 16];
     else c[u] = __ldg(coef + (e[u] >> 16));
   }
+  if constexpr (FOURS) {
+    stn_four<LPL>(N < 4 ? N : 4, c, x, acc);
+    if constexpr (N > 4) stn_four<LPL>(N - 4, c + 4, x + 4, acc);
+  } else {
 #pragma unroll
-  for (int u = 0; u < N; ++u)
+    for (int u = 0; u < N; ++u)
 #pragma unroll
-    for (int l = 0; l < LPL; ++l) cfma<T>(acc[l], c[u].x, c[u].y, x[u][l]);
+      for (int l = 0; l < LPL; ++l) cfma<T>(acc[l], c[u].x, c[u].y, x[u][l]);
+  }
 }
 
 // All hops of a row, U (4 or 8) at a time, then the remainder.
-template <typename T, int LPL, int U, bool C0>
+template <typename T, int LPL, int U, bool C0, bool FOURS>
 __device__ __forceinline__ void stn_row(const uint4* q, int left, const StnJobs<T>& P,
                                         const typename CoefT<T>::C* coef, const typename CT<T>::V* __restrict__ xs,
                                         uint32_t rowb, typename CT<T>::V (&acc)[LPL]) {
@@ -419,20 +476,20 @@ __device__ __forceinline__ void stn_row(const uint4* q, int left, const StnJobs<
       const uint32_t e[8] = {p.x, p.y, p.z, p.w, p2.x, p2.y, p2.z, p2.w};
       q += 2;
       p = __ldg(q);
-      stn_hops<T, LPL, 8, C0>(e, P, coef, xs, rowb, acc);
+      stn_hops<T, LPL, 8, C0, FOURS>(e, P, coef, xs, rowb, acc);
       left -= 8;
     }
   }
   while (left >= 4) {
     const uint32_t e[4] = {p.x, p.y, p.z, p.w};
     p = __ldg(++q);
-    stn_hops<T, LPL, 4, C0>(e, P, coef, xs, rowb, acc);
+    stn_hops<T, LPL, 4, C0, FOURS>(e, P, coef, xs, rowb, acc);
     left -= 4;
   }
   const uint32_t e[3] = {p.x, p.y, p.z};
-  if (left == 1) stn_hops<T, LPL, 1, C0>(e, P, coef, xs, rowb, acc);
-  else if (left == 2) stn_hops<T, LPL, 2, C0>(e, P, coef, xs, rowb, acc);
-  else if (left == 3) stn_hops<T, LPL, 3, C0>(e, P, coef, xs, rowb, acc);
+  if (left == 1) stn_hops<T, LPL, 1, C0, FOURS>(e, P, coef, xs, rowb, acc);
+  else if (left == 2) stn_hops<T, LPL, 2, C0, FOURS>(e, P, coef, xs, rowb, acc);
+  else if (left == 3) stn_hops<T, LPL, 3, C0, FOURS>(e, P, coef, xs, rowb, acc);
 }
 
 __device__ __forceinline__ void stn_finish(float4& y, const float4& x, float d, double* dot) {
@@ -453,7 +510,7 @@ __device__ __forceinline__ void stn_finish(double2& y, const double2& x, double 
 //
 // A warp takes a panel of a stencil row (32 lanes of LPL 16-byte chunks, 512 LPL
 // contiguous bytes per hop): the row's entries are warp-uniform (one broadcast
-// load per four hops, no shuffles, no divergence, no partial sums to fold). A
+// load per four hops, no shuffles, no divergence, no lanes' sums to fold). A
 // work unit is kStnRows stencil rows, kStnLane apart, of one panel;
 // kStnLane consecutive units cover kStnLane * kStnRows consecutive rows. A CTA
 // takes one unit per warp, consecutive ones, from a shared counter, so at any
@@ -461,6 +518,8 @@ __device__ __forceinline__ void stn_finish(double2& y, const double2& x, double 
 // among the low sites stay within a few hundred rows): a quarter of the
 // gathered sectors hit L1. Lanes past the end of a panel load what follows it
 // (the arrays end in kSweepPad spare bytes) and drop the result.
+//
+// A row's hops are added in fours or in a chain (stn_fours; the times below are the chain's).
 //
 // Bound: waits for gathered lines at 16-24 warps per SM (L1 67% busy with 30%
 // hits, L2 50%; 17-20 TB/s of gathered bytes). Per H*V, both sweeps, against the
@@ -482,7 +541,7 @@ __host__ __device__ __forceinline__ unsigned int stn_chunks(int64_t rows, int pe
 
 constexpr int kStnSlots = 128;  // dot terms of a warp: parts x 32 LPL chunks x vectors per chunk, at most
 
-template <typename T, int LPL, int U, int NT, int MINB>
+template <typename T, int LPL, int U, int NT, int MINB, bool FOURS>
 __global__ void __launch_bounds__(NT, MINB) k_hv_stn(const __grid_constant__ StnJobs<T> P,
                                                      const double* __restrict__ scale, fx128* __restrict__ partial,
                                                      unsigned int* __restrict__ next_item) {
@@ -570,8 +629,8 @@ __global__ void __launch_bounds__(NT, MINB) k_hv_stn(const __grid_constant__ Stn
         V xo[LPL];
 #pragma unroll
         for (int l = 0; l < LPL; ++l) xo[l] = __ldg(stn_at(xs, a, rowb) + l * 32);
-        if (C.c0) stn_row<T, LPL, U, true>(q4, left, P, J.coef, xs, rowb, acc);
-        else stn_row<T, LPL, U, false>(q4, left, P, J.coef, xs, rowb, acc);
+        if (C.c0) stn_row<T, LPL, U, true, FOURS>(q4, left, P, J.coef, xs, rowb, acc);
+        else stn_row<T, LPL, U, false, FOURS>(q4, left, P, J.coef, xs, rowb, acc);
 #pragma unroll
         for (int l = 0; l < LPL; ++l) {
           stn_finish(acc[l], xo[l], d[l], dot[l]);
@@ -753,6 +812,17 @@ void launch_seg(Ctx& c, Ctx& t, int var, const void* in, void* out, int nv, bool
 // units): 1.65, 1.63, 1.80; 4x4 (4,4), 5 FP64 vectors (4 k): 0.109, 0.087, 0.154.
 int stn_rows(int64_t dim, int cpr) { return dim * cpr >= (int64_t(1) << 27) ? 16 : 8; }
 
+// Whether a row's hops are added in fours or in one chain. A chain rounds a growing sum at
+// every hop, fours a quarter as often. The line lies where the error of H*V stays that of
+// the kernels that shared a row among 32 / chunks groups of lanes (8 below 5 chunks) and so
+// added sums as short. Relative to 64 bits, lane groups / chain / fours: 4x4 (3,4), FP32, 8
+// vectors 4.84e-8 / 6.83e-8 / 4.95e-8, 16 5.06 / 6.83 / 4.95, 32 5.67 / 6.83 / 4.95, 64 6.83 / 6.83 /
+// 4.95; FP64, 8 vectors 1.02e-16 / 1.33e-16 / 1.02e-16. Per H*V, chain / fours: 6x3 (5,5) 16 FP32
+// vectors 1.64 / 1.70 ms, 4x4 (4,4) 5 FP64 0.084 / 0.088, 4x4 (6,6) 2 FP32 0.283 / 0.278, 4x4 (5,5)
+// 128 2.32 / 2.5. Narrower sweeps all add in the same order, so a vector's product does
+// not depend on how many others there are.
+bool stn_fours(int nv, bool fp32) { return (fp32 ? nv / 2 : nv) < 32; }
+
 template <typename T>
 StnJob<T> stn_job(Ctx& t, const void* in, void* out, bool with_diag, const StnPanels& pan, int rows) {
   StnJob<T> j;
@@ -778,7 +848,7 @@ struct StnSweep {  // the two sweeps of one H*V: block order (with the diagonal)
   int n;
 };
 
-template <typename T, int LPL, int U, int NT, int MINB>
+template <typename T, int LPL, int U, int NT, int MINB, bool FOURS>
 int launch_stn_t(Ctx& c, const StnSweep& w, int nv, const double* scale, fx128* partial, unsigned int* counter) {
   StnJobs<T> P;
   P.njobs = w.n;
@@ -800,23 +870,23 @@ int launch_stn_t(Ctx& c, const StnSweep& w, int nv, const double* scale, fx128* 
   // the rest of the SM's 228 KB serves as L1, where most of the gather reuse is
   constexpr size_t kSmem = sizeof(fx128) * NT / 32 * kStnSlots + 2048;
   constexpr int kCarve = static_cast<int>((kSmem * MINB * 100 + 228 * 1024 - 1) / (228 * 1024));
-  FTLM_CUDA(cudaFuncSetAttribute(k_hv_stn<T, LPL, U, NT, MINB>, cudaFuncAttributePreferredSharedMemoryCarveout,
+  FTLM_CUDA(cudaFuncSetAttribute(k_hv_stn<T, LPL, U, NT, MINB, FOURS>, cudaFuncAttributePreferredSharedMemoryCarveout,
                                  kCarve));
-  k_hv_stn<T, LPL, U, NT, MINB><<<grid, NT, 0, c.stream>>>(P, scale, partial, counter);
+  k_hv_stn<T, LPL, U, NT, MINB, FOURS><<<grid, NT, 0, c.stream>>>(P, scale, partial, counter);
   return grid;
 }
 
 // Variants: chunks per lane (more amortise the entry load, fewer leave
 // registers for warps), gathers in flight, CTA shape. All sum a row's hops in
 // the same order, and the same dot terms.
-template <typename T>
+template <typename T, bool FOURS>
 int launch_stn_var(Ctx& c, int var, const StnSweep& w, int nv, const double* scale, fx128* partial, unsigned int* nr) {
   switch (var) {
-    case 0: return launch_stn_t<T, 2, 4, 256, 3>(c, w, nv, scale, partial, nr);
-    case 1: return launch_stn_t<T, 2, 8, 256, 2>(c, w, nv, scale, partial, nr);
-    case 2: return launch_stn_t<T, 1, 8, 256, 3>(c, w, nv, scale, partial, nr);
-    case 3: return launch_stn_t<T, 1, 4, 256, 4>(c, w, nv, scale, partial, nr);
-    case 4: return launch_stn_t<T, 2, 8, 256, 3>(c, w, nv, scale, partial, nr);
+    case 0: return launch_stn_t<T, 2, 4, 256, 3, FOURS>(c, w, nv, scale, partial, nr);
+    case 1: return launch_stn_t<T, 2, 8, 256, 2, FOURS>(c, w, nv, scale, partial, nr);
+    case 2: return launch_stn_t<T, 1, 8, 256, 3, FOURS>(c, w, nv, scale, partial, nr);
+    case 3: return launch_stn_t<T, 1, 4, 256, 4, FOURS>(c, w, nv, scale, partial, nr);
+    case 4: return launch_stn_t<T, 2, 8, 256, 3, FOURS>(c, w, nv, scale, partial, nr);
     default: break;
   }
   throw Error(FTLM_ERR_ARG, "bad H*V kernel variant");
@@ -830,8 +900,12 @@ int launch_stn(Ctx& c, int var, const StnSweep& w, int nv, bool fp32, const doub
     nr = c.seg_counter.as<unsigned int>();
     FTLM_CUDA(cudaMemsetAsync(nr, 0, sizeof(unsigned int), c.stream));
   }
-  const int grid = fp32 ? launch_stn_var<float>(c, var, w, nv, scale, partial, nr)
-                        : launch_stn_var<double>(c, var, w, nv, scale, partial, nr);
+  auto run = [&](auto fours) {
+    constexpr bool F = decltype(fours)::value;
+    return fp32 ? launch_stn_var<float, F>(c, var, w, nv, scale, partial, nr)
+                : launch_stn_var<double, F>(c, var, w, nv, scale, partial, nr);
+  };
+  const int grid = stn_fours(nv, fp32) ? run(std::true_type()) : run(std::false_type());
   FTLM_LAUNCH_CHECK();
   return grid;
 }
@@ -1201,7 +1275,8 @@ int seg_variant(Ctx& c, const void* in, void* out, int nv, bool fp32) {
   if (c.hv_forced >= 0 && c.hv_forced < kSegVariants) return c.hv_forced;
   int width = 1;  // the wide sweeps take any number of vectors: one measurement per power of two
   while (width < nv) width <<= 1;
-  const uint64_t key = static_cast<uint64_t>((c.wide ? 1 : 0) | 4 | (c.split_wide ? 8 : 0)) |
+  const bool fours = c.split_wide && stn_fours(nv, fp32);
+  const uint64_t key = static_cast<uint64_t>((c.wide ? 1 : 0) | (fours ? 2 : 0) | 4 | (c.split_wide ? 8 : 0)) |
                        (static_cast<uint64_t>(fp32 ? 1 : 0) << 4) |
                        (static_cast<uint64_t>(width) << 8) |
                        (static_cast<uint64_t>(hv_size_class(c.blk.dim)) << 20) |
