@@ -23,7 +23,8 @@
 // vectors x 80 steps, 288 blocks up to 1764 rows: 82 ms in 32 launches of 256
 // threads on 20-byte CSR entries, one after another (45 of 148 SMs busy),
 // against 27 ms of launches that overlap; 4x2 curve, 32 mixed vectors x 120
-// steps: 24 ms against 8.2.
+// steps: 24 ms against 8.2. With the fours the 3x3 curve's launches take 25 ms: the two
+// halves of a chain no longer wait for each other.
 //
 // Arithmetic is the reference's: w = H v; alpha = Re<v, w>;
 // w -= alpha v + beta_prev v_prev; beta = |w|; stop at beta < 1e-12 or the
@@ -90,6 +91,10 @@ template <typename T, int NT, int RPT>
 __global__ void __launch_bounds__(NT) k_lanczos_small(const __grid_constant__ SmallArgs A) {
   using C = typename CT<T>::C;
   constexpr int NW = NT / 32;
+  // An FP64 row's hops are added four at a time, the fours then to the row: the sums that
+  // round are as short as those of 8 lanes sharing a row. FP32 rows are added in FP64 too and
+  // rounded to FP32 at the end, where one chain does as well.
+  constexpr bool kFours = sizeof(T) == 8;
   extern __shared__ __align__(16) unsigned char small_smem[];
   __shared__ double red[2][32];
   __shared__ double s_ratio[kSmallRatios];
@@ -151,22 +156,29 @@ __global__ void __launch_bounds__(NT) k_lanczos_small(const __grid_constant__ Sm
         const C xi = v[i];
         double ar = 0.0, ai = 0.0;
         int n = len[q];
-        auto add = [&](uint32_t w) {
+        auto add = [&](uint32_t w, double& sr, double& si) {
           const double2 c = coef[(w >> 12) & 0x3FF];
           const double ratio = s_ratio[w >> 22];
           const C x = v[w & 0xFFF];
           const double cr = __dmul_rn(c.x, ratio), ci = __dmul_rn(c.y, ratio);
-          ar += cr * static_cast<double>(x.x) - ci * static_cast<double>(x.y);
-          ai += cr * static_cast<double>(x.y) + ci * static_cast<double>(x.x);
+          sr += cr * static_cast<double>(x.x) - ci * static_cast<double>(x.y);
+          si += cr * static_cast<double>(x.y) + ci * static_cast<double>(x.x);
         };
         for (; n >= 4; n -= 4, e += 4 * static_cast<int64_t>(D)) {
           const uint32_t w0 = __ldg(e), w1 = __ldg(e + D), w2 = __ldg(e + 2 * D), w3 = __ldg(e + 3 * D);
-          add(w0);
-          add(w1);
-          add(w2);
-          add(w3);
+          double sr = 0.0, si = 0.0;
+          double& r4 = kFours ? sr : ar;
+          double& i4 = kFours ? si : ai;
+          add(w0, r4, i4);
+          add(w1, r4, i4);
+          add(w2, r4, i4);
+          add(w3, r4, i4);
+          if constexpr (kFours) {
+            ar += sr;
+            ai += si;
+          }
         }
-        for (; n > 0; --n, e += D) add(__ldg(e));
+        for (; n > 0; --n, e += D) add(__ldg(e), ar, ai);
         ar += dg[q] * static_cast<double>(xi.x);
         ai += dg[q] * static_cast<double>(xi.y);
         h[q] = CT<T>::make(ar, ai);
