@@ -7,18 +7,27 @@
 
 namespace ftlm {
 
-// rr = |(f, g)| and its reciprocal. The squares are used as they are where they
-// neither overflow nor lose bits to underflow: one reciprocal root, where hypot
-// and two divisions were most of a rotation's dependent chain (5 x 80 steps: 2.8 ms
-// with them, 1.0 without and with the warp's search below).
-__device__ __forceinline__ void ql_norm(double f, double g, double& rr, double& inv) {
+// Rotation of (f, g) onto its norm: rr = |(f, g)|, s = f / rr, c = g / rr; rr = 0 for
+// a zero vector. The squares are used as they are where they neither overflow nor
+// lose bits to underflow, and everything comes from one reciprocal root h: a Newton
+// step corrects rr = r2 h by its residual r2 - rr^2, and each quotient q = f h by
+// f - q rr (Markstein's correction), so that all three are rounded about once, as
+// hypot (2 ulp) and two divisions gave them. Without the residuals they are 1 to 2 ulp off
+// and the eigenvalues' root-mean-square error on tridiagonals of 20 to 120 steps is
+// 15% larger. The rotation is most of the sweep's dependent chain (5 x 80 steps: 2.8 ms
+// with hypot and divisions, 2.0 with a root and divisions, 1.1 this way, 1.0 without
+// the residuals).
+__device__ __forceinline__ void ql_rotation(double f, double g, double& rr, double& s, double& c) {
   const double r2 = fma(f, f, g * g);
   if (r2 > 1e-200 && r2 < 1e200) {
-    inv = rsqrt(r2);
-    rr = r2 * inv;
+    const double h = rsqrt(r2), r0 = r2 * h, sf = f * h, cg = g * h;
+    rr = fma(0.5 * h, fma(-r0, r0, r2), r0);
+    s = fma(h, fma(-sf, rr, f), sf);
+    c = fma(h, fma(-cg, rr, g), cg);
   } else {
     rr = hypot(f, g);
-    inv = rr == 0.0 ? 0.0 : 1.0 / rr;
+    s = f / rr;
+    c = g / rr;
   }
 }
 
@@ -74,8 +83,8 @@ __device__ __forceinline__ bool ql_first_row(int n, A d, A z, A e) {
             zn = z[i - 1];
           }
           const double f = s * ei, b = c * ei;
-          double inv;
-          ql_norm(f, g, rr, inv);
+          double sn, cn;
+          ql_rotation(f, g, rr, sn, cn);
           e[i + 1] = rr;
           if (rr == 0.0) {
             d[i + 1] = dm - p;
@@ -84,8 +93,8 @@ __device__ __forceinline__ bool ql_first_row(int n, A d, A z, A e) {
             underflow = true;
             break;
           }
-          s = f * inv;
-          c = g * inv;
+          s = sn;
+          c = cn;
           g = dm - p;
           rr = (di - g) * s + 2.0 * c * b;
           p = s * rr;
