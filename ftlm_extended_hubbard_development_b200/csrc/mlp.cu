@@ -10,6 +10,7 @@
 // layer and direction; both stay in FP32.
 #include <algorithm>
 #include <cmath>
+#include <cstdlib>
 #include <cstring>
 #include <random>
 #include <type_traits>
@@ -38,6 +39,7 @@ struct ftlm_mlp {
   int64_t data_n = 0;
   int64_t batch_cap = 0;
   int64_t adam_t = 0;
+  bool fused_step = true;  // FTLM_TRAIN_STEP=layers: the per-layer kernels at every size
   std::string last_error;
 };
 
@@ -694,6 +696,7 @@ int ftlm_mlp_create(int32_t n_in, int32_t width, int32_t depth, int32_t n_out, u
   net->width = width;
   net->depth = depth;
   net->n_out = n_out;
+  if (const char* ts = std::getenv("FTLM_TRAIN_STEP")) net->fused_step = std::string(ts) != "layers";
   for (int l = 0; l <= depth; ++l) {
     net->fan_in.push_back(l == 0 ? n_in : width);
     net->fan_out.push_back(l == depth ? n_out : width);
@@ -835,7 +838,7 @@ int ftlm_mlp_train(ftlm_mlp* net, const float* x, const float* t, const float* m
     const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
     std::vector<int> batches(static_cast<size_t>(epochs), 0);
     ftlm::TrainNet N;
-    const bool fused = ftlm::train_net(m, B, N);
+    const bool fused = m->fused_step && ftlm::train_net(m, B, N);
     for (int e = 0; e < epochs; ++e) {
       std::shuffle(perm.begin(), perm.end(), rng);
       FTLM_CUDA(cudaStreamSynchronize(m->stream));  // the previous epoch's order is no longer read
