@@ -486,7 +486,7 @@ int ftlm_block_apply(ftlm_ctx* ctx, int32_t mx, int32_t my, int32_t nvec, const 
     // launches would take longer (host_convert).
     const int64_t elems = D * nvec;
     const bool as_is = !fp32 && NV == nvec && !reorder;
-    const bool on_host = !as_is && !reorder && elems < ftlm::host_convert(fp32);
+    const bool on_host = !as_is && !reorder && ftlm::host_convert(D, nvec, NV, fp32);
     const size_t raw = sizeof(double) * 2 * static_cast<size_t>(elems);
     std::vector<char> h;
     if (as_is) {
