@@ -1289,8 +1289,14 @@ int seg_variant(Ctx& c, const void* in, void* out, int nv, bool fp32) {
   FTLM_CUDA(cudaEventCreate(&e1));
   // best of several single-launch timings per variant, variants interleaved: of 3
   // after a warm run, or of 2 for the stencil sweeps, whose times repeat to 1% (a
-  // few steps of 2 vectors cost less than 20 launches)
+  // few steps of 2 vectors cost less than 20 launches). Sums of fours (stn_fours) take
+  // more registers: of their variants 1, with 128 registers, or 2, with one chunk a lane,
+  // was the fastest on every block (us per H*V, variants 0-4: 5x3 (12,5) 2 FP32 vectors 48
+  // 37 35 44 48, 4x3 (5,7) 4 FP64 43 31 32 35 52, 4x4 (12,5) 3 FP32 96 91 85 103 99, 6x3
+  // (14,14) 43 FP32 527 487 564 590 554), and only those two are timed: a single timing
+  // picked variant 3 on the first of them.
   const bool wide = c.split_wide;
+  auto timed = [&](int v) { return !fours || v == 1 || v == 2; };
   const StnSweep one{{&c, nullptr}, {in, nullptr}, {out, nullptr}, 1};
   auto run = [&](int v) {
     if (wide) launch_stn(c, v, one, nv, fp32, nullptr, nullptr);
@@ -1303,6 +1309,7 @@ int seg_variant(Ctx& c, const void* in, void* out, int nv, bool fp32) {
   }
   for (int rep = 0; rep < (wide ? 2 : 3); ++rep)
     for (int v = 0; v < kSegVariants; ++v) {
+      if (!timed(v)) continue;
       FTLM_CUDA(cudaEventRecord(e0, c.stream));
       run(v);
       FTLM_CUDA(cudaEventRecord(e1, c.stream));
@@ -1317,7 +1324,7 @@ int seg_variant(Ctx& c, const void* in, void* out, int nv, bool fp32) {
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   c.prof.tune_runs += 1;
-  c.prof.kernel_launches += (wide ? 2 : 4) * kSegVariants;
+  c.prof.kernel_launches += wide ? 2 * (fours ? 2 : kSegVariants) : 4 * kSegVariants;
   hv_tuned_store(c, key, best);
   return best;
 }
