@@ -26,7 +26,6 @@ namespace {
 constexpr int kEigThreads = 512;
 constexpr int kEigWarps = kEigThreads / 32;
 constexpr int kEigUnroll = 4;
-constexpr int kEigCols = 1;      // columns a warp updates at once (2: within 2%, slower on clusters of 8)
 constexpr int kMaxDense = 7000;
 constexpr size_t kEigMaxSmem = 200 * 1024;  // three complex work vectors per CTA, else in global memory
 
@@ -140,44 +139,27 @@ __device__ void dense_eig(int n, double2* __restrict__ A, double* __restrict__ w
     // pending update of the columns behind, and their products with u
     double2* p = pbuf + static_cast<int64_t>(k & 1) * n;
     const int c0 = k + 1;
-    int g = (c0 / kEigCols) / nwarps * nwarps + gwarp;  // this warp's column groups: g = gwarp (mod nwarps)
-    if (g < c0 / kEigCols) g += nwarps;
-    for (; g * kEigCols < n; g += nwarps) {
-      double2* a[kEigCols];
-      double2 wj[kEigCols], vj[kEigCols], s[kEigCols];
-      bool on[kEigCols];
-#pragma unroll
-      for (int c = 0; c < kEigCols; ++c) {
-        const int cc = g * kEigCols + c;
-        on[c] = cc >= c0 && cc < n;
-        const int j = on[c] ? cc - c0 : 0;
-        a[c] = A + c0 + static_cast<int64_t>(on[c] ? cc : c0) * n;
-        wj[c] = w[j + 1];
-        vj[c] = v[j + 1];
-        s[c] = make_double2(0.0, 0.0);
-      }
+    int j = c0 / nwarps * nwarps + gwarp;  // this warp's columns: j = gwarp (mod nwarps)
+    if (j < c0) j += nwarps;
+    for (; j < n; j += nwarps) {
+      double2* a = A + c0 + static_cast<int64_t>(j) * n;
+      const double2 wj = w[j - c0 + 1], vj = v[j - c0 + 1];
+      double2 s = make_double2(0.0, 0.0);
 #pragma unroll kEigUnroll
       for (int i = lane; i < m; i += 32) {
         const double2 vi = v[i + 1], wi = w[i + 1], ui = u[i];
-#pragma unroll
-        for (int c = 0; c < kEigCols; ++c) {
-          if (!on[c]) continue;
-          double2 b = a[c][i];
-          b.x -= (vi.x * wj[c].x + vi.y * wj[c].y) + (wi.x * vj[c].x + wi.y * vj[c].y);
-          b.y -= (vi.y * wj[c].x - vi.x * wj[c].y) + (wi.y * vj[c].x - wi.x * vj[c].y);
-          a[c][i] = b;
-          s[c].x += b.x * ui.x + b.y * ui.y;
-          s[c].y += b.x * ui.y - b.y * ui.x;
-        }
+        double2 b = a[i];
+        b.x -= (vi.x * wj.x + vi.y * wj.y) + (wi.x * vj.x + wi.y * vj.y);
+        b.y -= (vi.y * wj.x - vi.x * wj.y) + (wi.y * vj.x - wi.x * vj.y);
+        a[i] = b;
+        s.x += b.x * ui.x + b.y * ui.y;
+        s.y += b.x * ui.y - b.y * ui.x;
       }
-#pragma unroll
-      for (int c = 0; c < kEigCols; ++c) {
-        for (int o = 16; o > 0; o >>= 1) {
-          s[c].x += __shfl_xor_sync(0xffffffffu, s[c].x, o);
-          s[c].y += __shfl_xor_sync(0xffffffffu, s[c].y, o);
-        }
-        if (lane == 0 && on[c]) __stcg(p + (g * kEigCols + c - c0), make_double2(tau * s[c].x, tau * s[c].y));
+      for (int o = 16; o > 0; o >>= 1) {
+        s.x += __shfl_xor_sync(0xffffffffu, s.x, o);
+        s.y += __shfl_xor_sync(0xffffffffu, s.y, o);
       }
+      if (lane == 0) __stcg(p + (j - c0), make_double2(tau * s.x, tau * s.y));
     }
     group_sync(cluster);
     // w = p - (tau/2)(u^H p) u; v <- u

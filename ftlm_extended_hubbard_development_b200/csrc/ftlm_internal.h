@@ -197,8 +197,8 @@ struct FlipPhase {
   double re[64], im[64];
 };
 
-// Largest block dimension the small-block Lanczos launch takes (three FP64
-// complex vectors of this length fill 192 KB of shared memory).
+// Largest block dimension the small-block Lanczos launch takes (two FP64 complex
+// vectors of this length, 128 KB, live in shared memory; an entry keeps 12 bits of column).
 constexpr int64_t kSmallMaxDim = 4096;
 
 struct Ctx {

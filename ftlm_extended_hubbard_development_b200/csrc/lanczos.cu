@@ -375,8 +375,6 @@ __global__ void k_collect_steps(const double* __restrict__ st, int NV, int nva, 
   if (v < nva) out[v] = static_cast<int32_t>(st[S_STEPS * NV + v]);
 }
 
-// Algorithmic-byte model count: nonzero-amplitude hops with active
-// targets per block (the h_nz of the H*V roofline).
 int next_pow2(int x) {
   int p = 1;
   while (p < x) p <<= 1;

@@ -355,7 +355,6 @@ struct StnJob {
   const uint4* ent;
   const typename CoefT<T>::C* coef;
   const StnClass* cls;
-  int32_t ncls;
   int32_t units;  // work units (below) of the job
 };
 // A group's stencil row, S_g cpr chunks, is cut into `parts` panels of at most
@@ -511,8 +510,8 @@ __device__ __forceinline__ void stn_finish(double2& y, const double2& x, double 
 // A warp takes a panel of a stencil row (32 lanes of LPL 16-byte chunks, 512 LPL
 // contiguous bytes per hop): the row's entries are warp-uniform (one broadcast
 // load per four hops, no shuffles, no divergence, no lanes' sums to fold). A
-// work unit is kStnRows stencil rows, kStnLane apart, of one panel;
-// kStnLane consecutive units cover kStnLane * kStnRows consecutive rows. A CTA
+// work unit is P.rows stencil rows (stn_rows), kStnLane apart, of one panel;
+// kStnLane consecutive units cover kStnLane * P.rows consecutive rows. A CTA
 // takes one unit per warp, consecutive ones, from a shared counter, so at any
 // moment its warps are on neighbouring rows, which share gather targets (hops
 // among the low sites stay within a few hundred rows): a quarter of the
@@ -785,8 +784,7 @@ void launch_seg_nv(Ctx& c, Ctx& t, int var, const void* in, void* out, int nv, c
   throw Error(FTLM_ERR_ARG, "unsupported vectors per sweep: " + std::to_string(nv));
 }
 
-// next_row: c.seg_sched's counter for this sweep (zeroed here, on the
-// stream) or null for grid-stride rows.
+// Rows come from this sweep's counter (zeroed here, on the stream), or grid-stride.
 void launch_seg(Ctx& c, Ctx& t, int var, const void* in, void* out, int nv, bool fp32, const double* scale,
                 fx128* partial, int grid, bool with_diag, int counter_slot) {
   unsigned long long* nr = nullptr;
@@ -833,7 +831,6 @@ StnJob<T> stn_job(Ctx& t, const void* in, void* out, bool with_diag, const StnPa
   j.ent = t.stn_ent4.as<uint4>();
   j.coef = t.stn_coef.as<typename CoefT<T>::C>();
   j.cls = t.stn_cls.as<StnClass>();
-  j.ncls = static_cast<int32_t>(t.stn_classes.size() / 2);
   int64_t units = 0;
   for (size_t k = 0; k + 1 < t.stn_classes.size(); k += 2)
     units += stn_chunks(t.stn_classes[k + 1], rows) * pan.count(t.stn_classes[k]);
@@ -1078,7 +1075,7 @@ bool stencil_build_t(Ctx& c, Ctx& t) {
   t.stn_crb.ensure(sizeof(int64_t) * (S.nclass + 1));
   FTLM_CUDA(cudaMemcpyAsync(t.stn_crb.p, crb.data(), sizeof(int64_t) * crb.size(), cudaMemcpyHostToDevice, c.stream));
   t.stn_cnt.ensure(sizeof(int32_t) * std::max<int64_t>(rows, 1));
-  t.stn_rp.ensure(sizeof(int64_t) * (rows + 1));  // int64 scan, narrowed to int32 below
+  t.stn_rp.ensure(sizeof(int64_t) * (rows + 1));
   const int grid = grid_rows(rows, 128);
   k_stencil<W><<<grid, 128, 0, c.stream>>>(0, c.geom, S.nclass, t.stn_crb.as<int64_t>(), S.c_dn,
                                            B.act_list.as<uint32_t>(), B.dtab.as<uint64_t>(), S.dns.as<W>(),
