@@ -324,9 +324,9 @@ def run_ours(args):
                                              / hv_s / 1e9,
                              "note": ("split-spin sweeps: every gather is an L2 hit inside the segment being "
                                       "processed, so HBM carries only the compulsory bytes (ncu: 1.006x); the "
-                                      "sweeps are bound by L2 gather latency and instruction issue (ncu on the "
-                                      "4x4 (5,5) block: 61% issue, 50% of L2 throughput), "
-                                      "profiles/k_hv_stn_4x4_sector55_nv128_mixed_full.md")} if split else {})},
+                                      "sweeps are bound by gathers that miss L1 (ncu on the 4x4 (5,5) block, 32 "
+                                      "vectors: L1 67% busy with 30% hits, L2 50%, issue 49%), "
+                                      "profiles/k_hv_stn_4x4_sector55_nv32_mixed_sol.md")} if split else {})},
             "rate": {"hop_vector_products_per_s": prof["hv_hops"] / dev_s,
                      "hv_kernel_hop_vector_products_per_s": prof["hv_hops"] / hv_s,
                      "note": "nonzero off-diagonal hops x vectors per second: precision-neutral"},

@@ -95,7 +95,7 @@ __device__ __forceinline__ double2 ld_cg(const double2* p) { return __ldcg(p); }
 // Columns stay with the same warp throughout. Bound: L2 traffic, 32 bytes per
 // trailing element and step, and 4-6 us of barriers and dependent sums per
 // step. Against one 256-thread CTA per matrix with B v and the update in
-// separate passes: 620 matrices up to 622 rows (4x2 ED curve) 325 -> 29 ms,
+// separate passes: 620 matrices up to 622 rows (4x2 ED curve) 325 -> 27 ms,
 // nine of 1764 rows 7625 -> 299 ms, nine of 336 rows 49 -> 3.3 ms.
 __device__ void dense_eig(int n, double2* __restrict__ A, double* __restrict__ work, double* __restrict__ ev,
                           double2* v, double2* w, double2* u, int rank, int nr, double (*red)[kEigWarps], int& flip) {

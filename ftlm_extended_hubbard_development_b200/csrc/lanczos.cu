@@ -275,7 +275,7 @@ __global__ void k_start_gather(int64_t dim, int NV, int nva, const double2* __re
 // recurrence runs on one lane, the others help to load and store. With a vector
 // per lane every lane waited for the longest QL iteration of its 32 (sweeps of
 // one warp diverge at every deflation): 5 vectors x 80 steps took 3.2 ms and 72
-// blocks of 32 x 120 took 10.7; now 1.0 and 4.2 (with ql_norm, ql.cuh). Bound: the
+// blocks of 32 x 120 took 10.7; now 1.1 and 4.6 (with ql_rotation, ql.cuh). Bound: the
 // dependent chain of a rotation.
 // alpha/beta are [sweep][K][ld] (vector r = sweep r/nvmax, lane r%nvmax),
 // steps[r] the alphas taken. Outputs eigenvalues and z^2 * inv_r into [R][K]
