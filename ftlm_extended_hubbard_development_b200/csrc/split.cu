@@ -1268,7 +1268,7 @@ bool split_prepare(Ctx& c, int nv, bool fp32) {
   return true;
 }
 
-int seg_variant(Ctx& c, const void* in, void* out, int nv, bool fp32) {
+int seg_variant(Ctx& c, const StnSweep& both, int nv, bool fp32, const double* scale, fx128* partial) {
   if (c.hv_forced >= 0 && c.hv_forced < kSegVariants) return c.hv_forced;
   int width = 1;  // the wide sweeps take any number of vectors: one measurement per power of two
   while (width < nv) width <<= 1;
@@ -1290,13 +1290,17 @@ int seg_variant(Ctx& c, const void* in, void* out, int nv, bool fp32) {
   // more registers: of their variants 1, with 128 registers, or 2, with one chunk a lane,
   // was the fastest on every block (us per H*V, variants 0-4: 5x3 (12,5) 2 FP32 vectors 48
   // 37 35 44 48, 4x3 (5,7) 4 FP64 43 31 32 35 52, 4x4 (12,5) 3 FP32 96 91 85 103 99, 6x3
-  // (14,14) 43 FP32 527 487 564 590 554), and only those two are timed: a single timing
-  // picked variant 3 on the first of them.
+  // (14,14) 43 FP32 527 487 564 590 554). Only those two are timed, warm, by three launches
+  // of both sweeps with their dot products: cold single launches of one sweep picked the
+  // slower on 4x4 (12,5) and 5x3 (3,9) (91 for 85 us, 47 for 43) and variant 3 on 5x3 (12,5).
   const bool wide = c.split_wide;
   auto timed = [&](int v) { return !fours || v == 1 || v == 2; };
+  const void* in = both.in[0];
+  void* out = both.out[0];
   const StnSweep one{{&c, nullptr}, {in, nullptr}, {out, nullptr}, 1};
   auto run = [&](int v) {
-    if (wide) launch_stn(c, v, one, nv, fp32, nullptr, nullptr);
+    if (fours) launch_stn(c, v, both, nv, fp32, scale, partial);
+    else if (wide) launch_stn(c, v, one, nv, fp32, nullptr, nullptr);
     else launch_seg(c, c, v, in, out, nv, fp32, nullptr, nullptr, seg_grid(c, v), true, 0);
   };
   float best_ms[kSegVariants];
@@ -1304,11 +1308,12 @@ int seg_variant(Ctx& c, const void* in, void* out, int nv, bool fp32) {
     best_ms[v] = 1e30f;
     if (!wide) run(v);  // warm
   }
-  for (int rep = 0; rep < (wide ? 2 : 3); ++rep)
+  for (int rep = 0; rep < (fours ? 1 : wide ? 2 : 3); ++rep)
     for (int v = 0; v < kSegVariants; ++v) {
       if (!timed(v)) continue;
+      if (fours) run(v);
       FTLM_CUDA(cudaEventRecord(e0, c.stream));
-      run(v);
+      for (int k = 0; k < (fours ? 3 : 1); ++k) run(v);
       FTLM_CUDA(cudaEventRecord(e1, c.stream));
       FTLM_CUDA(cudaEventSynchronize(e1));
       float ms = 0.f;
@@ -1321,7 +1326,7 @@ int seg_variant(Ctx& c, const void* in, void* out, int nv, bool fp32) {
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   c.prof.tune_runs += 1;
-  c.prof.kernel_launches += wide ? 2 * (fours ? 2 : kSegVariants) : 4 * kSegVariants;
+  c.prof.kernel_launches += fours ? 4 * 2 : wide ? 2 * kSegVariants : 4 * kSegVariants;
   hv_tuned_store(c, key, best);
   return best;
 }
@@ -1329,10 +1334,10 @@ int seg_variant(Ctx& c, const void* in, void* out, int nv, bool fp32) {
 int hv_apply_split(Ctx& c, const void* in, const void* in_d, void* out, void* out_d, int nv, bool fp32,
                    const double* scale, fx128* partial) {
   Ctx& f = flipped_tables(c);
-  const int var = seg_variant(c, in, out, nv, fp32);
+  const StnSweep both{{&c, &f}, {in, in_d}, {out, out_d}, 2};
+  const int var = seg_variant(c, both, nv, fp32, scale, partial);
   c.prof.hv_variant = var;
   if (c.split_wide) {
-    const StnSweep both{{&c, &f}, {in, in_d}, {out, out_d}, 2};
     const int rows = launch_stn(c, var, both, nv, fp32, scale, partial);
     c.prof.kernel_launches += 1;
     return rows;
