@@ -365,22 +365,24 @@ inline int sweep_width(int nvec, bool fp32) { return fp32 ? (nvec + 1) / 2 * 2 :
 void vectors_from_host(Ctx& c, int nvec, int NV, bool fp32, const double* in, void* vec);
 void vectors_to_host(Ctx& c, int nvec, int NV, bool fp32, const void* vec, double* out);
 constexpr int64_t kConvertChunk = int64_t(1) << 24, kConvertLeast = int64_t(1) << 16;
-// Whether the host converts `rows` x nvec elements, padded to NV vectors. Its loops cost
-// by the padded element, most for one vector; the device's way costs two launches and
-// copies of 16 bytes an element, and FP64 padding needs no more than that. Whole calls,
+// Whether the host converts `rows` x nvec elements, padded to NV vectors. Its loops and
+// zero fill cost by the padded element, the device's way two launches and copies of 16
+// bytes by the element: the difference follows rows (3 NV - 2 nvec). One vector is dearer on
+// the host, and FP64 padding on the device needs no more than its elements. Whole calls,
 // host / device (us), mixed precision:
 //   1 vector   4036 rows 96 / 97, 5072 88 / 81, 14520 153 / 131
 //   2 vectors  8008 rows 113 / 137, 14520 182 / 211
-//   3 (4)      14520 rows 264 / 274
+//   3 (4)      14520 rows 264-283 / 274-314
 //   5 (8)      5072 rows 173 / 180, 8008 262 / 251, 14520 463 / 380
 //   8 vectors  8008 rows 296 / 350, 14520 538 / 521
+//   13 (16)    4368 rows 333 / 369
 //   14 (16)    4036 rows 283 / 321, 5072 340 / 367, 8008 552 / 505
 //   24 (32)    1176 rows 162 / 185, 4036 510 / 424
 // FP64 with padding (else nothing is converted): 198 elements 37 / 42, 2744 55 / 57, 4256
 // 68 / 71, 5292 77 / 74, 8820 113 / 87, 20180 216 / 147.
 inline bool host_convert(int64_t rows, int nvec, int NV, bool fp32) {
   if (!fp32) return rows * nvec < 5000;
-  return nvec == 1 ? rows < 4500 : rows * NV < (NV == nvec ? 100000 : 56000);
+  return nvec == 1 ? rows < 4500 : rows * (3 * NV - 2 * nvec) < (NV < 32 ? 100000 : 84000);
 }
 int hv_split_max_grid(const Ctx& c);
 // x_D[p(q)] = conj(f_q) x[q];  y[q] += f_q y_D[p(q)].
